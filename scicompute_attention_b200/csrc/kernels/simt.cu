@@ -1,4 +1,5 @@
-// Plain SIMT attention: the functional (not tuned) path behind the reference-level backends.
+// Plain SIMT attention: the functional (not tuned) path behind the reference-level backends. fp32 forward calls whose
+// rows allow 16-byte loads go to the tiled kernel of fp32_tiled.cu instead.
 //
 // It serves three reference entry points with one kernel:
 //   LaunchNaiveForward  (src/backends/naive/attention_naive.cuh:60)  - any dtype incl. fp32
@@ -163,6 +164,10 @@ int LaunchDecodePartialF32(const ScaDecodeFwdParams& d, cudaStream_t stream) {
     return LaunchSimt(p, SCA_DTYPE_F32, stream);
 }
 
+// fp32 inputs in tiles (fp32_tiled.cu).
+bool Fp32TiledTakes(const ScaFlashFwdParams& f);
+int LaunchFp32Tiled(const ScaFlashFwdParams& f, cudaStream_t stream);
+
 }  // namespace sca_b200
 
 using namespace sca_b200;
@@ -181,6 +186,7 @@ extern "C" int sca_launch_simt_forward(const ScaFlashFwdParams* params, void* st
         f.num_heads % f.num_kv_heads != 0) {
         return Fail(SCA_INVALID_ARGUMENT, "attention: invalid geometry");
     }
+    if (Fp32TiledTakes(f)) return LaunchFp32Tiled(f, static_cast<cudaStream_t>(stream));
     SimtParams p{};
     p.q = f.q; p.k = f.k; p.v = f.v; p.out = f.out;
     p.lse = f.return_lse ? f.lse : nullptr;
