@@ -106,6 +106,8 @@ struct FlashKernelParams {
     int causal;
     int diagonal;
     int m_blocks;
+    int pack_shift;      // log2 of the query heads that share a tile (see "Packed heads")
+    int tiles_per_item;  // query tiles a work item fills (at most QT)
     // packed variable-length batches (null for dense [B, H, S, D] problems): seqs[s] = {first query token,
     // first key token, S_q, S_kv}; entries[e] = {sequence, query block}, heaviest first
     const int4* seqs;
@@ -118,12 +120,12 @@ struct FlashKernelParams {
     int block_size, block_shift;  // block_size = 1 << block_shift
 };
 
-// KV tiles a query tile starting at row m0 of its sequence has to visit.
+// KV tiles a query tile of `tokens` tokens starting at token m0 of its sequence has to visit.
 template <int BN>
-__device__ __forceinline__ int TilesFor(int m0, int seq_q, int seq_kv, int causal, int diagonal) {
+__device__ __forceinline__ int TilesFor(int m0, int tokens, int seq_q, int seq_kv, int causal, int diagonal) {
     if (m0 >= seq_q) return 0;
     int64_t limit = seq_kv;
-    if (causal) limit = min(limit, static_cast<int64_t>(m0) + kBlockM + diagonal);
+    if (causal) limit = min(limit, static_cast<int64_t>(min(m0 + tokens, seq_q)) + diagonal);
     if (limit <= 0) return 0;
     return static_cast<int>((limit + BN - 1) / BN);
 }
@@ -178,18 +180,24 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    // ---- work items: (query block, batch*head), heaviest causal blocks first. The list is dealt to the
+    // ---- Packed heads: P = 1 << pack_shift query heads of one kv head share a query tile (row r = token m0 + r / P, head
+    // h + r % P). They read the same K/V tiles, so the rows of a short or ragged chunk fill up with other heads instead
+    // of padding, and the two tiles of a causal item lie 128 / P tokens apart instead of 128, so that both need the same
+    // number of KV tiles in all but one item of P (a tile left alone for a step has nothing to overlap with). ----
+    // ---- work items: (query block, batch * packed head), heaviest causal blocks first. The list is dealt to the
     // CTAs in rounds of gridDim.x items, every other round in reverse CTA order, so that the CTA that got
     // the heaviest item of one round gets the lightest of the next (the static schedule then ends within
     // about one KV tile of each other on all SMs). Every role of a CTA walks the same sequence. ----------
-    const int bh_count = p.batch * p.heads;
-    const int total_items = kVarlen ? p.num_entries * p.heads : p.m_blocks * bh_count;
+    const int tile_tokens = kBlockM >> p.pack_shift;
+    const int packed_heads = p.heads >> p.pack_shift;
+    const int bh_count = p.batch * packed_heads;
+    const int total_items = kVarlen ? p.num_entries * packed_heads : p.m_blocks * bh_count;
     struct Item {
-        int b, h, h_kv;
+        int b, h, h_kv;               // h: first of the item's query heads
         int seq;                      // index of the sequence (row of the page table); 0 for dense problems
         int q_tok0, kv_tok0;          // first row of the sequence in the packed tensors (0 for dense problems)
         int seq_q, seq_kv, diagonal;  // of this item's sequence
-        int m0[2];                    // first query row of each tile, relative to the sequence
+        int m0[2];                    // first token of each tile, relative to the sequence
         int ntiles[2];
         int n_max;
     };
@@ -197,12 +205,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         Item w;
         int mb;
         if constexpr (kVarlen) {
-            const int2 entry = __ldg(p.entries + idx / p.heads);
+            const int2 entry = __ldg(p.entries + idx / packed_heads);
             const int4 seq = __ldg(p.seqs + entry.x);
             mb = entry.y;
             w.seq = entry.x;
             w.b = 0;
-            w.h = idx % p.heads;
+            w.h = (idx % packed_heads) << p.pack_shift;
             w.q_tok0 = seq.x;
             w.kv_tok0 = seq.y;
             w.seq_q = seq.z;
@@ -212,8 +220,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             mb = p.m_blocks - 1 - idx / bh_count;
             w.seq = 0;
             const int bh = idx % bh_count;
-            w.b = bh / p.heads;
-            w.h = bh % p.heads;
+            w.b = bh / packed_heads;
+            w.h = (bh % packed_heads) << p.pack_shift;
             w.q_tok0 = 0;
             w.kv_tok0 = 0;
             w.seq_q = p.seq_q;
@@ -221,10 +229,10 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             w.diagonal = p.diagonal;
         }
         w.h_kv = w.h / (p.heads / p.kv_heads);
-        w.m0[0] = (mb * QT) * kBlockM;
-        w.m0[1] = (mb * QT + 1) * kBlockM;
-        w.ntiles[0] = TilesFor<BN>(w.m0[0], w.seq_q, w.seq_kv, p.causal, w.diagonal);
-        w.ntiles[1] = QT > 1 ? TilesFor<BN>(w.m0[1], w.seq_q, w.seq_kv, p.causal, w.diagonal) : 0;
+        w.m0[0] = mb * p.tiles_per_item * tile_tokens;
+        w.m0[1] = w.m0[0] + tile_tokens;
+        w.ntiles[0] = TilesFor<BN>(w.m0[0], tile_tokens, w.seq_q, w.seq_kv, p.causal, w.diagonal);
+        w.ntiles[1] = p.tiles_per_item > 1 ? TilesFor<BN>(w.m0[1], tile_tokens, w.seq_q, w.seq_kv, p.causal, w.diagonal) : 0;
         w.n_max = max(w.ntiles[0], w.ntiles[1]);
         return w;
     };
@@ -292,7 +300,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     MbarExpectTx(bar(kQFull + t), G::kQTileBytes);
                     for (int kb = 0; kb < G::kKBlocks; ++kb) {
                         TmaLoad4D(q_smem + t * G::kQTileBytes + kb * G::kQBlockBytes, &map_q, bar(kQFull + t), kb * 64,
-                                  w.q_tok0 + w.m0[t], w.h, w.b);
+                                  w.h, w.q_tok0 + w.m0[t], w.b);
                     }
                     ++q_uses[t];
                 }
@@ -374,7 +382,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     MbarExpectTx(bar(kQFull + t), G::kQTileBytes);
                     for (int kb = 0; kb < G::kKBlocks; ++kb) {
                         TmaLoad4D(q_smem + t * G::kQTileBytes + kb * G::kQBlockBytes, &map_q, bar(kQFull + t), kb * 64,
-                                  w.q_tok0 + w.m0[t], w.h, w.b);
+                                  w.h, w.q_tok0 + w.m0[t], w.b);
                     }
                     ++q_uses[t];
                 }
@@ -637,7 +645,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const uint32_t tiles_base = tiles_before;
             tiles_before += static_cast<uint32_t>(w.n_max);
             if (n_t == 0) continue;
-            const int row = w.m0[t] + row_in_tile;
+            const int row = w.m0[t] + (row_in_tile >> p.pack_shift);                 // token of the sequence
+            const int head = w.h + (row_in_tile & ((1 << p.pack_shift) - 1));
             float m_ref = -CUDART_INF_F;  // reference point of the exponentials (log2 domain)
             float l_sum = 0.0f;
 
@@ -769,7 +778,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (!ok) break;
             TcFenceAfter();
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-            T* o_row = reinterpret_cast<T*>(p.out) + w.b * p.o_sb + w.h * p.o_sh + static_cast<int64_t>(w.q_tok0 + row) * p.o_ss;
+            T* o_row = reinterpret_cast<T*>(p.out) + w.b * p.o_sb + head * p.o_sh + static_cast<int64_t>(w.q_tok0 + row) * p.o_ss;
 #pragma unroll
             for (int cblk = 0; cblk < DP / 32; ++cblk) {
                 uint32_t r[32];
@@ -795,7 +804,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
             }
             if (p.lse != nullptr && row < w.seq_q) {
-                p.lse[(static_cast<int64_t>(w.b) * p.heads + w.h) * p.seq_q + row] =
+                p.lse[(static_cast<int64_t>(w.b) * p.heads + head) * p.seq_q + row] =
                     l_sum > 0.0f ? (m_ref + log2f(l_sum)) * kLn2 : -CUDART_INF_F;
             }
         }
@@ -894,14 +903,14 @@ EncodeTiledFn GetEncodeTiled() {
 // [batch][heads][seq][D] through element strides (sb, sh, ss); box = 64 elements x box_rows rows, 128B swizzle,
 // out-of-range elements read as zero.
 int MakeMap(CUtensorMap* map, const void* base, int dtype_id, int64_t d, int64_t seq, int64_t heads, int64_t batch,
-            int64_t ss, int64_t sh, int64_t sb, int box_rows, const char* what) {
+            int64_t ss, int64_t sh, int64_t sb, int box_rows, const char* what, int box_heads = 1) {
     EncodeTiledFn encode = GetEncodeTiled();
     if (encode == nullptr) return Fail(SCA_CUDA_ERROR, "flash attention: cuTensorMapEncodeTiled is unavailable");
     const cuuint64_t dims[4] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(seq),
                                 static_cast<cuuint64_t>(heads), static_cast<cuuint64_t>(batch)};
     const cuuint64_t strides[3] = {static_cast<cuuint64_t>(ss) * 2, static_cast<cuuint64_t>(sh) * 2,
                                    static_cast<cuuint64_t>(sb) * 2};
-    const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};
+    const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_heads), 1};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
     const CUtensorMapDataType type =
         dtype_id == SCA_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -960,21 +969,41 @@ struct VarlenWork {
     int64_t workspace_bytes;
 };
 
+// Query heads that share a tile: the largest power of two that divides the GQA group, at most kMaxPack.
+constexpr int kMaxPackShift = 2;
+int PackShift(int64_t group) {
+    int shift = 0;
+    while (shift < kMaxPackShift && group % (2ll << shift) == 0) ++shift;
+    return shift;
+}
+
 int64_t VarlenWorkspaceBytes(int64_t num_seqs, int64_t total_q) {
-    // one int4 per sequence + one int2 per block of 128 query rows (an upper bound for both geometries)
-    return num_seqs * 16 + (total_q / kBlockM + num_seqs) * 8 + 64;
+    // one int4 per sequence + one int2 per work item and packed head; an item covers at least kBlockM >> kMaxPackShift tokens
+    return num_seqs * 16 + (total_q / (kBlockM >> kMaxPackShift) + num_seqs) * 8 + 64;
+}
+
+// Entries of the work list when one entry covers `tokens` query tokens, and the bytes the list takes.
+int64_t VarlenEntries(const VarlenWork& vw, int64_t tokens) {
+    int64_t n = 0;
+    for (int64_t s = 0; s < vw.num_seqs; ++s) n += std::max<int64_t>(0, (static_cast<int64_t>(vw.cu_q[s + 1]) - vw.cu_q[s] + tokens - 1) / tokens);
+    return n;
+}
+int64_t VarlenListBytes(const VarlenWork& vw, int64_t tokens) {
+    return vw.num_seqs * static_cast<int64_t>(sizeof(int4)) + VarlenEntries(vw, tokens) * static_cast<int64_t>(sizeof(int2));
 }
 
 // Builds {first q token, first kv token, S_q, S_kv} per sequence and the (sequence, query block) list, heaviest
-// block first, and copies both into the workspace (stream-ordered; the host vectors may die on return).
-int UploadVarlenWork(const VarlenWork& vw, int rows_per_entry, int block_n, bool causal, cudaStream_t stream,
+// block first, and copies both into the workspace (stream-ordered; the host vector may die on return).
+int UploadVarlenWork(const VarlenWork& vw, int tokens_per_entry, int block_n, bool causal, cudaStream_t stream,
                      const int4** seqs_out, const int2** entries_out, int* num_entries_out) {
-    std::vector<int4> seqs(static_cast<size_t>(vw.num_seqs));
+    const size_t seq_bytes = static_cast<size_t>(vw.num_seqs) * sizeof(int4);
     struct Weighted {
         int2 entry;
         int64_t tiles;
     };
+    std::vector<int4> image(static_cast<size_t>(vw.num_seqs));  // the sequences, then the entries
     std::vector<Weighted> list;
+    list.reserve(static_cast<size_t>(VarlenEntries(vw, tokens_per_entry)));
     for (int64_t s = 0; s < vw.num_seqs; ++s) {
         const int64_t sq = static_cast<int64_t>(vw.cu_q[s + 1]) - vw.cu_q[s];
         const int64_t skv = static_cast<int64_t>(vw.cu_kv[s + 1]) - vw.cu_kv[s];
@@ -982,32 +1011,29 @@ int UploadVarlenWork(const VarlenWork& vw, int rows_per_entry, int block_n, bool
             return Fail(SCA_INVALID_ARGUMENT, "flash varlen: sequence " + std::to_string(s) + " has S_q=" + std::to_string(sq) +
                                                   ", S_kv=" + std::to_string(skv) + (causal ? " (causal needs 0 < S_q <= S_kv)" : " (both must be > 0)"));
         }
-        seqs[static_cast<size_t>(s)] = make_int4(vw.cu_q[s], vw.cu_kv[s], static_cast<int>(sq), static_cast<int>(skv));
-        for (int64_t mb = 0; mb * rows_per_entry < sq; ++mb) {
+        image[static_cast<size_t>(s)] = make_int4(vw.cu_q[s], vw.cu_kv[s], static_cast<int>(sq), static_cast<int>(skv));
+        for (int64_t mb = 0; mb * tokens_per_entry < sq; ++mb) {
             int64_t limit = skv;
-            if (causal) limit = std::min<int64_t>(limit, std::min<int64_t>(sq, (mb + 1) * rows_per_entry) + (skv - sq));
+            if (causal) limit = std::min<int64_t>(limit, std::min<int64_t>(sq, (mb + 1) * tokens_per_entry) + (skv - sq));
             list.push_back({make_int2(static_cast<int>(s), static_cast<int>(mb)), (limit + block_n - 1) / block_n});
         }
     }
     std::stable_sort(list.begin(), list.end(), [](const Weighted& a, const Weighted& b) { return a.tiles > b.tiles; });
-    std::vector<int2> entries(list.size());
-    for (size_t i = 0; i < list.size(); ++i) entries[i] = list[i].entry;
-    const size_t seq_bytes = seqs.size() * sizeof(int4);
-    const size_t entry_bytes = entries.size() * sizeof(int2);
-    if (vw.workspace == nullptr || static_cast<int64_t>(seq_bytes + entry_bytes) > vw.workspace_bytes) {
+    const size_t bytes = seq_bytes + list.size() * sizeof(int2);
+    if (vw.workspace == nullptr || static_cast<int64_t>(bytes) > vw.workspace_bytes) {
         return Fail(SCA_INVALID_ARGUMENT, "flash varlen: workspace of " + std::to_string(vw.workspace_bytes) + " bytes is too small (" +
-                                              std::to_string(seq_bytes + entry_bytes) + " needed)");
+                                              std::to_string(bytes) + " needed)");
     }
+    image.resize((bytes + sizeof(int4) - 1) / sizeof(int4));
+    int2* entries = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(image.data()) + seq_bytes);
+    for (size_t i = 0; i < list.size(); ++i) entries[i] = list[i].entry;
     unsigned char* base = static_cast<unsigned char*>(vw.workspace);
-    if (cudaError_t e = cudaMemcpyAsync(base, seqs.data(), seq_bytes, cudaMemcpyHostToDevice, stream); e != cudaSuccess) {
-        return FailCuda(e, "cudaMemcpyAsync(varlen sequences)");
-    }
-    if (cudaError_t e = cudaMemcpyAsync(base + seq_bytes, entries.data(), entry_bytes, cudaMemcpyHostToDevice, stream); e != cudaSuccess) {
+    if (cudaError_t e = cudaMemcpyAsync(base, image.data(), bytes, cudaMemcpyHostToDevice, stream); e != cudaSuccess) {
         return FailCuda(e, "cudaMemcpyAsync(varlen work list)");
     }
     *seqs_out = reinterpret_cast<const int4*>(base);
     *entries_out = reinterpret_cast<const int2*>(base + seq_bytes);
-    *num_entries_out = static_cast<int>(entries.size());
+    *num_entries_out = static_cast<int>(list.size());
     return SCA_OK;
 }
 
@@ -1022,7 +1048,21 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
                 const PagedWork* paged = nullptr) {
     using G = FlashGeom<DP, QT, BN>;
     CUtensorMap map_q, map_k, map_v;
-    if (int rc = MakeMap(&map_q, f.q, f.dtype_id, f.head_dim, f.seq_q, f.num_heads, f.batch, f.q_ss, f.q_sh, f.q_sb, kBlockM, "q")) return rc;
+    // rows of a query tile: P heads x 128 / P tokens
+    int pack_shift = PackShift(f.num_heads / f.num_kv_heads);
+    int tiles_per_item = QT;
+    if (varlen != nullptr) {
+        while (pack_shift > 0 && VarlenListBytes(*varlen, (QT * kBlockM) >> pack_shift) > varlen->workspace_bytes) --pack_shift;
+    }
+    if (QT > 1) {
+        // fewer tiles than SMs: one tile per CTA (a step of one tile alone takes 0.9 of a step of two)
+        const int64_t tokens = kBlockM >> pack_shift;
+        const int64_t tiles = (varlen != nullptr ? VarlenEntries(*varlen, tokens) : (f.seq_q + tokens - 1) / tokens * f.batch) *
+                              (f.num_heads >> pack_shift);
+        if (tiles <= SmCount() && (varlen == nullptr || VarlenListBytes(*varlen, tokens) <= varlen->workspace_bytes)) tiles_per_item = 1;
+    }
+    if (int rc = MakeMap(&map_q, f.q, f.dtype_id, f.head_dim, f.num_heads, f.seq_q, f.batch, f.q_sh, f.q_ss, f.q_sb, 1 << pack_shift,
+                         "q", kBlockM >> pack_shift)) return rc;
     if (paged != nullptr) {
         // the pool as [rows = blocks * block_size, H_kv, D]; one box = one page of one kv head and column block
         const int64_t rows = paged->num_blocks * paged->block_size;
@@ -1084,12 +1124,15 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
     p.scale_log2 = f.scale * kLog2e;
     p.causal = f.causal ? 1 : 0;
     p.diagonal = static_cast<int>(f.causal ? f.diagonal : 0);
-    p.m_blocks = static_cast<int>((f.seq_q + QT * kBlockM - 1) / (QT * kBlockM));
+    p.pack_shift = pack_shift;
+    p.tiles_per_item = tiles_per_item;
+    const int item_tokens = (tiles_per_item * kBlockM) >> pack_shift;
+    p.m_blocks = static_cast<int>((f.seq_q + item_tokens - 1) / item_tokens);
     if (varlen != nullptr) {
-        if (int rc = UploadVarlenWork(*varlen, QT * kBlockM, BN, f.causal != 0, stream, &p.seqs, &p.entries, &p.num_entries)) return rc;
+        if (int rc = UploadVarlenWork(*varlen, item_tokens, BN, f.causal != 0, stream, &p.seqs, &p.entries, &p.num_entries)) return rc;
     }
-    const int64_t ctas = varlen != nullptr ? static_cast<int64_t>(p.num_entries) * p.heads
-                                           : static_cast<int64_t>(p.m_blocks) * p.batch * p.heads;
+    const int64_t ctas = (varlen != nullptr ? static_cast<int64_t>(p.num_entries) : static_cast<int64_t>(p.m_blocks) * p.batch) *
+                         (p.heads >> pack_shift);
     if (ctas <= 0 || ctas > 0x7fffffffLL) {
         return Fail(SCA_INVALID_ARGUMENT, "flash attention: grid of " + std::to_string(ctas) + " blocks is out of range");
     }
