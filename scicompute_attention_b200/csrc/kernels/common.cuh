@@ -113,6 +113,11 @@ __device__ __forceinline__ float2 Fma2(float2 a, float2 b, float2 c) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
     return d;
 }
+__device__ __forceinline__ float Max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 __device__ __forceinline__ float2 Add2(float2 a, float2 b) {
     uint64_t ra, rb, rd;
     asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));

@@ -72,7 +72,6 @@ struct PvFormat {
     using type = __half;
     static constexpr bool kConvertV = std::is_same<T, __nv_bfloat16>::value;
 };
-constexpr int kFlashThreads = 384;   // warp 0 TMA, 1 MMA, 2 TMEM owner, 3 idle, 4-7 / 8-11 softmax
 constexpr int kTmemColumns = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain: P stays <= 2^8
 
@@ -130,11 +129,19 @@ __device__ __forceinline__ int TilesFor(int m0, int tokens, int seq_q, int seq_k
     return static_cast<int>((limit + BN - 1) / BN);
 }
 
+// Threads of a CTA: warp 0 TMA and tensor-memory owner, 1 MMA, 2-5 softmax of tile 0, 6-9 softmax of tile 1 (where there
+// is one), and for paged bf16 one more warp that converts V. No idle warps: a softmax thread keeps a whole row of
+// scores in registers, and ten warps may have 200 registers a thread where twelve get 168.
+template <typename T, int QT, bool kPaged>
+constexpr int FlashThreads() {
+    return 32 * (2 + 4 * QT + (kPaged && PvFormat<T>::kConvertV ? 1 : 0));
+}
+
 // kVarlen: the work list comes from the (sequence, query block) table of a packed ragged batch; otherwise it is
 // computed from the dense [B, H, S, D] geometry and every per-sequence quantity is a launch constant.
 // kPaged (only with kVarlen): K and V of a sequence are scattered over the pages of a KV pool.
 template <typename T, int DP, int QT, int BN, bool kVarlen, bool kPaged = false>
-__global__ void __launch_bounds__(kFlashThreads, 1)
+__global__ void __launch_bounds__(FlashThreads<T, QT, kPaged>(), 1)
 flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const FlashKernelParams p) {
     using G = FlashGeom<DP, QT, BN>;
@@ -155,14 +162,18 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     constexpr int kODone = kPFull + 2;              // [2]
     constexpr int kQEmpty = kODone + 2;             // [2]
     constexpr int kOFree = kQEmpty + 2;             // [2]
-    constexpr int kVReady = kOFree + 2;             // [kSlots] paged bf16: V tile rewritten as fp16 in place
+    constexpr int kPLast = kOFree + 2;              // [2]
+    constexpr int kVReady = kPLast + 2;             // [kSlots] paged bf16: V tile rewritten as fp16 in place
     constexpr int kNumBars = kVReady + G::kSlots;
     // P and V enter the P V product as fp16 also for bf16 inputs (PvFormat). Contiguous V comes from an fp16 copy made
     // before the launch; the pages of a pool are rewritten tile by tile in shared memory by warps 2 and 3 instead
     // (a copy of the pool would cost more than the prefill), at the price of some issue slots of two schedulers.
     using PT = typename PvFormat<T>::type;
     constexpr bool kCvtInKernel = kPaged && PvFormat<T>::kConvertV;
-    constexpr int kConverterThreads = 64;
+    constexpr int kConverterThreads = 32;
+    constexpr int kConverterWarp = 2 + 4 * QT;
+    // P is handed over in two pieces: the first kPEarly keys let P V start while the rest is still in the softmax
+    constexpr int kPEarly = BN == 128 ? 96 : 32;
     static_assert(!kPaged || kVarlen, "paged K/V runs on the packed work list");
     static_assert(kNumBars * 8 + 16 <= G::kBarrierBytes, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + (bar_base - smem_base) + kNumBars * 8);
@@ -248,9 +259,10 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             MbarInit(bar(kQFull + i), 1);
             MbarInit(bar(kQEmpty + i), 1);
             MbarInit(bar(kSFull + i), 1);
-            MbarInit(bar(kPFull + i), 128);
+            MbarInit(bar(kPFull + i), 4);
+            MbarInit(bar(kPLast + i), 4);
             MbarInit(bar(kODone + i), 1);
-            MbarInit(bar(kOFree + i), 128);
+            MbarInit(bar(kOFree + i), 4);
         }
         for (int i = 0; i < G::kSlots; ++i) {
             MbarInit(bar(kKvFull + i), 1);
@@ -260,7 +272,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         *abort_flag = 0;
         FenceBarrierInit();
     }
-    if (warp == 2) {
+    if (warp == 0) {
         TmemAlloc(SmemAddr(tmem_slot), kTmemColumns);
         TmemRelinquish();
     }
@@ -350,7 +362,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     const int32_t id = __shfl_sync(0xffffffffu, phys, pg);
                     // an unmapped page reads from the first row behind the pool: all zeros
                     const int first_row = ((valid >> pg) & 1u) ? (id << p.block_shift) : (p.num_kv_blocks << p.block_shift);
-                    if (lane == 0) {
+                    if (ElectOne()) {
                         for (int kb = 0; kb < G::kKBlocks; ++kb) {
                             TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes + pg * page_bytes, map,
                                       bar(kKvFull + slot), kb * 64, first_row, w.h_kv, 0);
@@ -363,7 +375,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         failed = !ok;
     } else if (warp == 0) {
         // ================================ TMA producer =============================================
-        if (lane == 0) {
+        if (ElectOne()) {
             PrefetchTensorMap(&map_q);
             PrefetchTensorMap(&map_k);
             PrefetchTensorMap(&map_v);
@@ -422,7 +434,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
     } else if (warp == 1) {
         // ================================ MMA issuer ================================================
-        if (lane == 0) {
+        if (ElectOne()) {
             constexpr uint32_t fmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBf16;
             constexpr uint32_t idesc_s = MakeInstrDesc(fmt, fmt, 0, 0, kBlockM, BN);  // Q K^T: both K-major
             // P V: V is MN-major; both operands in the P V format (fp16 also for bf16 inputs, see PvFormat: V then
@@ -450,15 +462,23 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     else MmaSS<true>(d, a0 + qa, b0 + kb, idesc_s);
                 }
             };
-            auto issue_pv = [&](int t, uint32_t slot, bool first) {
+            // waits for the second piece of P (barrier `last`, parity `parity`) half-way
+            auto issue_pv = [&](int t, uint32_t slot, bool first, uint32_t last, uint32_t parity) {
                 const uint64_t b0 = vmajor_hi | ((ring_smem + slot * G::kKvTileBytes) >> 4);
+                const uint32_t a = kDoubleS ? s_tmem_db : s_tmem[t];
 #pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks) {
+                for (int ks = 0; ks < kPEarly / 16; ++ks) {
                     // 16 keys further: 8 packed P columns in tensor memory, 16 rows (2048 bytes) of V
-                    const uint32_t a = kDoubleS ? s_tmem_db : s_tmem[t];
                     if (ks == 0) MmaTSFlag(o_tmem[t], a, b0, idesc_o, first ? 0u : 1u);
                     else MmaTS<true>(o_tmem[t], a + ks * 8, b0 + ks * (2048 >> 4), idesc_o);
                 }
+                if (!MbarWait(last, parity, abort_flag)) return false;
+                TcFenceAfter();
+#pragma unroll
+                for (int ks = kPEarly / 16; ks < BN / 16; ++ks) {
+                    MmaTS<true>(o_tmem[t], a + ks * 8, b0 + ks * (2048 >> 4), idesc_o);
+                }
+                return true;
             };
             uint32_t q_uses[2] = {0, 0};    // items finished per query buffer
             uint32_t steps[2] = {0, 0};     // KV tiles processed per query tile (phase of s_full / p_full / o_done)
@@ -496,14 +516,15 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                     for (int j = 0; j < n && ok; ++j) {
                         const uint32_t buf = j & 1;
-                        ok = MbarWait(bar(kPFull + buf), buf_uses[buf] & 1u, abort_flag);
-                        ++buf_uses[buf];
+                        const uint32_t p_parity = buf_uses[buf]++ & 1u;
+                        ok = MbarWait(bar(kPFull + buf), p_parity, abort_flag);
                         if (ok && j == 0 && q_uses[0] > 0) ok = MbarWait(bar(kOFree), (q_uses[0] - 1) & 1u, abort_flag);
                         if (ok) ok = next_slot(&slot, true);  // V_j
                         if (!ok) break;
                         TcFenceAfter();
                         s_tmem_db = tmem_base + G::kSCol + buf * 64;
-                        issue_pv(0, slot, j == 0);
+                        ok = issue_pv(0, slot, j == 0, bar(kPLast + buf), p_parity);
+                        if (!ok) break;
                         MmaCommit(bar(kODone + buf));
                         MmaCommit(bar(kKvEmpty + slot));
                         if (j + 2 < n) {
@@ -555,7 +576,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (ok && j == 0 && q_uses[t] > 0) ok = MbarWait(bar(kOFree + t), (q_uses[t] - 1) & 1u, abort_flag);
                         if (!ok) break;
                         TcFenceAfter();
-                        issue_pv(t, slot_of(it_v), j == 0);
+                        ok = issue_pv(t, slot_of(it_v), j == 0, bar(kPLast + t), steps[t] & 1u);
+                        if (!ok) break;
                         MmaCommit(bar(kODone + t));
                         ++steps[t];
                         if (j + 1 < w.ntiles[t]) {
@@ -575,11 +597,10 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             failed = !ok;
         }
-    } else if (kCvtInKernel && warp < 4) {
-        // ================================ V converter (warps 2 and 3, paged bf16) ====================
+    } else if (kCvtInKernel && warp == kConverterWarp) {
+        // ================================ V converter (one warp, paged bf16) ========================
         // Walks the ring in the producer's order; every V tile is rewritten in place from bf16 to fp16 once its
         // bytes have landed, then handed to the MMA thread through v_ready. K tiles are not touched.
-        const int tid = threadIdx.x - 64;
         uint32_t kv_loads = 0;
         bool ok = true;
         for (int r = 0; r < rounds && ok; ++r) {
@@ -606,8 +627,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 ok = __all_sync(0xffffffffu, MbarWait(bar(kKvFull + slot), phase, abort_flag));
                 if (!ok) break;
                 uint4* tile = reinterpret_cast<uint4*>(smem + (ring_smem - smem_base) + slot * G::kKvTileBytes);
-#pragma unroll 4
-                for (int c = tid; c < G::kKvTileBytes / 16; c += kConverterThreads) {
+#pragma unroll 8
+                for (int c = lane; c < G::kKvTileBytes / 16; c += kConverterThreads) {
                     uint4 x = tile[c];
                     uint32_t* word = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
@@ -623,9 +644,9 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
         }
         failed = !ok;
-    } else if (warp >= 4) {
+    } else {
         // ================================ softmax groups ============================================
-        const int t = (warp - 4) >> 2;
+        const int t = (warp - 2) >> 2;
         const int quad = warp & 3;
         const int row_in_tile = quad * 32 + lane;
         const uint32_t lane_bits = static_cast<uint32_t>(quad * 32) << 16;
@@ -665,12 +686,11 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 ok = __all_sync(0xffffffffu, MbarWait(bar(kSFull + sync), s_phase, abort_flag));
                 if (!ok) break;
                 TcFenceAfter();
-                // One pass over the S row, 64 columns at a time. The exponentials use the reference point the row
-                // already has; the half's own max is only checked against it. If a half exceeds the reference by
-                // more than the threshold (always true for the first half of an item), the reference moves and
-                // whatever was accumulated under the old one is rescaled: O, the row sum and the half of P that
-                // this step has already written. P (16-bit pairs) lands on the first BN / 2 columns of S_t;
-                // the half-row written in step h only covers columns that step h has already consumed.
+                // The row goes to registers whole. The exponentials use the reference point the row already has; the
+                // row's maximum is only checked against it. If it exceeds the reference by more than the threshold
+                // (always in the first step of an item), the reference moves and O and the row sum are rescaled.
+                // P (16-bit pairs) lands on the first BN / 2 columns of S_t, which has been read by then; its first
+                // kPEarly keys are handed over early, so that P V starts under the last exponentials.
                 const int col0 = j * BN;
                 const int kv_limit = w.seq_kv - col0;                                   // columns >= kv_limit do not exist
                 const int causal_limit = p.causal ? (row + w.diagonal - col0 + 1) : BN;  // columns >= limit are masked
@@ -678,93 +698,79 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 const uint32_t pages = kPaged ? valid_ring[(tiles_base + j) % kValidRing] : 0u;
                 const bool holes = kPaged && pages != all_pages;   // some page of this tile is unmapped
                 const bool ragged = limit < BN || holes;
-                float part4[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // this step's share of the row sum
-    #pragma unroll
-                for (int half = 0; half < BN / 64; ++half) {
-                    uint32_t ra[32], rb[32];
-                    TmemLd32(s_addr + half * 64, ra);
-                    TmemLd32(s_addr + half * 64 + 32, rb);
-                    TmemWaitLd();
-                    if (ragged) {
-    #pragma unroll
+                uint32_t sc[BN / 32][32];
+#pragma unroll
+                for (int c = 0; c < BN / 32; ++c) TmemLd32(s_addr + c * 32, sc[c]);
+                TmemWaitLd();
+                if (ragged) {
+#pragma unroll
+                    for (int c = 0; c < BN / 32; ++c) {
+#pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const int ca = half * 64 + i, cb = half * 64 + 32 + i;
-                            const bool gone_a = kPaged && holes && !((pages >> (ca >> p.block_shift)) & 1u);
-                            const bool gone_b = kPaged && holes && !((pages >> (cb >> p.block_shift)) & 1u);
-                            if (ca >= limit || gone_a) ra[i] = 0xff800000u;       // -inf
-                            if (cb >= limit || gone_b) rb[i] = 0xff800000u;
+                            const int col = c * 32 + i;
+                            const bool gone = kPaged && holes && !((pages >> (col >> p.block_shift)) & 1u);
+                            if (col >= limit || gone) sc[c][i] = 0xff800000u;  // -inf
                         }
                     }
-                    float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-    #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            mx4[e] = fmaxf(mx4[e], fmaxf(__uint_as_float(ra[i + e]), __uint_as_float(rb[i + e])));
-                        }
+                }
+                float mx4[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(__uint_as_float(sc[0][e]), __uint_as_float(sc[0][4 + e]));
+#pragma unroll
+                for (int i = 8; i < BN; i += 8) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        mx4[e] = Max3(mx4[e], __uint_as_float(sc[i / 32][i % 32 + e]), __uint_as_float(sc[i / 32][i % 32 + 4 + e]));
                     }
-                    const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0
-                    const bool move = mx > m_ref + kRescaleThreshold;  // false for a fully masked half (-inf)
-                    if (__any_sync(0xffffffffu, move)) {
-                        const float alpha = move ? Exp2(m_ref - mx) : 1.0f;  // m_ref = -inf -> 0
-                        if (j > 0) {
-                            ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + prev_sync), prev_phase, abort_flag));
-                            if (!ok) break;
-                            TcFenceAfter();
-    #pragma unroll 1
-                            for (int cblk = 0; cblk < DP / 32; ++cblk) {
-                                uint32_t r[32];
-                                TmemLd32(o_addr + cblk * 32, r);
-                                TmemWaitLd();
-    #pragma unroll
-                                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                                TmemSt32(o_addr + cblk * 32, r);
-                            }
-                        }
-                        l_sum *= alpha;
-    #pragma unroll
-                        for (int e = 0; e < 4; ++e) part4[e] *= alpha;
-                        if (half > 0) {  // the first half of P was written under the old reference
-                            uint32_t q[32];
-                            TmemWaitSt();
-                            TmemLd32(s_addr, q);
+                }
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0
+                const bool move = mx > m_ref + kRescaleThreshold;  // false for a fully masked row (-inf)
+                if (__any_sync(0xffffffffu, move)) {
+                    const float alpha = move ? Exp2(m_ref - mx) : 1.0f;  // m_ref = -inf -> 0
+                    if (j > 0) {
+                        ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + prev_sync), prev_phase, abort_flag));
+                        if (!ok) break;
+                        TcFenceAfter();
+#pragma unroll 1
+                        for (int cblk = 0; cblk < DP / 16; ++cblk) {
+                            uint32_t r[16];
+                            TmemLd16(o_addr + cblk * 16, r);
                             TmemWaitLd();
-    #pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                const float2 f = Unpack2<PT>(q[i]);
-                                q[i] = Pack2<PT>(f.x * alpha, f.y * alpha);
-                            }
-                            TmemSt32(s_addr, q);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+                            TmemSt16(o_addr + cblk * 16, r);
                         }
-                        if (move) m_ref = mx;
                     }
-                    const float neg_m = (m_ref == -CUDART_INF_F) ? 0.0f : -m_ref;
-                    uint32_t pk[32];
-                    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
-                    const float2 shift2 = make_float2(neg_m, neg_m);
-                    float2 sum_a = make_float2(part4[0], part4[1]), sum_b = make_float2(part4[2], part4[3]);
-    #pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float2 xa = Fma2(make_float2(__uint_as_float(ra[i]), __uint_as_float(ra[i + 1])), scale2, shift2);
-                        const float2 xb = Fma2(make_float2(__uint_as_float(rb[i]), __uint_as_float(rb[i + 1])), scale2, shift2);
+                    l_sum *= alpha;
+                    if (move) m_ref = mx;
+                }
+                const float neg_m = (m_ref == -CUDART_INF_F) ? 0.0f : -m_ref;
+                const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+                const float2 shift2 = make_float2(neg_m, neg_m);
+                float2 sum_a = make_float2(0.0f, 0.0f), sum_b = sum_a;
+#pragma unroll
+                for (int c = 0; c < BN / 32; ++c) {
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        const float2 xa = Fma2(make_float2(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, shift2);
+                        const float2 xb = Fma2(make_float2(__uint_as_float(sc[c][i + 2]), __uint_as_float(sc[c][i + 3])), scale2, shift2);
                         const float2 ea = make_float2(Exp2(xa.x), Exp2(xa.y));
                         const float2 eb = make_float2(Exp2(xb.x), Exp2(xb.y));
                         sum_a = Add2(sum_a, ea);
                         sum_b = Add2(sum_b, eb);
                         pk[i / 2] = Pack2<PT>(ea.x, ea.y);
-                        pk[16 + i / 2] = Pack2<PT>(eb.x, eb.y);
+                        pk[i / 2 + 1] = Pack2<PT>(eb.x, eb.y);
                     }
-                    part4[0] = sum_a.x;
-                    part4[1] = sum_a.y;
-                    part4[2] = sum_b.x;
-                    part4[3] = sum_b.y;
-                    TmemSt32(s_addr + half * 32, pk);
+                    TmemSt16(s_addr + c * 16, pk);
+                    if ((c + 1) * 32 == kPEarly || c + 1 == BN / 32) {
+                        TmemWaitSt();
+                        TcFenceBefore();
+                        __syncwarp();
+                        if (lane == 0) MbarArrive(bar((c + 1 == BN / 32 ? kPLast : kPFull) + sync));
+                    }
                 }
-                if (!ok) break;
-                l_sum += (part4[0] + part4[1]) + (part4[2] + part4[3]);
-                TmemWaitSt();
-                TcFenceBefore();
-                MbarArrive(bar(kPFull + sync));
+                l_sum += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
             }
             if (!ok) break;
 
@@ -786,7 +792,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 TmemWaitLd();
                 if (cblk == DP / 32 - 1) {
                     TcFenceBefore();
-                    MbarArrive(bar(kOFree + t));
+                    __syncwarp();
+                    if (lane == 0) MbarArrive(bar(kOFree + t));
                 }
                 if (row < w.seq_q) {
 #pragma unroll
@@ -816,7 +823,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // ---- teardown ------------------------------------------------------------------------------------
     TcFenceBefore();
     __syncthreads();
-    if (warp == 2) {
+    if (warp == 0) {
         TcFenceAfter();
         TmemDealloc(tmem_base, kTmemColumns);
     }
@@ -1137,6 +1144,7 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         return Fail(SCA_INVALID_ARGUMENT, "flash attention: grid of " + std::to_string(ctas) + " blocks is out of range");
     }
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ctas, SmCount()));  // one persistent CTA per SM
+    const unsigned threads = paged != nullptr ? FlashThreads<T, QT, true>() : FlashThreads<T, QT, false>();
     if (paged != nullptr) {
         p.page_table = paged->page_table;
         p.max_blocks_per_seq = static_cast<int>(paged->max_blocks_per_seq);
@@ -1146,15 +1154,15 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         while ((1 << p.block_shift) < p.block_size) ++p.block_shift;
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, true, true>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, true, true><<<grid, kFlashThreads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        flash_fwd_sm100_kernel<T, DP, QT, BN, true, true><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
     } else if (varlen != nullptr) {
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, true>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, true><<<grid, kFlashThreads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        flash_fwd_sm100_kernel<T, DP, QT, BN, true><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
     } else {
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, false>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, false><<<grid, kFlashThreads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        flash_fwd_sm100_kernel<T, DP, QT, BN, false><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
     }
     if (int rc = CheckLaunch("flash_fwd_sm100_kernel", stream)) return rc;
     // With SCI_ATTENTION_DEBUG_SYNC=1 CheckLaunch has waited for the kernel: a wait that ran out is known now.
