@@ -5,9 +5,9 @@
 // tile). Same arithmetic contract - fp16/bf16 inputs, fp32 accumulation, online softmax through
 // exp2, bottom-right aligned causal mask, GQA, optional log-sum-exp - on a Blackwell execution plan:
 //
-//   * one persistent CTA per SM walks a list of work items; an item is 256 query rows of one
-//     (batch, head): two 128-row tiles that ping-pong, so the tensor core works on one tile while
-//     the other tile's softmax runs;
+//   * one persistent CTA per SM walks a list of work items; an item is 256 query rows of one batch element and kv
+//     head - up to four query heads that share the kv head, interleaved token by token - as two 128-row tiles that
+//     ping-pong, so the tensor core works on one tile while the other tile's softmax runs;
 //   * warp 0 is the TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a ring of 128-byte
 //     swizzled shared-memory slots, each guarded by a full/empty mbarrier pair. Loads are plain
 //     per-CTA tensor loads (one CTA, one destination); K/V reuse between the CTAs of a kv head comes
@@ -15,12 +15,12 @@
 //   * warp 1 issues every tcgen05.mma from one thread: S_t = Q_t K_j^T (both operands in shared
 //     memory, K-major) into tensor memory, and O_t += P_t V_j with P_t read from tensor memory and
 //     V_j as an MN-major shared-memory operand (no transposition of V anywhere);
-//   * warps 4-7 and 8-11 are the two softmax groups, one thread per query row: they read their S row
-//     from tensor memory once, 64 columns at a time, exponentiate against the reference point the
-//     row already has, keep the running sum in registers and write P back over S as packed 16-bit
-//     values. The reference point moves (and O, the sum and the part of P already written are
-//     rescaled) only when a half-row exceeds it by more than 2^8; the final division by the row sum
-//     absorbs the stale reference point exactly;
+//   * warps 2-5 and 6-9 are the two softmax groups, one thread per query row: they read their S row from tensor
+//     memory once, exponentiate against the reference point the row already has, keep the running sum in registers
+//     and write P back over S as packed 16-bit values, handed over in two pieces so that P V starts under the last
+//     exponentials. The reference point moves (and O and the sum are rescaled) only when a row exceeds it by more
+//     than 2^8; the final division by the row sum absorbs the stale reference point exactly;
+//   * bf16: one or two more warps rewrite each V tile in shared memory as fp16 (see PvFormat);
 //   * tensor memory: S_0 | S_1 | O_0 | O_1, 128 (or D) fp32 columns each, 512 columns in total;
 //   * head dims above 128 leave room for one query tile only (O needs 256 columns). There the scores of
 //     64-key tiles are double-buffered instead: S(j+1) is computed while the softmax of tile j runs, and
@@ -63,10 +63,10 @@ __device__ __forceinline__ float2 Unpack2<__half>(uint32_t v) {
 // bf16 inputs: the probabilities are handed to the P V product as fp16, not bf16. They lie in [0, 2^8], where fp16
 // resolves 2^-11 relative against 2^-8 - with bf16 the rounding of P alone costs about 1e-3 of relative L2 error in
 // the output. The tensor core wants both operands of one product in the same 16-bit format (a descriptor that mixes
-// them raises "illegal instruction" on sm_100a), so for bf16 inputs a small kernel first rewrites V as fp16 into a
-// stream-ordered temporary (values beyond the fp16 range saturate) and the prefill kernel reads V from there.
-// (Rewriting the V tiles in shared memory by the two idle warps was measured too: 7 % slower than this, because
-// the extra instructions land on two of the four schedulers the softmax warps run on.)
+// them raises "illegal instruction" on sm_100a), so for bf16 inputs V is rewritten as fp16 in shared memory, tile by
+// tile, by warps that do nothing else (values beyond the fp16 range saturate). A copy of V made by a kernel of its own
+// ahead of the launch is no faster at the largest sizes (B=4, S=4096, D=128: 15 us of copying and a 5 us gap in 537 us,
+// against 523 us) and costs a short prompt a second launch and an allocation (S=203: 35 against 27 us).
 template <typename T>
 struct PvFormat {
     using type = __half;
@@ -86,7 +86,7 @@ struct FlashGeom {
     static constexpr int kQTileBytes = kKBlocks * kQBlockBytes;
     static constexpr int kKvTileBytes = kKBlocks * kKvBlockBytes;
     static constexpr int kSlots = (DP == 64) ? 8 : 5;  // K/V ring
-    static constexpr int kBarrierBytes = 384;
+    static constexpr int kBarrierBytes = 512;
     static constexpr int kSmemBytes = 1024 + QT * kQTileBytes + kSlots * kKvTileBytes + kBarrierBytes;
     static constexpr int kSCol = 0;                         // S_t at kSCol + t * 128
     static constexpr int kOCol = 256;                       // O_t at kOCol + t * DP
@@ -130,18 +130,23 @@ __device__ __forceinline__ int TilesFor(int m0, int tokens, int seq_q, int seq_k
 }
 
 // Threads of a CTA: warp 0 TMA and tensor-memory owner, 1 MMA, 2-5 softmax of tile 0, 6-9 softmax of tile 1 (where there
-// is one), and for paged bf16 one more warp that converts V. No idle warps: a softmax thread keeps a whole row of
-// scores in registers, and ten warps may have 200 registers a thread where twelve get 168.
-template <typename T, int QT, bool kPaged>
+// is one), and for bf16 the warps that convert V. Two of them, except for the half-size tiles of D=64 on paged K/V:
+// chunked prefill of 20 sequences, D=128: 390 us with two, 415 with one; D=64: 337 with two, 309 with one (packed
+// D=64, four prompts of 4096: 407 with two, 428 with one).
+template <typename T, int DP, bool kPaged>
+constexpr int ConverterWarps() {
+    return !PvFormat<T>::kConvertV ? 0 : kPaged && DP == 64 ? 1 : 2;
+}
+template <typename T, int DP, int QT, bool kPaged>
 constexpr int FlashThreads() {
-    return 32 * (2 + 4 * QT + (kPaged && PvFormat<T>::kConvertV ? 1 : 0));
+    return 32 * (2 + 4 * QT + ConverterWarps<T, DP, kPaged>());
 }
 
 // kVarlen: the work list comes from the (sequence, query block) table of a packed ragged batch; otherwise it is
 // computed from the dense [B, H, S, D] geometry and every per-sequence quantity is a launch constant.
 // kPaged (only with kVarlen): K and V of a sequence are scattered over the pages of a KV pool.
 template <typename T, int DP, int QT, int BN, bool kVarlen, bool kPaged = false>
-__global__ void __launch_bounds__(FlashThreads<T, QT, kPaged>(), 1)
+__global__ void __launch_bounds__(FlashThreads<T, DP, QT, kPaged>(), 1)
 flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const FlashKernelParams p) {
     using G = FlashGeom<DP, QT, BN>;
@@ -163,15 +168,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     constexpr int kQEmpty = kODone + 2;             // [2]
     constexpr int kOFree = kQEmpty + 2;             // [2]
     constexpr int kPLast = kOFree + 2;              // [2]
-    constexpr int kVReady = kPLast + 2;             // [kSlots] paged bf16: V tile rewritten as fp16 in place
+    constexpr int kVReady = kPLast + 2;             // [kSlots] bf16: V tile rewritten as fp16 in place
     constexpr int kNumBars = kVReady + G::kSlots;
-    // P and V enter the P V product as fp16 also for bf16 inputs (PvFormat). Contiguous V comes from an fp16 copy made
-    // before the launch; the pages of a pool are rewritten tile by tile in shared memory by warps 2 and 3 instead
-    // (a copy of the pool would cost more than the prefill), at the price of some issue slots of two schedulers.
     using PT = typename PvFormat<T>::type;
-    constexpr bool kCvtInKernel = kPaged && PvFormat<T>::kConvertV;
-    constexpr int kConverterThreads = 32;
-    constexpr int kConverterWarp = 2 + 4 * QT;
+    constexpr bool kCvtInKernel = PvFormat<T>::kConvertV;
+    constexpr int kConverterThreads = 32 * ConverterWarps<T, DP, kPaged>();
+    constexpr int kFirstConverter = 2 + 4 * QT;
     // P is handed over in two pieces: the first kPEarly keys let P V start while the rest is still in the softmax
     constexpr int kPEarly = BN == 128 ? 96 : 32;
     static_assert(!kPaged || kVarlen, "paged K/V runs on the packed work list");
@@ -437,8 +439,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (ElectOne()) {
             constexpr uint32_t fmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBf16;
             constexpr uint32_t idesc_s = MakeInstrDesc(fmt, fmt, 0, 0, kBlockM, BN);  // Q K^T: both K-major
-            // P V: V is MN-major; both operands in the P V format (fp16 also for bf16 inputs, see PvFormat: V then
-            // comes from the fp16 copy map_v points at)
+            // P V: V is MN-major; both operands in the P V format (fp16 also for bf16 inputs, see PvFormat)
             constexpr uint32_t fmt_pv = PvFormat<T>::kConvertV ? kFmtF16 : fmt;
             constexpr uint32_t idesc_o = MakeInstrDesc(fmt_pv, fmt_pv, 0, 1, kBlockM, DP);
             // Descriptors are built once and advanced by compile-time constants, so that issuing one
@@ -462,8 +463,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     else MmaSS<true>(d, a0 + qa, b0 + kb, idesc_s);
                 }
             };
-            // waits for the second piece of P (barrier `last`, parity `parity`) half-way
-            auto issue_pv = [&](int t, uint32_t slot, bool first, uint32_t last, uint32_t parity) {
+            // waits for the second piece of P (barriers `sync`, parity `parity`) half-way
+            auto issue_pv = [&](int t, uint32_t slot, bool first, int sync, uint32_t parity) {
                 const uint64_t b0 = vmajor_hi | ((ring_smem + slot * G::kKvTileBytes) >> 4);
                 const uint32_t a = kDoubleS ? s_tmem_db : s_tmem[t];
 #pragma unroll
@@ -472,7 +473,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (ks == 0) MmaTSFlag(o_tmem[t], a, b0, idesc_o, first ? 0u : 1u);
                     else MmaTS<true>(o_tmem[t], a + ks * 8, b0 + ks * (2048 >> 4), idesc_o);
                 }
-                if (!MbarWait(last, parity, abort_flag)) return false;
+                if (!MbarWait(bar(kPLast + sync), parity, abort_flag)) return false;
                 TcFenceAfter();
 #pragma unroll
                 for (int ks = kPEarly / 16; ks < BN / 16; ++ks) {
@@ -483,8 +484,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             uint32_t q_uses[2] = {0, 0};    // items finished per query buffer
             uint32_t steps[2] = {0, 0};     // KV tiles processed per query tile (phase of s_full / p_full / o_done)
             uint32_t kv_base = 0;           // ring position of this item's K_0
-            uint32_t v_uses[G::kSlots] = {};  // V tiles consumed per ring slot (phase of v_ready)
+            uint32_t v_parity = 0;          // bit s: phase of v_ready[s]
             bool ok = true;
+            auto v_ready = [&](uint32_t slot) {
+                const uint32_t parity = (v_parity >> slot) & 1u;
+                v_parity ^= 1u << slot;
+                return MbarWait(bar(kVReady + slot), parity, abort_flag);
+            };
             if constexpr (kDoubleS) {
                 // single query tile, two score buffers: S(0), S(1), then P(j) V_j followed by S(j+2) into the buffer
                 // P(j) came from (same in-order stream, so the overwrite happens after the read)
@@ -493,7 +499,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     *slot = kv_base % G::kSlots;
                     const uint32_t phase = (kv_base / G::kSlots) & 1u;
                     ++kv_base;
-                    if (kCvtInKernel && is_v) return MbarWait(bar(kVReady + *slot), v_uses[*slot]++ & 1u, abort_flag);
+                    if (kCvtInKernel && is_v) return v_ready(*slot);
                     return MbarWait(bar(kKvFull + *slot), phase, abort_flag);
                 };
                 for (int r = 0; r < rounds && ok; ++r) {
@@ -523,7 +529,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (!ok) break;
                         TcFenceAfter();
                         s_tmem_db = tmem_base + G::kSCol + buf * 64;
-                        ok = issue_pv(0, slot, j == 0, bar(kPLast + buf), p_parity);
+                        ok = issue_pv(0, slot, j == 0, buf, p_parity);
                         if (!ok) break;
                         MmaCommit(bar(kODone + buf));
                         MmaCommit(bar(kKvEmpty + slot));
@@ -565,7 +571,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int j = 0; j < w.n_max && ok; ++j) {
                     const int it_v = 2 * j + 1;
                     const int it_k = 2 * j + 2;
-                    if (kCvtInKernel) ok = MbarWait(bar(kVReady + slot_of(it_v)), v_uses[slot_of(it_v)]++ & 1u, abort_flag);
+                    if (kCvtInKernel) ok = v_ready(slot_of(it_v));
                     else ok = MbarWait(bar(kKvFull + slot_of(it_v)), phase_of(it_v), abort_flag);
                     if (ok && j + 1 < w.n_max) ok = MbarWait(bar(kKvFull + slot_of(it_k)), phase_of(it_k), abort_flag);
                     if (!ok) break;
@@ -576,7 +582,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (ok && j == 0 && q_uses[t] > 0) ok = MbarWait(bar(kOFree + t), (q_uses[t] - 1) & 1u, abort_flag);
                         if (!ok) break;
                         TcFenceAfter();
-                        ok = issue_pv(t, slot_of(it_v), j == 0, bar(kPLast + t), steps[t] & 1u);
+                        ok = issue_pv(t, slot_of(it_v), j == 0, t, steps[t] & 1u);
                         if (!ok) break;
                         MmaCommit(bar(kODone + t));
                         ++steps[t];
@@ -597,8 +603,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             failed = !ok;
         }
-    } else if (kCvtInKernel && warp == kConverterWarp) {
-        // ================================ V converter (one warp, paged bf16) ========================
+    } else if (kCvtInKernel && warp >= kFirstConverter) {
+        // ================================ V converter (bf16) ========================================
         // Walks the ring in the producer's order; every V tile is rewritten in place from bf16 to fp16 once its
         // bytes have landed, then handed to the MMA thread through v_ready. K tiles are not touched.
         uint32_t kv_loads = 0;
@@ -628,7 +634,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 if (!ok) break;
                 uint4* tile = reinterpret_cast<uint4*>(smem + (ring_smem - smem_base) + slot * G::kKvTileBytes);
 #pragma unroll 8
-                for (int c = lane; c < G::kKvTileBytes / 16; c += kConverterThreads) {
+                for (int c = threadIdx.x - 32 * kFirstConverter; c < G::kKvTileBytes / 16; c += kConverterThreads) {
                     uint4 x = tile[c];
                     uint32_t* word = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
@@ -713,64 +719,93 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         }
                     }
                 }
-                float mx4[4];
+                {
+                    float mx4[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(__uint_as_float(sc[0][e]), __uint_as_float(sc[0][4 + e]));
+                    for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(__uint_as_float(sc[0][e]), __uint_as_float(sc[0][4 + e]));
 #pragma unroll
-                for (int i = 8; i < BN; i += 8) {
+                    for (int i = 8; i < BN; i += 8) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        mx4[e] = Max3(mx4[e], __uint_as_float(sc[i / 32][i % 32 + e]), __uint_as_float(sc[i / 32][i % 32 + 4 + e]));
-                    }
-                }
-                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0
-                const bool move = mx > m_ref + kRescaleThreshold;  // false for a fully masked row (-inf)
-                if (__any_sync(0xffffffffu, move)) {
-                    const float alpha = move ? Exp2(m_ref - mx) : 1.0f;  // m_ref = -inf -> 0
-                    if (j > 0) {
-                        ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + prev_sync), prev_phase, abort_flag));
-                        if (!ok) break;
-                        TcFenceAfter();
-#pragma unroll 1
-                        for (int cblk = 0; cblk < DP / 16; ++cblk) {
-                            uint32_t r[16];
-                            TmemLd16(o_addr + cblk * 16, r);
-                            TmemWaitLd();
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                            TmemSt16(o_addr + cblk * 16, r);
+                        for (int e = 0; e < 4; ++e) {
+                            mx4[e] = Max3(mx4[e], __uint_as_float(sc[i / 32][i % 32 + e]), __uint_as_float(sc[i / 32][i % 32 + 4 + e]));
                         }
                     }
-                    l_sum *= alpha;
-                    if (move) m_ref = mx;
+                    const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0
+                    const bool move = mx > m_ref + kRescaleThreshold;  // false for a fully masked row (-inf)
+                    if (__any_sync(0xffffffffu, move)) {
+                        const float alpha = move ? Exp2(m_ref - mx) : 1.0f;  // m_ref = -inf -> 0
+                        if (j > 0) {
+                            ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + prev_sync), prev_phase, abort_flag));
+                            if (!ok) break;
+                            TcFenceAfter();
+#pragma unroll 1
+                            for (int cblk = 0; cblk < DP / 16; ++cblk) {
+                                uint32_t r[16];
+                                TmemLd16(o_addr + cblk * 16, r);
+                                TmemWaitLd();
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+                                TmemSt16(o_addr + cblk * 16, r);
+                            }
+                        }
+                        l_sum *= alpha;
+                        if (move) m_ref = mx;
+                    }
                 }
-                const float neg_m = (m_ref == -CUDART_INF_F) ? 0.0f : -m_ref;
+                // Exponentials of columns [32 * first, 32 * end): P to tensor memory, returns their sum. With kBehind the
+                // additions and conversions of a batch of 8 come behind the exponentials of the next one: a warp alone on
+                // its scheduler takes 1190 clocks for 128 exponentials that way and 1331 when it waits for each batch
+                // (1030 is the rate of the special-function unit), two warps 2070 and 2110. D=128, where the groups meet
+                // the products half of the time, gains 2 % (528 against 535 us at B=4, S=4096); D=64, where they mostly
+                // run side by side, loses 10 % (359 against 322 us at B=3, S=2900).
+                constexpr bool kBehind = DP == 128;
                 const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
-                const float2 shift2 = make_float2(neg_m, neg_m);
-                float2 sum_a = make_float2(0.0f, 0.0f), sum_b = sum_a;
+                float2 sum[4];
 #pragma unroll
-                for (int c = 0; c < BN / 32; ++c) {
+                for (int e = 0; e < 4; ++e) sum[e] = make_float2(0.0f, 0.0f);
+                auto fold_sum = [&] {
+                    l_sum += ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y)) + ((sum[2].x + sum[2].y) + (sum[3].x + sum[3].y));
+                };
+                auto exponentials = [&](int first, int end) {
+                    const float neg_m = (m_ref == -CUDART_INF_F) ? 0.0f : -m_ref;
+                    const float2 shift2 = make_float2(neg_m, neg_m);
+                    float2 x[2][4];
                     uint32_t pk[16];
+                    constexpr int kLag = kBehind ? 1 : 0;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        const float2 xa = Fma2(make_float2(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, shift2);
-                        const float2 xb = Fma2(make_float2(__uint_as_float(sc[c][i + 2]), __uint_as_float(sc[c][i + 3])), scale2, shift2);
-                        const float2 ea = make_float2(Exp2(xa.x), Exp2(xa.y));
-                        const float2 eb = make_float2(Exp2(xb.x), Exp2(xb.y));
-                        sum_a = Add2(sum_a, ea);
-                        sum_b = Add2(sum_b, eb);
-                        pk[i / 2] = Pack2<PT>(ea.x, ea.y);
-                        pk[i / 2 + 1] = Pack2<PT>(eb.x, eb.y);
+                    for (int b = 0; b < BN / 8 + kLag; ++b) {
+                        if (b < 4 * first || b >= 4 * end + kLag) continue;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (b < 4 * end) {
+                                x[b & 1][e] = Fma2(make_float2(__uint_as_float(sc[b / 4][(b % 4) * 8 + 2 * e]), __uint_as_float(sc[b / 4][(b % 4) * 8 + 2 * e + 1])), scale2, shift2);
+                                x[b & 1][e] = make_float2(Exp2(x[b & 1][e].x), Exp2(x[b & 1][e].y));
+                            }
+                            const int d = b - kLag;
+                            if (d >= 4 * first) {
+                                sum[kBehind ? e : e & 1] = Add2(sum[kBehind ? e : e & 1], x[d & 1][e]);
+                                pk[(d % 4) * 4 + e] = Pack2<PT>(x[d & 1][e].x, x[d & 1][e].y);
+                            }
+                        }
+                        if (b - kLag >= 4 * first && (b - kLag) % 4 == 3) TmemSt16(s_addr + (b - kLag) / 4 * 16, pk);
                     }
-                    TmemSt16(s_addr + c * 16, pk);
-                    if ((c + 1) * 32 == kPEarly || c + 1 == BN / 32) {
-                        TmemWaitSt();
-                        TcFenceBefore();
-                        __syncwarp();
-                        if (lane == 0) MbarArrive(bar((c + 1 == BN / 32 ? kPLast : kPFull) + sync));
-                    }
+                };
+                auto hand_over = [&](uint32_t barrier) {
+                    TmemWaitSt();
+                    TcFenceBefore();
+                    __syncwarp();
+                    if (lane == 0) MbarArrive(barrier);
+                };
+                exponentials(0, kPEarly / 32);
+                hand_over(bar(kPFull + sync));
+                if (kBehind) {  // eight registers less across the second piece
+                    fold_sum();
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[e] = make_float2(0.0f, 0.0f);
                 }
-                l_sum += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+                exponentials(kPEarly / 32, BN / 32);
+                hand_over(bar(kPLast + sync));
+                fold_sum();
             }
             if (!ok) break;
 
@@ -829,65 +864,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
 }
 
-// V [batch, heads, seq, D] (any strides, bf16) -> compact fp16 [batch, heads, seq, D]; 8 elements per thread.
-__global__ void __launch_bounds__(256) flash_v_to_f16_kernel(const __nv_bfloat16* __restrict__ v, __half* __restrict__ out,
-                                                              int64_t batch, int64_t heads, int64_t seq, int64_t head_dim,
-                                                              int64_t sb, int64_t sh, int64_t ss) {
-    const int64_t chunks_per_row = head_dim / 8;
-    const int64_t total = batch * heads * seq * chunks_per_row;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        int64_t rest = i;
-        const int64_t c = rest % chunks_per_row;
-        rest /= chunks_per_row;
-        const int64_t s = rest % seq;
-        rest /= seq;
-        const int64_t h = rest % heads;
-        const int64_t b = rest / heads;
-        uint4 x = *reinterpret_cast<const uint4*>(v + b * sb + h * sh + s * ss + c * 8);
-        uint32_t* word = reinterpret_cast<uint32_t*>(&x);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = Unpack2<__nv_bfloat16>(word[e]);
-            // one instruction for both lanes; values beyond the fp16 range saturate instead of becoming inf
-            asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(word[e]) : "f"(f.y), "f"(f.x));
-        }
-        reinterpret_cast<uint4*>(out)[i] = x;
-    }
-}
-
 // ---- host side -----------------------------------------------------------------------------------------
 constexpr int kMaxStatusDevices = 64;
-
-// Stream-ordered temporaries come from a pool of this library's own (one per device, created on first use) that keeps
-// what is freed: the default pool hands its memory back to the driver at every synchronisation, after which the next
-// allocation costs a trip to the driver again.
-cudaMemPool_t TemporaryPool() {
-    static std::mutex mu;
-    static cudaMemPool_t pools[kMaxStatusDevices] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxStatusDevices) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    std::lock_guard<std::mutex> lock(mu);
-    if (pools[device] == nullptr) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        unsigned long long keep = ~0ull;
-        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
-        pools[device] = pool;
-    }
-    return pools[device];
-}
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1080,38 +1058,10 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
                              static_cast<int>(paged->block_size), "v pool")) return rc;
     } else
     if (int rc = MakeMap(&map_k, f.k, f.dtype_id, f.head_dim, f.seq_kv, f.num_kv_heads, f.batch, f.k_ss, f.k_sh, f.k_sb, BN, "k")) return rc;
-    // bf16: V goes through an fp16 copy (PvFormat). The copy is a stream-ordered temporary, released behind the launch.
-    struct Temporary {
-        void* ptr = nullptr;
-        cudaStream_t stream = nullptr;
-        ~Temporary() {
-            if (ptr != nullptr && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
-        }
-    } v16;
-    if (paged != nullptr) {
-        // map_v is set above: the pool is read in place, in the input format
-    } else if (PvFormat<T>::kConvertV) {
-        if (!Aligned16(f.v) || f.v_sb % 8 != 0 || f.v_sh % 8 != 0 || f.v_ss % 8 != 0 || f.head_dim % 8 != 0) {
+    if (paged == nullptr) {
+        if (PvFormat<T>::kConvertV && (!Aligned16(f.v) || f.v_sb % 8 != 0 || f.v_sh % 8 != 0 || f.v_ss % 8 != 0)) {
             return Fail(SCA_INVALID_ARGUMENT, "flash attention: v must be 16-byte aligned with strides that are multiples of 8 elements");
         }
-        const int64_t elements = f.batch * f.num_kv_heads * f.seq_kv * f.head_dim;
-        v16.stream = stream;
-        cudaMemPool_t pool = TemporaryPool();
-        const cudaError_t e = pool != nullptr ? cudaMallocFromPoolAsync(&v16.ptr, static_cast<size_t>(elements) * 2, pool, stream)
-                                              : cudaMallocAsync(&v16.ptr, static_cast<size_t>(elements) * 2, stream);
-        if (e != cudaSuccess) {
-            v16.ptr = nullptr;
-            cudaGetLastError();
-            return FailCuda(e, "flash attention: cudaMallocAsync(fp16 copy of V)");
-        }
-        const int64_t threads_needed = elements / 8;
-        const unsigned blocks = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((threads_needed + 255) / 256, static_cast<int64_t>(SmCount()) * 16)));
-        flash_v_to_f16_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(f.v), static_cast<__half*>(v16.ptr),
-                                                          f.batch, f.num_kv_heads, f.seq_kv, f.head_dim, f.v_sb, f.v_sh, f.v_ss);
-        if (int rc = CheckLaunch("flash_v_to_f16_kernel", stream)) return rc;
-        if (int rc = MakeMap(&map_v, v16.ptr, SCA_DTYPE_F16, f.head_dim, f.seq_kv, f.num_kv_heads, f.batch, f.head_dim,
-                             f.seq_kv * f.head_dim, f.num_kv_heads * f.seq_kv * f.head_dim, BN, "v (fp16 copy)")) return rc;
-    } else {
         if (int rc = MakeMap(&map_v, f.v, f.dtype_id, f.head_dim, f.seq_kv, f.num_kv_heads, f.batch, f.v_ss, f.v_sh, f.v_sb, BN, "v")) return rc;
     }
 
@@ -1144,7 +1094,7 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         return Fail(SCA_INVALID_ARGUMENT, "flash attention: grid of " + std::to_string(ctas) + " blocks is out of range");
     }
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ctas, SmCount()));  // one persistent CTA per SM
-    const unsigned threads = paged != nullptr ? FlashThreads<T, QT, true>() : FlashThreads<T, QT, false>();
+    const unsigned threads = paged != nullptr ? FlashThreads<T, DP, QT, true>() : FlashThreads<T, DP, QT, false>();
     if (paged != nullptr) {
         p.page_table = paged->page_table;
         p.max_blocks_per_seq = static_cast<int>(paged->max_blocks_per_seq);
