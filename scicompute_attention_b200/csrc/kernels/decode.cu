@@ -17,7 +17,9 @@
 //     consumed in a permuted order that both operands agree on, which is why no ldmatrix and no
 //     transposition of V is needed; XOR swizzles keep those loads bank-conflict free;
 //   * page tables are resolved once per token row by 16 lanes (one table read per row, broadcast
-//     by shuffle), never per element.
+//     by shuffle), never per element;
+//   * calls that do not fill the machine run in one launch: a cluster of CTAs takes each (sequence, kv head, head
+//     chunk) and merges through distributed shared memory (decode_cluster_kernel).
 //
 // Algorithmic HBM traffic per token and kv head: 2 * D * sizeof(T) bytes (K row + V row), read once.
 #include <algorithm>
@@ -33,6 +35,7 @@ constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr int kTile = 16;   // tokens per warp step (k extent of the P.V product)
 constexpr int kStages = 3;  // ring depth per warp
+constexpr int kMaxCluster = 8;  // CTAs that may share one (sequence, kv head, head chunk) in the one-launch kernel
 
 template <int D>
 struct DecodeGeom {
@@ -46,7 +49,7 @@ struct DecodeGeom {
     static constexpr int kKRounds = D / 32;         // 16-byte K loads per lane and token tile half
     static constexpr int kVRounds = (D + 63) / 64;  // groups of eight n8 output tiles
     static_assert(D % 32 == 0, "head_dim must be a multiple of 32");
-    static_assert(kWarpBytes >= (32 + 16 * D) * 4, "merge staging must fit in the warp's ring");
+    static_assert(kWarpBytes >= 2 * (32 + 16 * D) * 4, "merge staging and the CTA's partial must fit in a warp's ring");
 };
 
 __device__ __forceinline__ float2 Unpack2Bf16(uint32_t v) {
@@ -82,8 +85,13 @@ __device__ __forceinline__ int64_t StepsFor(int64_t len) {
 }
 
 // One segment = tokens [j_begin, j_end) of one (sequence, kv head, head chunk): streams K/V once, keeps the running
-// softmax state of up to 16 query heads, and writes one (m, l, O) partial per head into `slot`.
-template <typename T, int D, bool kPaged, bool kHi>
+// softmax state of up to 16 query heads, and leaves one (m, l, O) partial per head: in `slot` of the partial arrays, or
+// (kToShared) in this CTA's shared memory at CtaPartial<D>(smem): m[16] in the log2 domain, l[16], O[16][D].
+template <int D>
+__device__ __forceinline__ float* CtaPartial(unsigned char* smem) {
+    return reinterpret_cast<float*>(smem) + 32 + 16 * D;  // behind warp 0's staging area, inside its ring
+}
+template <typename T, int D, bool kPaged, bool kHi, bool kToShared = false>
 __device__ __forceinline__ void DecodeSegment(const ScaDecodeFwdParams& p, unsigned char* smem, const int64_t b,
                                               const int hk, const int hc, const int64_t j_begin, const int64_t j_end,
                                               const int slot) {
@@ -356,6 +364,15 @@ __device__ __forceinline__ void DecodeSegment(const ScaDecodeFwdParams& p, unsig
             acc += wm[32 + row * D + d] * wgt;
             l_all += wm[16 + row] * wgt;
         }
+        if (kToShared) {
+            float* partial = CtaPartial<D>(smem);
+            partial[32 + row * D + d] = acc;
+            if (d == 0) {
+                partial[row] = m_all;
+                partial[16 + row] = l_all;
+            }
+            continue;
+        }
         const int64_t flat = (b * p.num_heads + head0 + row) * p.num_splits + slot;
         p.partial_o[flat * D + d] = acc;
         if (d == 0) {
@@ -528,6 +545,69 @@ decode_partial_kernel(const ScaDecodeFwdParams p, const int head_chunks) {
     }
 }
 
+__device__ __forceinline__ uint32_t ClusterRank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void ClusterBarrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// A float in the shared memory of CTA `rank` of this cluster, at this CTA's address `addr`.
+__device__ __forceinline__ float LoadFromRank(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
+// Decode of a problem that does not fill the machine, in one launch: the CTAs of a cluster split one (sequence, kv head,
+// head chunk) and merge their partials through distributed shared memory. Bound by latency - a step or two of K/V per
+// CTA, then the exchange - so what counts is that there is no second kernel and no trip through memory in between.
+template <typename T, int D, bool kPaged, bool kHi>
+__global__ void __launch_bounds__(kThreads)
+decode_cluster_kernel(const ScaDecodeFwdParams p, const int head_chunks, const int cluster) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int columns = static_cast<int>(p.num_kv_heads) * head_chunks;
+    const int rank = static_cast<int>(ClusterRank());
+    const int unit = static_cast<int>(blockIdx.x) / cluster;
+    const int64_t b = unit / columns;
+    const int hk = (unit % columns) / head_chunks, hc = (unit % columns) % head_chunks;
+    const int64_t len = SeqLen<kPaged>(p, b);
+    const int64_t steps = StepsFor(len);
+    const int64_t share = (steps + cluster - 1) / cluster;
+    const int64_t t0 = rank * share < steps ? rank * share : steps;
+    const int64_t t1 = t0 + share < steps ? t0 + share : steps;
+    const int64_t j_end = t1 * kSpan < len ? t1 * kSpan : len;
+    DecodeSegment<T, D, kPaged, kHi, true>(p, smem, b, hk, hc, t0 * kSpan, j_end, 0);
+    ClusterBarrier();
+    const int group = static_cast<int>(p.num_heads / p.num_kv_heads);
+    const int head0 = hk * group + hc * 16;
+    const int total = min(16, group - hc * 16) * D;
+    const uint32_t partial = SmemAddr(CtaPartial<D>(smem));
+    T* out = reinterpret_cast<T*>(p.out) + b * p.o_stride.s_b;
+    for (int item = rank * kThreads + threadIdx.x; item < total; item += cluster * kThreads) {
+        const int row = item / D, d = item % D;
+        float m[kMaxCluster], l_all = 0.0f, acc = 0.0f, m_all = -CUDART_INF_F;
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+            m[r] = r < cluster ? LoadFromRank(partial + 4 * row, r) : -CUDART_INF_F;
+            m_all = fmaxf(m_all, m[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+            if (m[r] == -CUDART_INF_F) continue;
+            const float weight = Exp2(m[r] - m_all);
+            l_all += LoadFromRank(partial + 4 * (16 + row), r) * weight;
+            acc += LoadFromRank(partial + 4 * (32 + row * D + d), r) * weight;
+        }
+        const float inv = l_all > 0.0f ? 1.0f / l_all : 0.0f;
+        out[(head0 + row) * p.o_stride.s_h + d] = FromFloat<T>(acc * inv);
+    }
+    ClusterBarrier();  // nobody leaves while its shared memory is being read
+}
+
 // Where the parts of one output row live: element (row, part) of m / l is at
 // m[row * m_row_stride + part * m_part_stride]; its O vector starts at
 // o[row * o_row_stride + part * o_part_stride].
@@ -601,26 +681,105 @@ void LaunchMerge(unsigned blocks, cudaStream_t stream, bool after_partial, const
     cudaLaunchKernelEx(&cfg, decode_merge_kernel<T, kTriples>, src, rows, parts, head_dim, out, heads, o_sb, o_sh);
 }
 
+cudaLaunchConfig_t ClusterConfig(unsigned grid, int cluster, int smem_bytes, cudaStream_t stream, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+    cfg.stream = stream;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// CTAs of the decode kernels that stay resident together.
+template <typename T, int D, bool kPaged, bool kHi>
+int64_t ResidentCtas() {
+    static int resident_per_sm = 0;  // per instantiation; the same on every device of one model
+    if (resident_per_sm == 0) {
+        int n = 0;
+        // the query answers for the shared memory the kernel is allowed at that point
+        const void* fn = reinterpret_cast<const void*>(&decode_partial_kernel<T, D, kPaged, kHi>);
+        if (EnsureDynamicSmem(fn, DecodeGeom<D>::kSmemBytes, "decode_partial_kernel") != SCA_OK ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_partial_kernel<T, D, kPaged, kHi>, kThreads,
+                                                          DecodeGeom<D>::kSmemBytes) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = 1;
+        }
+        resident_per_sm = n;
+    }
+    return static_cast<int64_t>(SmCount()) * resident_per_sm;
+}
+// Steps of the longest sequence the call may hold, as far as the host knows.
+template <bool kPaged>
+int64_t MostSteps(const ScaDecodeFwdParams& p) {
+    const int64_t upper = kPaged ? p.max_blocks_per_seq * p.block_size : p.seq_kv;
+    return std::max<int64_t>(1, (std::min(p.seq_kv, upper) + kSpan - 1) / kSpan);
+}
+
+// Clusters of `cluster` CTAs of decode_cluster_kernel that run at the same time (0 when the device cannot say).
+template <typename T, int D, bool kPaged, bool kHi>
+int64_t ResidentClusters(int cluster) {
+    static int resident[kMaxCluster + 1] = {};  // per instantiation; the same on every device of one model
+    if (resident[cluster] == 0) {
+        cudaLaunchAttribute attr{};
+        cudaLaunchConfig_t cfg = ClusterConfig(static_cast<unsigned>(cluster), cluster, DecodeGeom<D>::kSmemBytes, nullptr, &attr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, decode_cluster_kernel<T, D, kPaged, kHi>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        resident[cluster] = n > 0 ? n : -1;
+    }
+    return resident[cluster] > 0 ? resident[cluster] : 0;
+}
+
+// Whether the one-launch kernel is the faster one for `units` (sequence, kv head, head chunk) columns of `steps` steps
+// (the longest) on clusters of `cluster` CTAs. Both times in us, fitted to graph-timed calls of D=128 on a B200 (one-wave
+// schedule with its merge / one launch): B=1, S=1000 10.9 / 6.2, S=4000 18.5 / 11.1, S=16000 27.5 / 28.5, S=60000 57 /
+// 90; B=4, S=4000 21.0 / 16.5; B=16, S=2000 29.9 / 27.5, paged with lengths from 250 to 2000 25.6 / 27.7; paged B=4, 500
+// to 4000 22.6 / 16.9, B=8 26.9 / 27.2. A step costs more the more CTAs share the memory; the schedule works on what a
+// ragged batch holds (0.55 of the bound is assumed), a cluster waits for the longest sequence.
+bool ClusterIsFaster(int64_t units, int64_t steps, int cluster, int64_t resident, bool ragged) {
+    const double busy = static_cast<double>(units * cluster) / resident;
+    const double one_launch = 4.8 + static_cast<double>((steps + cluster - 1) / cluster) * (0.55 + 1.1 * busy);
+    const double wave = static_cast<double>(units * steps) * (ragged ? 0.55 : 1.0) / resident;
+    return one_launch < 11.5 + 1.55 * std::max(1.0, wave);
+}
+
+// Launches decode_cluster_kernel if it is the kernel for this call (*taken).
+template <typename T, int D, bool kPaged, bool kHi>
+int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, bool* taken) {
+    const int64_t units = p.batch * p.num_kv_heads * head_chunks;
+    const void* fn = reinterpret_cast<const void*>(&decode_cluster_kernel<T, D, kPaged, kHi>);
+    if (int rc = EnsureDynamicSmem(fn, DecodeGeom<D>::kSmemBytes, "decode_cluster_kernel")) return rc;
+    const int64_t steps = MostSteps<kPaged>(p);
+    const int64_t resident = ResidentCtas<T, D, kPaged, kHi>();
+    // as many CTAs per cluster as let all clusters run at the same time (B=8, S=1000: 11.6 us with 4, 16.4 with 8 in turns)
+    int cluster = kMaxCluster;
+    while (cluster >= 2 && units > ResidentClusters<T, D, kPaged, kHi>(cluster)) cluster /= 2;
+    if (cluster < 2 || !ClusterIsFaster(units, steps, cluster, resident, p.seq_lens != nullptr)) cluster = 0;
+    *taken = cluster > 0;
+    if (!*taken) return SCA_OK;
+    cudaLaunchAttribute attr{};
+    const cudaLaunchConfig_t cfg = ClusterConfig(static_cast<unsigned>(units * cluster), cluster, DecodeGeom<D>::kSmemBytes, stream, &attr);
+    cudaLaunchKernelEx(&cfg, decode_cluster_kernel<T, D, kPaged, kHi>, p, head_chunks, cluster);
+    return CheckLaunch("decode_cluster_kernel", stream);
+}
+
 template <typename T, int D, bool kPaged, bool kHi>
 int LaunchPartial(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream) {
     using G = DecodeGeom<D>;
     const void* fn = reinterpret_cast<const void*>(&decode_partial_kernel<T, D, kPaged, kHi>);
     if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "decode_partial_kernel")) return rc;
     // one wave: as many CTAs as stay resident together, fewer when there is less work than that
-    static int resident_per_sm = 0;  // per instantiation; the same on every device of one model
-    if (resident_per_sm == 0) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_partial_kernel<T, D, kPaged, kHi>, kThreads,
-                                                          G::kSmemBytes) != cudaSuccess || n < 1) {
-            cudaGetLastError();
-            n = 1;
-        }
-        resident_per_sm = n;
-    }
     const int64_t columns = p.num_kv_heads * head_chunks;
-    const int64_t resident = static_cast<int64_t>(SmCount()) * resident_per_sm;
-    const int64_t upper = kPaged ? p.max_blocks_per_seq * p.block_size : p.seq_kv;
-    const int64_t steps = std::max<int64_t>(1, (std::min(p.seq_kv, upper) + kSpan - 1) / kSpan);
+    const int64_t resident = ResidentCtas<T, D, kPaged, kHi>();
+    const int64_t steps = MostSteps<kPaged>(p);
     // CTAs per column: as many as stay resident, never more than the column has steps (or sequences, with one slot)
     const int64_t useful = p.num_splits == 1 ? p.batch : p.batch * steps;
     int64_t blocks;
@@ -634,30 +793,40 @@ int LaunchPartial(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     return CheckLaunch("decode_partial_kernel", stream);
 }
 
+// `merged` (may be null): set when the launch has written the output itself, so that no merge is needed.
+template <typename T, int D, bool kPaged, bool kHi>
+int LaunchOne(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, bool* merged) {
+    if (merged != nullptr) {
+        if (int rc = LaunchCluster<T, D, kPaged, kHi>(p, head_chunks, stream, merged)) return rc;
+        if (*merged) return SCA_OK;
+    }
+    return LaunchPartial<T, D, kPaged, kHi>(p, head_chunks, stream);
+}
+
 template <typename T, int D>
-int LaunchPartialForDim(const ScaDecodeFwdParams& p, cudaStream_t stream) {
+int LaunchPartialForDim(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged) {
     const int group = static_cast<int>(p.num_heads / p.num_kv_heads);
     const int head_chunks = (group + 15) / 16;
     const bool paged = p.page_table != nullptr;
     const bool hi = group > 8;
     if (paged) {
-        return hi ? LaunchPartial<T, D, true, true>(p, head_chunks, stream)
-                  : LaunchPartial<T, D, true, false>(p, head_chunks, stream);
+        return hi ? LaunchOne<T, D, true, true>(p, head_chunks, stream, merged)
+                  : LaunchOne<T, D, true, false>(p, head_chunks, stream, merged);
     }
-    return hi ? LaunchPartial<T, D, false, true>(p, head_chunks, stream)
-              : LaunchPartial<T, D, false, false>(p, head_chunks, stream);
+    return hi ? LaunchOne<T, D, false, true>(p, head_chunks, stream, merged)
+              : LaunchOne<T, D, false, false>(p, head_chunks, stream, merged);
 }
 
 template <typename T>
-int LaunchPartialTyped(const ScaDecodeFwdParams& p, cudaStream_t stream) {
+int LaunchPartialTyped(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged) {
     switch (p.head_dim) {
-        case 32: return LaunchPartialForDim<T, 32>(p, stream);
-        case 64: return LaunchPartialForDim<T, 64>(p, stream);
-        case 96: return LaunchPartialForDim<T, 96>(p, stream);
-        case 128: return LaunchPartialForDim<T, 128>(p, stream);
-        case 160: return LaunchPartialForDim<T, 160>(p, stream);
-        case 192: return LaunchPartialForDim<T, 192>(p, stream);
-        case 256: return LaunchPartialForDim<T, 256>(p, stream);
+        case 32: return LaunchPartialForDim<T, 32>(p, stream, merged);
+        case 64: return LaunchPartialForDim<T, 64>(p, stream, merged);
+        case 96: return LaunchPartialForDim<T, 96>(p, stream, merged);
+        case 128: return LaunchPartialForDim<T, 128>(p, stream, merged);
+        case 160: return LaunchPartialForDim<T, 160>(p, stream, merged);
+        case 192: return LaunchPartialForDim<T, 192>(p, stream, merged);
+        case 256: return LaunchPartialForDim<T, 256>(p, stream, merged);
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT,
@@ -726,14 +895,21 @@ int LaunchMergeOut(const ScaDecodeFwdParams& p, cudaStream_t stream) {
 // fp32 inputs take the SIMT partial kernel (simt.cu); declared here, defined there.
 int LaunchDecodePartialF32(const ScaDecodeFwdParams& p, cudaStream_t stream);
 
-int LaunchDecodePartials(const ScaDecodeFwdParams& p, cudaStream_t stream) {
+int LaunchDecodePartials(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged = nullptr) {
     switch (p.dtype) {
-        case SCA_DTYPE_F16: return LaunchPartialTyped<__half>(p, stream);
-        case SCA_DTYPE_BF16: return LaunchPartialTyped<__nv_bfloat16>(p, stream);
+        case SCA_DTYPE_F16: return LaunchPartialTyped<__half>(p, stream, merged);
+        case SCA_DTYPE_BF16: return LaunchPartialTyped<__nv_bfloat16>(p, stream, merged);
         case SCA_DTYPE_F32: return LaunchDecodePartialF32(p, stream);
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT, "decode: unsupported dtype id");
+}
+
+// Partials and merge, or both in one launch where that is faster.
+int LaunchDecode(const ScaDecodeFwdParams& p, cudaStream_t stream) {
+    bool merged = false;
+    if (int rc = LaunchDecodePartials(p, stream, &merged)) return rc;
+    return merged ? SCA_OK : LaunchMergeOut(p, stream);
 }
 
 }  // namespace sca_b200
@@ -784,8 +960,7 @@ extern "C" int sca_launch_decode_splitk(const ScaDecodeFwdParams* params, void* 
     ClearError();
     if (int rc = ValidateDecode(params, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (int rc = LaunchDecodePartials(*params, s)) return rc;
-    return LaunchMergeOut(*params, s);
+    return LaunchDecode(*params, s);
 }
 
 extern "C" int sca_launch_decode_splitk_paged(const ScaDecodeFwdParams* params, void* stream) {
@@ -820,8 +995,7 @@ extern "C" int sca_launch_paged_attention_ordered(const ScaPagedDecodeParams* pa
     if (int rc = ValidateDecode(&p, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     (void)seq_order;  // the kernel deals out equal shares of the K/V stream itself; the hint has nothing left to improve
-    if (int rc = LaunchDecodePartials(p, s)) return rc;
-    return LaunchMergeOut(p, s);
+    return LaunchDecode(p, s);
 }
 
 extern "C" int sca_launch_paged_attention(const ScaPagedDecodeParams* params, void* stream) {
@@ -915,6 +1089,5 @@ extern "C" int sca_launch_decode_splitk_static(const ScaDecodeFwdParams* params,
     p.partial_o = scratch + 2 * base;
     if (int rc = ValidateDecode(&p, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (int rc = LaunchDecodePartials(p, s)) return rc;
-    return LaunchMergeOut(p, s);
+    return LaunchDecode(p, s);
 }
