@@ -9,7 +9,9 @@ outputs are always freshly allocated contiguous BHSD tensors.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
+import struct
 
 import torch
 
@@ -32,8 +34,10 @@ def dtype_id(dtype: torch.dtype) -> int:
 
 
 def _stream_ptr(stream=None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the handle of torch.cuda.current_stream() without the Stream object around it
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
@@ -124,7 +128,12 @@ def effective_scale(scale, head_dim: int) -> float:
     """cfg.scale > 0 wins, otherwise float(1 / sqrt(double(D))) (reference: api_validate.cpp:31-35)."""
     if scale is not None and scale > 0:
         return float(scale)
-    return float(torch.tensor(1.0 / math.sqrt(float(head_dim)), dtype=torch.float32).item())
+    return _default_scale(head_dim)
+
+
+@functools.lru_cache(maxsize=64)
+def _default_scale(head_dim: int) -> float:
+    return struct.unpack("f", struct.pack("f", 1.0 / math.sqrt(float(head_dim))))[0]  # rounded to fp32
 
 
 # ------------------------------------------------------------------------------------------------
