@@ -141,25 +141,40 @@ __device__ __forceinline__ void DecodeSegment(const ScaDecodeFwdParams& p, unsig
     unsigned char* ring = smem + warp * G::kWarpBytes;
     const uint32_t ring_addr = SmemAddr(ring);
 
-    // Issues the copies of this warp's `tl`-th tile into `stage`; returns the 16-bit token validity.
+    // Paged: this lane's token of the next tile to be issued, as (page of the sequence, offset in the page), moved on by
+    // kSpan tokens per tile without a division, and the page's table entry, fetched one tile ahead so that the copies do
+    // not wait for it.
+    int64_t page = 0, page_step = 0;
+    int offset = 0, offset_step = 0, block_size = 1;
+    int32_t phys_next = -1;
+    auto fetch_entry = [&](int64_t jt) {
+        phys_next = (lane < kTile && jt < j_end && page < p.max_blocks_per_seq) ? __ldg(table_row + page) : -1;
+    };
+    if (kPaged) {
+        block_size = static_cast<int>(p.block_size);
+        const int64_t jt = j_begin + warp * kTile + (lane & (kTile - 1));
+        page = jt / block_size;
+        offset = static_cast<int>(jt - page * block_size);
+        page_step = kSpan / block_size;
+        offset_step = kSpan % block_size;
+        fetch_entry(jt);
+    }
+
+    // Issues the copies of this warp's `tl`-th tile into `stage`, tile after tile; returns the 16-bit token validity.
     auto issue = [&](int tl, int stage) -> uint32_t {
-        const int64_t jt0 = j_begin + static_cast<int64_t>(warp + tl * kWarps) * kTile;
+        const int64_t jt = j_begin + static_cast<int64_t>(warp + tl * kWarps) * kTile + (lane & (kTile - 1));
         int prow = -1;  // row of the pool / the K/V slab; pools stay below 2^31 rows
-        if (lane < kTile) {
-            const int64_t jt = jt0 + lane;
-            if (jt < j_end) {
-                if (kPaged) {
-                    const int64_t logical = jt / p.block_size;
-                    if (logical < p.max_blocks_per_seq) {
-                        const int32_t phys = __ldg(table_row + logical);
-                        if (phys >= 0 && phys < p.num_kv_blocks) {
-                            prow = static_cast<int>(phys * p.block_size + jt % p.block_size);
-                        }
-                    }
-                } else {
-                    prow = static_cast<int>(jt);
-                }
+        if (kPaged) {
+            if (phys_next >= 0 && phys_next < p.num_kv_blocks) prow = phys_next * block_size + offset;
+            page += page_step;
+            offset += offset_step;
+            if (offset >= block_size) {
+                offset -= block_size;
+                ++page;
             }
+            fetch_entry(jt + kSpan);
+        } else if (lane < kTile && jt < j_end) {
+            prow = static_cast<int>(jt);
         }
         const uint32_t mask = __ballot_sync(0xffffffffu, prow >= 0) & 0xffffu;
         const uint32_t k_stage = ring_addr + stage * G::kStageBytes;
