@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kv_ring.cuh"
 #include "sm100.cuh"
 
 namespace sca_b200 {
@@ -160,8 +161,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     auto bar = [&](int i) { return bar_base + 8u * i; };
     // barrier indices
     constexpr int kQFull = 0;                       // [2]
-    constexpr int kKvFull = 2;                      // [kSlots]
-    constexpr int kKvEmpty = kKvFull + G::kSlots;   // [kSlots]
+    constexpr int kKvFull = 2;                      // [2 * kSlots], see RingFullBarrier
+    constexpr int kKvEmpty = kKvFull + 2 * G::kSlots;   // [kSlots]
     constexpr int kSFull = kKvEmpty + G::kSlots;    // [2]
     constexpr int kPFull = kSFull + 2;              // [2]
     constexpr int kODone = kPFull + 2;              // [2]
@@ -170,6 +171,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     constexpr int kPLast = kOFree + 2;              // [2]
     constexpr int kVReady = kPLast + 2;             // [kSlots] bf16: V tile rewritten as fp16 in place
     constexpr int kNumBars = kVReady + G::kSlots;
+    auto full_bar = [&](bool is_v, uint32_t slot) { return bar(kKvFull + RingFullBarrier(is_v, static_cast<int>(slot), G::kSlots)); };
     using PT = typename PvFormat<T>::type;
     constexpr bool kCvtInKernel = PvFormat<T>::kConvertV;
     constexpr int kConverterThreads = 32 * ConverterWarps<T, DP, kPaged>();
@@ -266,8 +268,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             MbarInit(bar(kODone + i), 1);
             MbarInit(bar(kOFree + i), 4);
         }
+        for (int i = 0; i < 2 * G::kSlots; ++i) MbarInit(bar(kKvFull + i), 1);
         for (int i = 0; i < G::kSlots; ++i) {
-            MbarInit(bar(kKvFull + i), 1);
             MbarInit(bar(kKvEmpty + i), 1);
             MbarInit(bar(kVReady + i), kConverterThreads);
         }
@@ -322,23 +324,9 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             const int32_t* row = p.page_table + static_cast<int64_t>(w.seq) * p.max_blocks_per_seq;
             for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                bool is_v;
-                int tile;
-                if (kDoubleS) {
-                    const int n = w.n_max;
-                    const int lead = n > 1 ? 2 : 1;
-                    if (it < lead) {
-                        is_v = false;
-                        tile = it;
-                    } else {
-                        const int f = it - lead, kk = n - lead;
-                        is_v = f >= 2 * kk || (f & 1) == 0;
-                        tile = f < 2 * kk ? (is_v ? (f >> 1) : (f >> 1) + 2) : kk + (f - 2 * kk);
-                    }
-                } else {
-                    is_v = (it & 1) != 0;
-                    tile = it >> 1;
-                }
+                const RingLoad load = RingOrder(it, w.n_max, kDoubleS);
+                const bool is_v = load.is_v;
+                const int tile = load.tile;
                 // page ids of this tile, one per lane
                 const int logical = tile * pages_per_tile + lane;
                 int32_t phys = -1;
@@ -354,7 +342,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     ok = MbarWait(bar(kKvEmpty + slot), phase ^ 1u, abort_flag);
                     if (ok) {
                         if (!is_v) valid_ring[(tiles_before + tile) % kValidRing] = valid;
-                        MbarExpectTx(bar(kKvFull + slot), G::kKvTileBytes);
+                        MbarExpectTx(full_bar(is_v, slot), G::kKvTileBytes);
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -367,7 +355,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (ElectOne()) {
                         for (int kb = 0; kb < G::kKBlocks; ++kb) {
                             TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes + pg * page_bytes, map,
-                                      bar(kKvFull + slot), kb * 64, first_row, w.h_kv, 0);
+                                      full_bar(is_v, slot), kb * 64, first_row, w.h_kv, 0);
                         }
                     }
                 }
@@ -400,35 +388,18 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                     ++q_uses[t];
                 }
-                // ring order = the order the MMA stream consumes the tiles: K_0 V_0 K_1 V_1 ..., or with double-
-                // buffered scores K_0 K_1 V_0 K_2 V_1 K_3 ... (S(j+2) follows P(j) V_j)
                 for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                    bool is_v;
-                    int tile;
-                    if (kDoubleS) {
-                        const int n = w.n_max;
-                        const int lead = n > 1 ? 2 : 1;
-                        if (it < lead) {
-                            is_v = false;
-                            tile = it;
-                        } else {
-                            const int f = it - lead, kk = n - lead;  // kk K tiles still to come, one after each V
-                            is_v = f >= 2 * kk || (f & 1) == 0;
-                            tile = f < 2 * kk ? (is_v ? (f >> 1) : (f >> 1) + 2) : kk + (f - 2 * kk);
-                        }
-                    } else {
-                        is_v = (it & 1) != 0;
-                        tile = it >> 1;
-                    }
+                    const RingLoad load = RingOrder(it, w.n_max, kDoubleS);
                     const uint32_t slot = kv_loads % G::kSlots;
                     const uint32_t phase = (kv_loads / G::kSlots) & 1u;
                     ok = MbarWait(bar(kKvEmpty + slot), phase ^ 1u, abort_flag);
                     if (!ok) break;
-                    MbarExpectTx(bar(kKvFull + slot), G::kKvTileBytes);
-                    const CUtensorMap* map = is_v ? &map_v : &map_k;
+                    const uint32_t full = full_bar(load.is_v, slot);
+                    MbarExpectTx(full, G::kKvTileBytes);
+                    const CUtensorMap* map = load.is_v ? &map_v : &map_k;
                     for (int kb = 0; kb < G::kKBlocks; ++kb) {
-                        TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes, map, bar(kKvFull + slot),
-                                  kb * 64, w.kv_tok0 + tile * BN, w.h_kv, w.b);
+                        TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes, map, full, kb * 64,
+                                  w.kv_tok0 + load.tile * BN, w.h_kv, w.b);
                     }
                 }
             }
@@ -484,23 +455,19 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             uint32_t q_uses[2] = {0, 0};    // items finished per query buffer
             uint32_t steps[2] = {0, 0};     // KV tiles processed per query tile (phase of s_full / p_full / o_done)
             uint32_t kv_base = 0;           // ring position of this item's K_0
-            uint32_t v_parity = 0;          // bit s: phase of v_ready[s]
+            RingPhases k_phases, v_phases;  // of the K barriers and of v_ready (no converter: the V barriers)
             bool ok = true;
+            auto k_landed = [&](uint32_t slot) { return MbarWait(full_bar(false, slot), k_phases.Take(slot), abort_flag); };
             auto v_ready = [&](uint32_t slot) {
-                const uint32_t parity = (v_parity >> slot) & 1u;
-                v_parity ^= 1u << slot;
-                return MbarWait(bar(kVReady + slot), parity, abort_flag);
+                return MbarWait(kCvtInKernel ? bar(kVReady + slot) : full_bar(true, slot), v_phases.Take(slot), abort_flag);
             };
             if constexpr (kDoubleS) {
                 // single query tile, two score buffers: S(0), S(1), then P(j) V_j followed by S(j+2) into the buffer
                 // P(j) came from (same in-order stream, so the overwrite happens after the read)
                 uint32_t buf_uses[2] = {0, 0};  // P tiles consumed per score buffer (phase of p_full)
                 auto next_slot = [&](uint32_t* slot, bool is_v) {
-                    *slot = kv_base % G::kSlots;
-                    const uint32_t phase = (kv_base / G::kSlots) & 1u;
-                    ++kv_base;
-                    if (kCvtInKernel && is_v) return v_ready(*slot);
-                    return MbarWait(bar(kKvFull + *slot), phase, abort_flag);
+                    *slot = kv_base++ % G::kSlots;
+                    return is_v ? v_ready(*slot) : k_landed(*slot);
                 };
                 for (int r = 0; r < rounds && ok; ++r) {
                     const int idx = item_of_round(r);
@@ -551,12 +518,11 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 if (idx < 0) continue;
                 const Item w = decode_item(idx);
                 auto slot_of = [&](int it) { return (kv_base + it) % G::kSlots; };
-                auto phase_of = [&](int it) { return ((kv_base + it) / G::kSlots) & 1u; };
                 for (int t = 0; t < QT && ok; ++t) {
                     if (w.ntiles[t] > 0) ok = MbarWait(bar(kQFull + t), q_uses[t] & 1u, abort_flag);
                 }
                 if (ok && w.n_max > 0) {
-                    ok = MbarWait(bar(kKvFull + slot_of(0)), phase_of(0), abort_flag);
+                    ok = k_landed(slot_of(0));
                     if (ok) {
                         TcFenceAfter();
                         for (int t = 0; t < QT; ++t) {
@@ -571,9 +537,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int j = 0; j < w.n_max && ok; ++j) {
                     const int it_v = 2 * j + 1;
                     const int it_k = 2 * j + 2;
-                    if (kCvtInKernel) ok = v_ready(slot_of(it_v));
-                    else ok = MbarWait(bar(kKvFull + slot_of(it_v)), phase_of(it_v), abort_flag);
-                    if (ok && j + 1 < w.n_max) ok = MbarWait(bar(kKvFull + slot_of(it_k)), phase_of(it_k), abort_flag);
+                    ok = v_ready(slot_of(it_v));
+                    if (ok && j + 1 < w.n_max) ok = k_landed(slot_of(it_k));
                     if (!ok) break;
                     for (int t = 0; t < QT; ++t) {
                         if (j >= w.ntiles[t]) continue;
@@ -608,29 +573,16 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // Walks the ring in the producer's order; every V tile is rewritten in place from bf16 to fp16 once its
         // bytes have landed, then handed to the MMA thread through v_ready. K tiles are not touched.
         uint32_t kv_loads = 0;
+        RingPhases v_phases;
         bool ok = true;
         for (int r = 0; r < rounds && ok; ++r) {
             const int idx = item_of_round(r);
             if (idx < 0) continue;
             const Item w = decode_item(idx);
             for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                bool is_v;
-                if (kDoubleS) {
-                    const int n = w.n_max;
-                    const int lead = n > 1 ? 2 : 1;
-                    if (it < lead) {
-                        is_v = false;
-                    } else {
-                        const int f = it - lead, kk = n - lead;
-                        is_v = f >= 2 * kk || (f & 1) == 0;
-                    }
-                } else {
-                    is_v = (it & 1) != 0;
-                }
-                if (!is_v) continue;
+                if (!RingOrder(it, w.n_max, kDoubleS).is_v) continue;
                 const uint32_t slot = kv_loads % G::kSlots;
-                const uint32_t phase = (kv_loads / G::kSlots) & 1u;
-                ok = __all_sync(0xffffffffu, MbarWait(bar(kKvFull + slot), phase, abort_flag));
+                ok = __all_sync(0xffffffffu, MbarWait(full_bar(true, slot), v_phases.Take(slot), abort_flag));
                 if (!ok) break;
                 uint4* tile = reinterpret_cast<uint4*>(smem + (ring_smem - smem_base) + slot * G::kKvTileBytes);
 #pragma unroll 8
