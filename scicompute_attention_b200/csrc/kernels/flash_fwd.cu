@@ -260,18 +260,18 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
-            MbarInit(bar(kQFull + i), 1);
-            MbarInit(bar(kQEmpty + i), 1);
-            MbarInit(bar(kSFull + i), 1);
-            MbarInit(bar(kPFull + i), 4);
-            MbarInit(bar(kPLast + i), 4);
-            MbarInit(bar(kODone + i), 1);
-            MbarInit(bar(kOFree + i), 4);
+            MbarInit<1>(bar(kQFull + i));
+            MbarInit<1>(bar(kQEmpty + i));
+            MbarInit<1>(bar(kSFull + i));
+            MbarInit<4>(bar(kPFull + i));
+            MbarInit<4>(bar(kPLast + i));
+            MbarInit<1>(bar(kODone + i));
+            MbarInit<4>(bar(kOFree + i));
         }
-        for (int i = 0; i < 2 * G::kSlots; ++i) MbarInit(bar(kKvFull + i), 1);
+        for (int i = 0; i < 2 * G::kSlots; ++i) MbarInit<1>(bar(kKvFull + i));
         for (int i = 0; i < G::kSlots; ++i) {
-            MbarInit(bar(kKvEmpty + i), 1);
-            MbarInit(bar(kVReady + i), kConverterThreads);
+            MbarInit<1>(bar(kKvEmpty + i));
+            if constexpr (kCvtInKernel) MbarInit<kConverterThreads>(bar(kVReady + i));
         }
         *abort_flag = 0;
         FenceBarrierInit();

@@ -12,8 +12,10 @@ namespace sca_b200 {
 namespace sm100 {
 
 // ---- mbarrier ------------------------------------------------------------------------------------
-__device__ __forceinline__ void MbarInit(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+template <uint32_t kCount>
+__device__ __forceinline__ void MbarInit(uint32_t bar) {
+    static_assert(kCount >= 1 && kCount < (1u << 20), "arrival count of an mbarrier");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "n"(kCount) : "memory");
 }
 __device__ __forceinline__ void FenceBarrierInit() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
