@@ -277,6 +277,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         FenceBarrierInit();
     }
     if (warp == 0) {
+        __syncwarp();  // lane 0 comes from the initialisation; the instruction wants the whole warp
         TmemAlloc(SmemAddr(tmem_slot), kTmemColumns);
         TmemRelinquish();
     }
@@ -808,9 +809,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (failed && p.error_word != nullptr) *p.error_word = 1 + warp;
 
     // ---- teardown ------------------------------------------------------------------------------------
+    // One lane of warps 0 and 1 comes from its loop long after the others; the tensor-memory instructions are for whole
+    // warps, and neither the end of a branch nor __syncthreads promises that the lanes have met.
+    __syncwarp();
     TcFenceBefore();
     __syncthreads();
     if (warp == 0) {
+        __syncwarp();
         TcFenceAfter();
         TmemDealloc(tmem_base, kTmemColumns);
     }
