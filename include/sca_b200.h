@@ -154,8 +154,13 @@ typedef struct ScaDecodeFwdParams {
     const int32_t* seq_lens;   /* [batch] or NULL (= seq_kv for every sequence)                   */
 } ScaDecodeFwdParams;          /* 248 bytes: field for field the reference's DecodeFwdParams      */
 
-/* partial kernel + merge kernel on `stream` */
+/* partial kernel + merge kernel on `stream`: the caller's num_splits, and the partials stay in the caller's arrays */
 SCA_ABI int sca_launch_decode_splitk(const ScaDecodeFwdParams* params, void* stream);
+/* The same output by the faster way for the size of the call (no counterpart in the reference): the two kernels above, or
+ * for calls that do not fill the machine one launch in which clusters of CTAs split a sequence and merge on chip. The
+ * arrays and num_splits have to be valid either way; one launch leaves the arrays alone and does not look at num_splits.
+ * page_table != NULL selects paged K/V. cluster_ctas (may be NULL): CTAs per cluster of the one launch, 0 = two kernels. */
+SCA_ABI int sca_launch_decode_auto(const ScaDecodeFwdParams* params, int32_t* cluster_ctas, void* stream);
 /* same, but requires the page-table fields (decode_splitk.cu:245-253) */
 SCA_ABI int sca_launch_decode_splitk_paged(const ScaDecodeFwdParams* params, void* stream);
 

@@ -19,7 +19,7 @@ MGPU_ID_BYTES = 128
 # every symbol include/sca_b200.h declares (tests check that the library exports all of them)
 EXPORTED_SYMBOLS = [
     "sca_last_error", "sca_probe_device", "sca_probe_device_b200", "sca_mem_get_info", "sca_launch_flash_fwd", "sca_flash_status",
-    "sca_flash_smem_bytes_for", "sca_launch_decode_splitk", "sca_launch_decode_splitk_paged",
+    "sca_flash_smem_bytes_for", "sca_launch_decode_splitk", "sca_launch_decode_auto", "sca_launch_decode_splitk_paged",
     "sca_launch_paged_attention", "sca_launch_paged_attention_ordered", "sca_launch_decode_splitk_static", "sca_launch_decode_triples", "sca_launch_merge_triples",
     "sca_launch_simt_forward", "sca_naive_score_bytes", "sca_launch_naive_forward", "sca_launch_kv_append", "sca_launch_kv_reset_block",
     "sca_launch_kv_gather", "sca_launch_kv_append_batched", "sca_launch_decode_partials",
@@ -143,6 +143,7 @@ def lib() -> C.CDLL:
     l.sca_naive_score_bytes.argtypes = [C.c_int64] * 4
     l.sca_naive_score_bytes.restype = C.c_longlong
     l.sca_launch_decode_splitk.argtypes = [C.POINTER(DecodeFwdParams), C.c_void_p]
+    l.sca_launch_decode_auto.argtypes = [C.POINTER(DecodeFwdParams), C.POINTER(C.c_int32), C.c_void_p]
     l.sca_launch_decode_splitk_paged.argtypes = [C.POINTER(DecodeFwdParams), C.c_void_p]
     l.sca_launch_paged_attention.argtypes = [C.POINTER(PagedDecodeParams), C.c_void_p]
     l.sca_launch_paged_attention_ordered.argtypes = [C.POINTER(PagedDecodeParams), C.c_void_p, C.c_void_p]

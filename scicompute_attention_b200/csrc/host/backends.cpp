@@ -572,14 +572,15 @@ public:
         p.o_stride = {os.s_b, os.s_h, os.s_s};
         p.scale = EffectiveScale(cfg, shape);
         p.dtype = DtypeId(q.dtype());
-        if (sci::Status s = FromAbi(sca_launch_decode_splitk(&p, StreamHandle(cfg.stream))); !s.ok()) {
-            return sci::MakeUnexpected<AttentionResult>(s);
-        }
+        int32_t cluster = 0;  // an explicit split count asks for that many partials
+        const int rc = cfg.num_splits > 0 ? sca_launch_decode_splitk(&p, StreamHandle(cfg.stream))
+                                          : sca_launch_decode_auto(&p, &cluster, StreamHandle(cfg.stream));
+        if (sci::Status s = FromAbi(rc); !s.ok()) return sci::MakeUnexpected<AttentionResult>(s);
         result.stats.used_backend = BackendKind::kDecode;
         result.stats.workspace_bytes = static_cast<size_t>(elements) * sizeof(float);
-        result.stats.num_splits = splits;
-        result.stats.note = "split-K decode: " + std::to_string(splits) + " splits, FP32 partials in workspace; layout=" +
-                            std::string(LayoutName(cfg.layout));
+        result.stats.num_splits = cluster > 0 ? cluster : splits;
+        result.stats.note = "split-K decode: " + std::to_string(result.stats.num_splits) + " splits, FP32 partials " +
+                            (cluster > 0 ? "on chip (one launch)" : "in workspace") + "; layout=" + std::string(LayoutName(cfg.layout));
         return sci::Ok(std::move(result));
     }
     sci::Result<AttentionResult> ForwardVarlen(const sci::Tensor&, const sci::Tensor&, const sci::Tensor&, int64_t,
@@ -671,8 +672,7 @@ sci::Result<AttentionResult> RunPaged(const sci::Tensor& q, const PagedKVCache& 
     shape.num_kv_heads = kcfg.num_kv_heads;
     shape.head_dim = d;
 
-    ScaPagedDecodeParams pp{};
-    ScaDecodeFwdParams& p = pp.base;
+    ScaDecodeFwdParams p{};
     p.q = q.data();
     p.k = kv.Storage().K(params.layer).data();
     p.v = kv.Storage().V(params.layer).data();
@@ -693,20 +693,20 @@ sci::Result<AttentionResult> RunPaged(const sci::Tensor& q, const PagedKVCache& 
     p.scale = EffectiveScale(cfg, shape);
     p.dtype = DtypeId(q.dtype());
     p.seq_lens = params.seq_lens;
-    pp.page_table = table;
-    pp.block_size = block_size;
-    pp.max_blocks_per_seq = max_blocks;
-    pp.num_kv_blocks = kcfg.num_blocks;
-    // scheduling hint only: any permutation gives the same result
-    const int32_t* order = kv.SeqOrderDevicePtr(num_seqs);
-    if (sci::Status s = FromAbi(sca_launch_paged_attention_ordered(&pp, order, StreamHandle(cfg.stream))); !s.ok()) {
-        return sci::MakeUnexpected<AttentionResult>(s);
-    }
+    p.page_table = table;
+    p.block_size = block_size;
+    p.max_blocks_per_seq = max_blocks;
+    p.num_kv_blocks = kcfg.num_blocks;
+    int32_t cluster = 0;  // an explicit split count asks for that many partials
+    const int rc = cfg.num_splits > 0 ? sca_launch_decode_splitk_paged(&p, StreamHandle(cfg.stream))
+                                      : sca_launch_decode_auto(&p, &cluster, StreamHandle(cfg.stream));
+    if (sci::Status s = FromAbi(rc); !s.ok()) return sci::MakeUnexpected<AttentionResult>(s);
     result.stats.used_backend = BackendKind::kPaged;
     result.stats.workspace_bytes = static_cast<size_t>(elements) * sizeof(float);
-    result.stats.num_splits = splits;
+    result.stats.num_splits = cluster > 0 ? cluster : splits;
     result.stats.kv_bytes = kv.Storage().MemoryBytes();
-    result.stats.note = "paged decode: " + std::to_string(splits) + " splits, block_size=" + std::to_string(block_size) +
+    result.stats.note = "paged decode: " + std::to_string(result.stats.num_splits) +
+                        (cluster > 0 ? " splits on chip (one launch), block_size=" : " splits, block_size=") + std::to_string(block_size) +
                         ", layer=" + std::to_string(params.layer);
     return sci::Ok(std::move(result));
 }

@@ -766,9 +766,9 @@ bool ClusterIsFaster(int64_t units, int64_t steps, int cluster, int64_t resident
     return one_launch < 11.5 + 1.55 * std::max(1.0, wave);
 }
 
-// Launches decode_cluster_kernel if it is the kernel for this call (*taken).
+// Launches decode_cluster_kernel if it is the kernel for this call; *taken = its CTAs per cluster, 0 if it is not.
 template <typename T, int D, bool kPaged, bool kHi>
-int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, bool* taken) {
+int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, int* taken) {
     const int64_t units = p.batch * p.num_kv_heads * head_chunks;
     const void* fn = reinterpret_cast<const void*>(&decode_cluster_kernel<T, D, kPaged, kHi>);
     if (int rc = EnsureDynamicSmem(fn, DecodeGeom<D>::kSmemBytes, "decode_cluster_kernel")) return rc;
@@ -778,8 +778,8 @@ int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     int cluster = kMaxCluster;
     while (cluster >= 2 && units > ResidentClusters<T, D, kPaged, kHi>(cluster)) cluster /= 2;
     if (cluster < 2 || !ClusterIsFaster(units, steps, cluster, resident, p.seq_lens != nullptr)) cluster = 0;
-    *taken = cluster > 0;
-    if (!*taken) return SCA_OK;
+    *taken = cluster;
+    if (cluster == 0) return SCA_OK;
     cudaLaunchAttribute attr{};
     const cudaLaunchConfig_t cfg = ClusterConfig(static_cast<unsigned>(units * cluster), cluster, DecodeGeom<D>::kSmemBytes, stream, &attr);
     cudaLaunchKernelEx(&cfg, decode_cluster_kernel<T, D, kPaged, kHi>, p, head_chunks, cluster);
@@ -808,40 +808,41 @@ int LaunchPartial(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     return CheckLaunch("decode_partial_kernel", stream);
 }
 
-// `merged` (may be null): set when the launch has written the output itself, so that no merge is needed.
+// `cluster` null: the partials, whatever the size of the call. Otherwise the launch may write the output itself, on
+// clusters of *cluster CTAs and without partials; *cluster = 0 says that it has not.
 template <typename T, int D, bool kPaged, bool kHi>
-int LaunchOne(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, bool* merged) {
-    if (merged != nullptr) {
-        if (int rc = LaunchCluster<T, D, kPaged, kHi>(p, head_chunks, stream, merged)) return rc;
-        if (*merged) return SCA_OK;
+int LaunchOne(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t stream, int* cluster) {
+    if (cluster != nullptr) {
+        if (int rc = LaunchCluster<T, D, kPaged, kHi>(p, head_chunks, stream, cluster)) return rc;
+        if (*cluster > 0) return SCA_OK;
     }
     return LaunchPartial<T, D, kPaged, kHi>(p, head_chunks, stream);
 }
 
 template <typename T, int D>
-int LaunchPartialForDim(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged) {
+int LaunchPartialForDim(const ScaDecodeFwdParams& p, cudaStream_t stream, int* cluster) {
     const int group = static_cast<int>(p.num_heads / p.num_kv_heads);
     const int head_chunks = (group + 15) / 16;
     const bool paged = p.page_table != nullptr;
     const bool hi = group > 8;
     if (paged) {
-        return hi ? LaunchOne<T, D, true, true>(p, head_chunks, stream, merged)
-                  : LaunchOne<T, D, true, false>(p, head_chunks, stream, merged);
+        return hi ? LaunchOne<T, D, true, true>(p, head_chunks, stream, cluster)
+                  : LaunchOne<T, D, true, false>(p, head_chunks, stream, cluster);
     }
-    return hi ? LaunchOne<T, D, false, true>(p, head_chunks, stream, merged)
-              : LaunchOne<T, D, false, false>(p, head_chunks, stream, merged);
+    return hi ? LaunchOne<T, D, false, true>(p, head_chunks, stream, cluster)
+              : LaunchOne<T, D, false, false>(p, head_chunks, stream, cluster);
 }
 
 template <typename T>
-int LaunchPartialTyped(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged) {
+int LaunchPartialTyped(const ScaDecodeFwdParams& p, cudaStream_t stream, int* cluster) {
     switch (p.head_dim) {
-        case 32: return LaunchPartialForDim<T, 32>(p, stream, merged);
-        case 64: return LaunchPartialForDim<T, 64>(p, stream, merged);
-        case 96: return LaunchPartialForDim<T, 96>(p, stream, merged);
-        case 128: return LaunchPartialForDim<T, 128>(p, stream, merged);
-        case 160: return LaunchPartialForDim<T, 160>(p, stream, merged);
-        case 192: return LaunchPartialForDim<T, 192>(p, stream, merged);
-        case 256: return LaunchPartialForDim<T, 256>(p, stream, merged);
+        case 32: return LaunchPartialForDim<T, 32>(p, stream, cluster);
+        case 64: return LaunchPartialForDim<T, 64>(p, stream, cluster);
+        case 96: return LaunchPartialForDim<T, 96>(p, stream, cluster);
+        case 128: return LaunchPartialForDim<T, 128>(p, stream, cluster);
+        case 160: return LaunchPartialForDim<T, 160>(p, stream, cluster);
+        case 192: return LaunchPartialForDim<T, 192>(p, stream, cluster);
+        case 256: return LaunchPartialForDim<T, 256>(p, stream, cluster);
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT,
@@ -910,21 +911,20 @@ int LaunchMergeOut(const ScaDecodeFwdParams& p, cudaStream_t stream) {
 // fp32 inputs take the SIMT partial kernel (simt.cu); declared here, defined there.
 int LaunchDecodePartialF32(const ScaDecodeFwdParams& p, cudaStream_t stream);
 
-int LaunchDecodePartials(const ScaDecodeFwdParams& p, cudaStream_t stream, bool* merged = nullptr) {
+int LaunchDecodePartials(const ScaDecodeFwdParams& p, cudaStream_t stream, int* cluster = nullptr) {
     switch (p.dtype) {
-        case SCA_DTYPE_F16: return LaunchPartialTyped<__half>(p, stream, merged);
-        case SCA_DTYPE_BF16: return LaunchPartialTyped<__nv_bfloat16>(p, stream, merged);
+        case SCA_DTYPE_F16: return LaunchPartialTyped<__half>(p, stream, cluster);
+        case SCA_DTYPE_BF16: return LaunchPartialTyped<__nv_bfloat16>(p, stream, cluster);
         case SCA_DTYPE_F32: return LaunchDecodePartialF32(p, stream);
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT, "decode: unsupported dtype id");
 }
 
-// Partials and merge, or both in one launch where that is faster.
-int LaunchDecode(const ScaDecodeFwdParams& p, cudaStream_t stream) {
-    bool merged = false;
-    if (int rc = LaunchDecodePartials(p, stream, &merged)) return rc;
-    return merged ? SCA_OK : LaunchMergeOut(p, stream);
+// Partials and merge.
+int LaunchSplitK(const ScaDecodeFwdParams& p, cudaStream_t stream) {
+    if (int rc = LaunchDecodePartials(p, stream)) return rc;
+    return LaunchMergeOut(p, stream);
 }
 
 }  // namespace sca_b200
@@ -975,7 +975,22 @@ extern "C" int sca_launch_decode_splitk(const ScaDecodeFwdParams* params, void* 
     ClearError();
     if (int rc = ValidateDecode(params, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return LaunchDecode(*params, s);
+    return LaunchSplitK(*params, s);
+}
+
+extern "C" int sca_launch_decode_auto(const ScaDecodeFwdParams* params, int32_t* cluster_ctas, void* stream) {
+    ClearError();
+    if (int rc = ValidateDecode(params, true)) return rc;
+    const ScaDecodeFwdParams& p = *params;
+    if (p.page_table != nullptr && (p.block_size <= 0 || p.max_blocks_per_seq <= 0 || p.num_kv_blocks <= 0)) {
+        return Fail(SCA_INVALID_ARGUMENT,
+                    "paged attention: block_size/max_blocks_per_seq/num_kv_blocks must be positive");
+    }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int cluster = 0;
+    if (int rc = LaunchDecodePartials(p, s, &cluster)) return rc;
+    if (cluster_ctas != nullptr) *cluster_ctas = cluster;
+    return cluster > 0 ? SCA_OK : LaunchMergeOut(p, s);
 }
 
 extern "C" int sca_launch_decode_splitk_paged(const ScaDecodeFwdParams* params, void* stream) {
@@ -1010,7 +1025,7 @@ extern "C" int sca_launch_paged_attention_ordered(const ScaPagedDecodeParams* pa
     if (int rc = ValidateDecode(&p, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     (void)seq_order;  // the kernel deals out equal shares of the K/V stream itself; the hint has nothing left to improve
-    return LaunchDecode(p, s);
+    return LaunchSplitK(p, s);
 }
 
 extern "C" int sca_launch_paged_attention(const ScaPagedDecodeParams* params, void* stream) {
@@ -1104,5 +1119,5 @@ extern "C" int sca_launch_decode_splitk_static(const ScaDecodeFwdParams* params,
     p.partial_o = scratch + 2 * base;
     if (int rc = ValidateDecode(&p, true)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return LaunchDecode(p, s);
+    return LaunchSplitK(p, s);
 }

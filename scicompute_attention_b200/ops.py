@@ -17,7 +17,7 @@ import torch
 
 from . import _lib
 from ._lib import (DTYPE_BF16, DTYPE_F16, DTYPE_F32, DecodeFwdParams, DecodeStrides, FlashFwdParams,
-                   KvCacheShape, PagedDecodeParams, check, lib)
+                   KvCacheShape, check, lib)
 
 MAX_SPLITS = 64          # upper bound of the automatic split count on B200
 
@@ -170,10 +170,22 @@ def decode_attention(q, k, v, *, scale=None, num_splits: int = 0, layout: str = 
     p.dtype = dtype_id(q.dtype)
     p.page_table = None
     p.seq_lens = seq_lens.data_ptr() if seq_lens is not None else None
-    check(lib().sca_launch_decode_splitk(C.byref(p), _stream_ptr(stream)))
-    if return_stats:
-        return out, {"num_splits": splits, "workspace_bytes": base * (2 + d) * 4}
-    return out
+    return _launch_decode(p, num_splits, stream, out, return_stats)
+
+
+def _launch_decode(p, num_splits, stream, out, return_stats):
+    """An explicit split count asks for that many partials in the scratch; otherwise the size of the call decides."""
+    cluster = C.c_int32(0)
+    if num_splits > 0:
+        launch = lib().sca_launch_decode_splitk_paged if p.page_table else lib().sca_launch_decode_splitk
+        check(launch(C.byref(p), _stream_ptr(stream)))
+    else:
+        check(lib().sca_launch_decode_auto(C.byref(p), C.byref(cluster), _stream_ptr(stream)))
+    if not return_stats:
+        return out
+    # num_splits: pieces a sequence is cut into at most; cluster: CTAs per cluster of the one-launch kernel, 0 = two kernels
+    return out, {"num_splits": cluster.value or p.num_splits, "cluster": cluster.value,
+                 "workspace_bytes": p.batch * p.num_heads * p.num_splits * (2 + p.head_dim) * 4}
 
 
 def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int, scale=None,
@@ -222,19 +234,13 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
     p.scale = effective_scale(scale, d)
     p.dtype = dtype_id(q.dtype)
     p.seq_lens = seq_lens.data_ptr() if seq_lens is not None else None
-    order_ptr = None
-    if seq_order is not None:
-        if seq_order.dtype != torch.int32 or seq_order.numel() != s or not seq_order.is_cuda:
-            raise _lib.ScaError(4, "seq_order must be a device int32 permutation of the sequences")
-        order_ptr = seq_order.data_ptr()
-    pp = PagedDecodeParams()
-    pp.base = p
-    pp.page_table = page_table.data_ptr()
-    pp.block_size, pp.max_blocks_per_seq, pp.num_kv_blocks = bs, max_blocks, nblk
-    check(lib().sca_launch_paged_attention_ordered(C.byref(pp), order_ptr, _stream_ptr(stream)))
-    if return_stats:
-        return out, {"num_splits": splits, "workspace_bytes": base * (2 + d) * 4}
-    return out
+    if seq_order is not None and (seq_order.dtype != torch.int32 or seq_order.numel() != s or not seq_order.is_cuda):
+        raise _lib.ScaError(4, "seq_order must be a device int32 permutation of the sequences")
+    p.page_table = page_table.data_ptr()
+    if not p.page_table:
+        raise _lib.ScaError(4, "paged attention: null page table")
+    p.block_size, p.max_blocks_per_seq, p.num_kv_blocks = bs, max_blocks, nblk
+    return _launch_decode(p, num_splits, stream, out, return_stats)
 
 
 def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
