@@ -52,6 +52,9 @@ private:
     bool previous_active_;
 };
 
+// Whether work queued on `cuda_stream` is being captured into a graph.
+bool StreamIsCapturing(void* cuda_stream);
+
 class DeviceManager {
 public:
     static DeviceManager& Instance();

@@ -153,11 +153,11 @@ public:
         if (sci::Status s = AllocateOutputs(q, shape, cfg.return_lse, &result); !s.ok()) {
             return sci::MakeUnexpected<AttentionResult>(s);
         }
-        const sci::Result<float*> scores =
-            runtime::AcquireScratchFp32(runtime::ScratchKind::kScoresFp32, need / sizeof(float), q.device());
+        const sci::Result<runtime::ScratchLease> scores =
+            runtime::AcquireScratchFp32(runtime::ScratchKind::kScoresFp32, need / sizeof(float), q.device(), StreamHandle(cfg.stream));
         if (!scores.ok()) return sci::MakeUnexpected<AttentionResult>(scores.error());
         const ScaFlashFwdParams p = PackForward(q, k, v, &result, cfg, shape);
-        if (sci::Status s = FromAbi(sca_launch_naive_forward(&p, *scores, StreamHandle(cfg.stream))); !s.ok()) {
+        if (sci::Status s = FromAbi(sca_launch_naive_forward(&p, scores->data, StreamHandle(cfg.stream))); !s.ok()) {
             return sci::MakeUnexpected<AttentionResult>(s);
         }
         result.stats.used_backend = BackendKind::kNaive;
@@ -540,8 +540,8 @@ public:
         }
         const int64_t splits = ResolveSplits(cfg, shape, DeviceCapability::ForDevice(0));
         const int64_t elements = tables::PartialElements(shape.batch, shape.num_heads, splits, shape.head_dim);
-        const sci::Result<float*> scratch =
-            runtime::AcquireScratchFp32(runtime::ScratchKind::kDecodePartials, static_cast<size_t>(elements), q.device());
+        const sci::Result<runtime::ScratchLease> scratch = runtime::AcquireScratchFp32(
+            runtime::ScratchKind::kDecodePartials, static_cast<size_t>(elements), q.device(), StreamHandle(cfg.stream));
         if (!scratch.ok()) return sci::MakeUnexpected<AttentionResult>(scratch.error());
 
         AttentionResult result;
@@ -557,9 +557,9 @@ public:
         p.k = k.data();
         p.v = v.data();
         p.out = result.out.data();
-        p.partial_m = *scratch;
-        p.partial_l = *scratch + base;
-        p.partial_o = *scratch + 2 * base;
+        p.partial_m = scratch->data;
+        p.partial_l = scratch->data + base;
+        p.partial_o = scratch->data + 2 * base;
         p.batch = shape.batch;
         p.num_heads = shape.num_heads;
         p.num_kv_heads = shape.num_kv_heads;
@@ -654,8 +654,8 @@ sci::Result<AttentionResult> RunPaged(const sci::Tensor& q, const PagedKVCache& 
         splits = tables::SlotsForSchedule(total_steps, longest_steps, columns, DeviceCapability::ForDevice(0).sm_count);
     }
     const int64_t elements = tables::PartialElements(num_seqs, heads, splits, d);
-    const sci::Result<float*> scratch =
-        runtime::AcquireScratchFp32(runtime::ScratchKind::kDecodePartials, static_cast<size_t>(elements), q.device());
+    const sci::Result<runtime::ScratchLease> scratch = runtime::AcquireScratchFp32(
+        runtime::ScratchKind::kDecodePartials, static_cast<size_t>(elements), q.device(), StreamHandle(cfg.stream));
     if (!scratch.ok()) return sci::MakeUnexpected<AttentionResult>(scratch.error());
 
     AttentionResult result;
@@ -677,9 +677,9 @@ sci::Result<AttentionResult> RunPaged(const sci::Tensor& q, const PagedKVCache& 
     p.k = kv.Storage().K(params.layer).data();
     p.v = kv.Storage().V(params.layer).data();
     p.out = result.out.data();
-    p.partial_m = *scratch;
-    p.partial_l = *scratch + base;
-    p.partial_o = *scratch + 2 * base;
+    p.partial_m = scratch->data;
+    p.partial_l = scratch->data + base;
+    p.partial_o = scratch->data + 2 * base;
     p.batch = num_seqs;
     p.num_heads = heads;
     p.num_kv_heads = kcfg.num_kv_heads;

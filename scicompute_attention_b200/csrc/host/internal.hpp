@@ -16,9 +16,15 @@ const IAttentionBackend* FlashBackendInstance() noexcept;
 const IAttentionBackend* DecodeBackendInstance() noexcept;
 const IAttentionBackend* PagedBackendInstance() noexcept;
 
-// Grow-only fp32 scratch per (device, kind); see scratch.cpp.
+// fp32 scratch for one call on `stream`, from a grow-only pool per (device, kind, stream): calls on different streams may
+// run at the same time. A call that is being captured gets memory of its own, which the graph takes and gives back, so that
+// no graph holds a pointer into the pool. The lease outlives the launch and no more.
 enum class ScratchKind : int { kScoresFp32 = 0, kDecodePartials = 1, kGeneric = 2, kCount = 3 };
-sci::Result<float*> AcquireScratchFp32(ScratchKind kind, size_t elements, sci::Device& device);
+struct ScratchLease {
+    float* data{nullptr};
+    sci::Tensor own;  // memory of this call alone
+};
+sci::Result<ScratchLease> AcquireScratchFp32(ScratchKind kind, size_t elements, sci::Device& device, void* stream);
 sci::Status ReleaseScratch();
 size_t ScratchHighWaterMarkBytes();
 

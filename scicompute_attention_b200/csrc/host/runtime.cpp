@@ -3,10 +3,13 @@
 // Behaviour follows src/runtime/capability.cpp, scratch_pool.cpp and workspace.cpp of the reference.
 #include <algorithm>
 #include <cstdlib>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <unordered_map>
 #include <utility>
 
+#include "device/cuda_device.hpp"
 #include "device/stream.hpp"
 #include "internal.hpp"
 
@@ -32,37 +35,63 @@ std::mutex& ScratchMutex() {
     static std::mutex m;
     return m;
 }
+using ScratchKey = std::tuple<int, int, void*>;  // device, kind, stream
+// More streams than this give the pool back and start anew.
+constexpr size_t kMaxScratchEntries = 64;
 // Leaked on purpose: freeing device memory from a static destructor runs after the CUDA runtime is gone.
-std::unordered_map<int, ScratchEntry>& ScratchMap() {
-    static auto* map = new std::unordered_map<int, ScratchEntry>();
+std::map<ScratchKey, ScratchEntry>& ScratchMap() {
+    static auto* map = new std::map<ScratchKey, ScratchEntry>();
     return *map;
 }
 size_t g_scratch_peak_bytes = 0;
+
+// The streams that used an entry may be gone, so there is nothing to order its release on: wait for the device.
+void ClearScratch() {
+    for (auto& item : ScratchMap()) {
+        if (item.second.buffer.data() != nullptr) item.second.buffer.device().synchronize();
+    }
+    ScratchMap().clear();
+}
 }  // namespace
 
-sci::Result<float*> AcquireScratchFp32(ScratchKind kind, size_t elements, sci::Device& device) {
+sci::Result<ScratchLease> AcquireScratchFp32(ScratchKind kind, size_t elements, sci::Device& device, void* stream) {
     if (elements == 0) {
-        return sci::MakeUnexpected<float*>(MakeStatus(AttnStatusCode::kWorkspaceExceeded, "scratch request with 0 elements"));
+        return sci::MakeUnexpected<ScratchLease>(MakeStatus(AttnStatusCode::kWorkspaceExceeded, "scratch request with 0 elements"));
     }
+    auto allocate = [&](size_t n) { return sci::Tensor(sci::TensorShape({static_cast<sci::index_t>(n)}), sci::DType::kFloat32, device); };
+    auto refuse = [](size_t n) {
+        return sci::MakeUnexpected<ScratchLease>(MakeStatus(
+            AttnStatusCode::kWorkspaceExceeded, "scratch allocation of " + std::to_string(n * sizeof(float)) + " B failed"));
+    };
+    ScratchLease lease;
+    const bool capturing = sci::StreamIsCapturing(stream);
     std::lock_guard<std::mutex> lock(ScratchMutex());
-    ScratchEntry& entry = ScratchMap()[device.id() * 16 + static_cast<int>(kind)];
+    if (capturing) {
+        lease.own = allocate(elements);
+        lease.data = static_cast<float*>(lease.own.data());
+        if (lease.data == nullptr) return refuse(elements);
+        return sci::Ok(std::move(lease));
+    }
+    const ScratchKey key{device.id(), static_cast<int>(kind), stream};
+    if (ScratchMap().size() >= kMaxScratchEntries && ScratchMap().count(key) == 0) ClearScratch();
+    ScratchEntry& entry = ScratchMap()[key];
     if (entry.buffer.data() == nullptr || entry.elements < elements) {
         const size_t grown = static_cast<size_t>(static_cast<double>(elements) * 1.25) + 1024;
-        entry.buffer = sci::Tensor(sci::TensorShape({static_cast<sci::index_t>(grown)}), sci::DType::kFloat32, device);
+        entry.buffer = allocate(grown);  // inside the call's StreamOrderedScope: the old one is released in stream order
         if (entry.buffer.data() == nullptr) {
             entry.elements = 0;
-            return sci::MakeUnexpected<float*>(MakeStatus(
-                AttnStatusCode::kWorkspaceExceeded, "scratch allocation of " + std::to_string(grown * sizeof(float)) + " B failed"));
+            return refuse(grown);
         }
         entry.elements = grown;
         g_scratch_peak_bytes = std::max(g_scratch_peak_bytes, grown * sizeof(float));
     }
-    return sci::Ok(static_cast<float*>(entry.buffer.data()));
+    lease.data = static_cast<float*>(entry.buffer.data());
+    return sci::Ok(std::move(lease));
 }
 
 sci::Status ReleaseScratch() {
     std::lock_guard<std::mutex> lock(ScratchMutex());
-    ScratchMap().clear();
+    ClearScratch();
     return sci::Status::Ok();
 }
 

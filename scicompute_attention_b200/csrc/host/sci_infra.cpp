@@ -145,6 +145,8 @@ bool IsCapturing(cudaStream_t stream) {
 }
 }  // namespace
 
+SCI_EXPORT bool StreamIsCapturing(void* cuda_stream) { return IsCapturing(static_cast<cudaStream_t>(cuda_stream)); }
+
 SCI_EXPORT StreamOrderedScope::StreamOrderedScope(void* cuda_stream)
     : previous_(g_scope_stream), previous_active_(g_scope_active) {
     g_scope_stream = cuda_stream;

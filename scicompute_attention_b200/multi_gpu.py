@@ -16,6 +16,7 @@ local memory; peers are only touched by plain stores from that kernel.
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Callable, Sequence
 
 
@@ -76,7 +77,7 @@ class MgpuComm:
         import torch
         from . import ops
         rows, width = mine.shape
-        out = torch.empty((self.world, rows, width), dtype=torch.float32, device=mine.device)
+        out = ops._empty((self.world, rows, width), torch.float32, mine.device, stream)
         limit = self.timeout_ms if timeout_ms is None else timeout_ms
         self._lib.check(self._lib.lib().sca_mgpu_allgather_triples(self._comm, mine.contiguous().data_ptr(), out.data_ptr(),
                                                                    rows * width, ops._stream_ptr(stream), limit))
@@ -197,10 +198,11 @@ class PeerExchange:
         else:
             # a rank without tokens contributes m = -inf, l = 0, O = 0 and is skipped by the merge
             splits = 1
-            ws = torch.zeros(self.rows * (2 + d), dtype=torch.float32, device=q.device)
-            ws[: self.rows] = float("-inf")
+            with contextlib.nullcontext() if stream is None else ops._on(stream):
+                ws = torch.zeros(self.rows * (2 + d), dtype=torch.float32, device=q.device)
+                ws[: self.rows] = float("-inf")
             pm, pl, po = ws[: self.rows], ws[self.rows: 2 * self.rows], ws[2 * self.rows:]
-        out = torch.empty((self.rows, d), dtype=q.dtype, device=q.device)
+        out = ops._empty((self.rows, d), q.dtype, q.device, stream)
         x = _lib.SeqSplitExchange()
         for r, ptr in enumerate(self._peers):
             x.peer_buffers[r] = ptr

@@ -4,7 +4,7 @@ taking torch CUDA tensors only as device memory + stream providers.
 
 Argument meaning follows the reference's public API (include/scicompute_attention/*.hpp):
 q is [B, H_q, S_q, D] (layout "bhsd") or [B, S_q, H_q, D] ("bshd"); k/v likewise with H_kv;
-outputs are always freshly allocated contiguous BHSD tensors.
+outputs are always freshly allocated contiguous BHSD tensors, allocated on `stream` where one is given.
 """
 from __future__ import annotations
 
@@ -12,6 +12,7 @@ import ctypes as C
 import functools
 import math
 import struct
+import threading
 
 import torch
 
@@ -22,7 +23,15 @@ from ._lib import (DTYPE_BF16, DTYPE_F16, DTYPE_F32, DecodeFwdParams, DecodeStri
 MAX_SPLITS = 64          # upper bound of the automatic split count on B200
 
 _DTYPE_IDS = {torch.float32: DTYPE_F32, torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16}
-_scratch: dict[tuple[int, int], torch.Tensor] = {}
+MAX_SCRATCH_BUFFERS = 32  # scratch buffers a thread keeps
+
+
+class _Scratch(threading.local):
+    def __init__(self):
+        self.pool: dict[tuple[int, int, int], torch.Tensor] = {}
+
+
+_scratch = _Scratch()
 _sm_count: dict[int, int] = {}
 
 
@@ -55,16 +64,41 @@ def sm_count(device: torch.device) -> int:
     return _sm_count[idx]
 
 
-def acquire_scratch_fp32(elements: int, device: torch.device, kind: int = 1) -> torch.Tensor:
-    """Process-wide grow-only fp32 scratch per (device, kind); same growth rule as the reference's
-    pool (src/runtime/scratch_pool.cpp:38-60): 1.25 x request + 1024 elements."""
+def _on(stream):
+    """Makes `stream` the current one: what is allocated there is reused in that stream's order."""
+    return torch.cuda.stream(stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream))
+
+
+def _empty(shape, dtype, device, stream=None) -> torch.Tensor:
+    """Device memory for a launch on `stream` (None: the current one)."""
+    if stream is None:
+        return torch.empty(shape, dtype=dtype, device=device)
+    with _on(stream):
+        return torch.empty(shape, dtype=dtype, device=device)
+
+
+def _is_capturing(stream) -> bool:
+    if stream is None:
+        return torch.cuda.is_current_stream_capturing()
+    with _on(stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
+def acquire_scratch_fp32(elements: int, device: torch.device, kind: int = 1, *, stream=None) -> torch.Tensor:
+    """Grow-only fp32 scratch of this thread per (device, kind, stream), so that calls that may overlap on the GPU never
+    share it; same growth rule as the reference's pool (src/runtime/scratch_pool.cpp:38-60): 1.25 x request + 1024
+    elements. A call that is being captured gets memory of the graph's own pool: no graph points into this one."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, kind)
-    cur = _scratch.get(key)
+    if _is_capturing(stream):
+        return _empty(elements, torch.float32, device, stream)
+    key = (idx, kind, _stream_ptr(stream))
+    pool = _scratch.pool
+    cur = pool.get(key)
     if cur is None or cur.numel() < elements:
-        grown = int(elements * 1.25) + 1024
-        cur = torch.empty(grown, dtype=torch.float32, device=device)
-        _scratch[key] = cur
+        pool.pop(key, None)
+        if len(pool) >= MAX_SCRATCH_BUFFERS:
+            del pool[next(iter(pool))]  # the oldest; the allocator reuses it in the order of its stream
+        cur = pool[key] = _empty(int(elements * 1.25) + 1024, torch.float32, device, stream)
     return cur
 
 
@@ -153,8 +187,8 @@ def decode_attention(q, k, v, *, scale=None, num_splits: int = 0, layout: str = 
         raise _lib.ScaError(4, f"num_heads={hq} % num_kv_heads={hkv} != 0")
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
     base = b * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device)
-    out = torch.empty((b, hq, 1, d), dtype=q.dtype, device=q.device)
+    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
+    out = _empty((b, hq, 1, d), q.dtype, q.device, stream)
 
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
@@ -218,8 +252,8 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
         splits = paged_splits_for(typical_len if typical_len > 0 else min(upper, max_blocks * bs), s, hkv,
                                   hq // hkv, sm_count(q.device), longest_len)
     base = s * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device)
-    out = torch.empty((s, hq, 1, d), dtype=q.dtype, device=q.device)
+    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
+    out = _empty((s, hq, 1, d), q.dtype, q.device, stream)
 
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr()
@@ -251,8 +285,8 @@ def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     _, hkv, skv, _ = _dims(k, "bhsd")
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
     base = b * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device)
-    triples = torch.empty((b * hq, 2 + d), dtype=torch.float32, device=q.device)
+    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
+    triples = _empty((b * hq, 2 + d), torch.float32, q.device, stream)
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), None
     p.partial_m = ws.data_ptr()
@@ -271,13 +305,13 @@ def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
 
 def decode_partials(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     """The split-K partial kernel alone. Returns (m [rows, splits], l [rows, splits], O [rows, splits, D],
-    splits) as fp32 views of the scratch pool (valid until the next decode call on this device)."""
+    splits) as fp32 views of the scratch pool (valid until this thread's next decode call on the stream)."""
     _require_cuda(q, k, v)
     b, hq, sq, d = _dims(q, "bhsd")
     _, hkv, skv, _ = _dims(k, "bhsd")
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
     base = b * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device)
+    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), None
     p.partial_m = ws.data_ptr()
@@ -299,7 +333,7 @@ def merge_triples(gathered, out_dtype, *, stream=None):
     _require_cuda(gathered)
     ranks, rows, width = gathered.shape
     d = width - 2
-    out = torch.empty((rows, d), dtype=out_dtype, device=gathered.device)
+    out = _empty((rows, d), out_dtype, gathered.device, stream)
     check(lib().sca_launch_merge_triples(gathered.data_ptr(), ranks, rows, d, out.data_ptr(),
                                          dtype_id(out_dtype), _stream_ptr(stream)))
     return out
@@ -331,10 +365,10 @@ def _fwd_params(q, k, v, out, lse, causal, scale, layout):
     return p
 
 
-def _alloc_out(q, layout, return_lse):
+def _alloc_out(q, layout, return_lse, stream):
     b, hq, sq, d = _dims(q, layout)
-    out = torch.empty((b, hq, sq, d), dtype=q.dtype, device=q.device)
-    lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device) if return_lse else None
+    out = _empty((b, hq, sq, d), q.dtype, q.device, stream)
+    lse = _empty((b, hq, sq), torch.float32, q.device, stream) if return_lse else None
     return out, lse
 
 
@@ -355,7 +389,7 @@ def flash_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layo
         raise _lib.ScaError(4, "flash backend computes in fp16/bf16; dtype=float32 is served by the naive "
                                "(reference) or tiled backend")
     if out is None:
-        out, lse = _alloc_out(q, layout, return_lse)
+        out, lse = _alloc_out(q, layout, return_lse, stream)
     p = _fwd_params(q, k, v, out, lse, causal, scale, layout)
     check(lib().sca_launch_flash_fwd(C.byref(p), _stream_ptr(stream)))
     return (out, lse) if return_lse else out
@@ -375,9 +409,9 @@ def flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_kv, *, causal=False
     tq, hq, d = q.shape
     tkv, hkv, _ = k.shape
     n = cu_q.shape[0] - 1
-    out = torch.empty_like(q)
+    out = _empty(q.shape, q.dtype, q.device, stream)
     ws_bytes = lib().sca_flash_varlen_workspace_bytes(n, tq)
-    ws = torch.empty(max(int(ws_bytes), 16), dtype=torch.uint8, device=q.device)
+    ws = _empty(max(int(ws_bytes), 16), torch.uint8, q.device, stream)
     p = _lib.FlashVarlenParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
     p.total_q, p.total_kv, p.num_heads, p.num_kv_heads, p.head_dim, p.num_seqs = tq, tkv, hq, hkv, d, n
@@ -387,8 +421,6 @@ def flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_kv, *, causal=False
     p.dtype_id = dtype_id(q.dtype)
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     check(lib().sca_launch_flash_varlen(C.byref(p), _stream_ptr(stream)))
-    if stream is None:
-        ws.record_stream(torch.cuda.current_stream(q.device))
     return out
 
 
@@ -413,9 +445,9 @@ def flash_attention_paged(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_
     nblk, bs, hkv, dk = k_pool.shape
     if dk != d:
         raise _lib.ScaError(4, "pool head_dim differs from q")
-    out = torch.empty_like(q)
+    out = _empty(q.shape, q.dtype, q.device, stream)
     ws_bytes = lib().sca_flash_varlen_workspace_bytes(n, tq)
-    ws = torch.empty(max(int(ws_bytes), 16), dtype=torch.uint8, device=q.device)
+    ws = _empty(max(int(ws_bytes), 16), torch.uint8, q.device, stream)
     p = _lib.FlashPagedParams()
     p.q, p.out, p.k_pool, p.v_pool, p.page_table = q.data_ptr(), out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), page_table.data_ptr()
     p.total_q, p.num_heads, p.num_kv_heads, p.head_dim, p.num_seqs = tq, hq, hkv, d, n
@@ -426,15 +458,13 @@ def flash_attention_paged(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_
     p.dtype_id = dtype_id(q.dtype)
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     check(lib().sca_launch_flash_paged(C.byref(p), _stream_ptr(stream)))
-    if stream is None:
-        ws.record_stream(torch.cuda.current_stream(q.device))
     return out
 
 
 def simt_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layout="bhsd", stream=None):
     """Functional SIMT attention behind the naive / tiled backends (any compute dtype)."""
     _require_cuda(q, k, v)
-    out, lse = _alloc_out(q, layout, return_lse)
+    out, lse = _alloc_out(q, layout, return_lse, stream)
     p = _fwd_params(q, k, v, out, lse, causal, scale, layout)
     check(lib().sca_launch_simt_forward(C.byref(p), _stream_ptr(stream)))
     return (out, lse) if return_lse else out
@@ -443,12 +473,12 @@ def simt_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layou
 def naive_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layout="bhsd", stream=None):
     """Level-1 attention with the fp32 score matrix materialised in scratch (sca::naive_attention)."""
     _require_cuda(q, k, v)
-    out, lse = _alloc_out(q, layout, return_lse)
+    out, lse = _alloc_out(q, layout, return_lse, stream)
     p = _fwd_params(q, k, v, out, lse, causal, scale, layout)
     need = lib().sca_naive_score_bytes(p.batch, p.num_heads, p.seq_q, p.seq_kv)
     if need <= 0:
         raise _lib.ScaError(4, "naive attention: invalid geometry")
-    scores = acquire_scratch_fp32(need // 4, q.device)
+    scores = _empty(need // 4, torch.float32, q.device, stream)
     check(lib().sca_launch_naive_forward(C.byref(p), scores.data_ptr(), _stream_ptr(stream)))
     return (out, lse) if return_lse else out
 
@@ -491,7 +521,7 @@ def kv_reset(layer_k, layer_v, block_ids, *, stream=None) -> None:
 def kv_gather(layer, block_ids, *, stream=None) -> torch.Tensor:
     _require_cuda(layer, block_ids)
     shape = _kv_shape(layer)
-    out = torch.empty((block_ids.numel(),) + tuple(layer.shape[1:]), dtype=layer.dtype, device=layer.device)
+    out = _empty((block_ids.numel(),) + tuple(layer.shape[1:]), layer.dtype, layer.device, stream)
     check(lib().sca_launch_kv_gather(layer.data_ptr(), block_ids.data_ptr(), block_ids.numel(),
                                      out.data_ptr(), C.byref(shape), layer.element_size(),
                                      _stream_ptr(stream)))

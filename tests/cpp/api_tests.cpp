@@ -504,6 +504,51 @@ TEST(Streams, FlashAndDecodeOnANonBlockingStream) {
     cudaStreamDestroy(raw);
 }
 
+// Decode calls on two streams without an order between them run at the same time: each needs partials of its own.
+TEST(Streams, DecodeOnTwoStreamsAtOnce) {
+    auto dev = Gpu();
+    if (!dev) SKIP_TEST("no CUDA device");
+    cudaStream_t raw[2] = {};
+    for (cudaStream_t& s : raw) ASSERT_TRUE(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess);
+    sci::Stream streams[2] = {sci::Stream(raw[0]), sci::Stream(raw[1])};
+    const int64_t b = 4, hq = 32, hkv = 8, skv = 6000, d = 128;
+    std::vector<sci::Tensor> q, k, v;
+    std::vector<std::vector<float>> alone;
+    for (int i = 0; i < 2; ++i) {
+        auto make = [&](int64_t heads, int64_t seq, uint32_t seed) {
+            const Encoded e = Encode(RandomFloats(size_t(b * heads * seq * d), seed), DType::kFloat16);
+            return ToDevice({b, heads, seq, d}, DType::kFloat16, e.bytes, *dev);
+        };
+        q.push_back(make(hq, 1, 48000 + i));
+        k.push_back(make(hkv, skv, 48010 + i));
+        v.push_back(make(hkv, skv, 48020 + i));
+    }
+    dev->synchronize();
+    auto run = [&](int i) {
+        sca::AttentionConfig cfg;
+        cfg.causal = true;
+        cfg.num_splits = 16;  // partials in scratch
+        cfg.stream = &streams[i];
+        return sca::decode_attention(q[i], k[i], v[i], cfg);
+    };
+    for (int i = 0; i < 2; ++i) {
+        const auto r = run(i);
+        ASSERT_TRUE(r.ok());
+        dev->synchronize();
+        alone.push_back(ReadFloats(r->out));
+    }
+    for (int rep = 0; rep < 20; ++rep) {
+        std::vector<sci::Result<sca::AttentionResult>> results;
+        for (int i = 0; i < 6; ++i) results.push_back(run(i % 2));
+        dev->synchronize();
+        for (int i = 0; i < 6; ++i) {
+            ASSERT_TRUE(results[i].ok());
+            EXPECT_TRUE(ReadFloats(results[i]->out) == alone[i % 2]);
+        }
+    }
+    for (cudaStream_t s : raw) cudaStreamDestroy(s);
+}
+
 TEST(Flash, VarlenPackedBatches) {
     auto dev = Gpu();
     if (!dev) SKIP_TEST("no CUDA device");
