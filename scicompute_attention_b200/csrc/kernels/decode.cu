@@ -23,6 +23,7 @@
 //
 // Algorithmic HBM traffic per token and kv head: 2 * D * sizeof(T) bytes (K row + V row), read once.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -711,11 +712,32 @@ cudaLaunchConfig_t ClusterConfig(unsigned grid, int cluster, int smem_bytes, cud
     return cfg;
 }
 
+// The answer of an occupancy query, kept per device. `ask` returns a negative number when the device cannot say; that is
+// not kept. Threads that ask at the same time store the same number.
+class PerDevice {
+public:
+    template <typename Ask>
+    int Get(Ask ask) {
+        int device = 0;
+        const bool kept = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < kMaxDevices;
+        if (kept) {
+            if (const int n = answers_[device].load(std::memory_order_relaxed); n != 0) return n - 1;
+        }
+        const int n = ask();
+        if (kept && n >= 0) answers_[device].store(n + 1, std::memory_order_relaxed);
+        return n;
+    }
+
+private:
+    static constexpr int kMaxDevices = 64;
+    std::atomic<int> answers_[kMaxDevices] = {};  // answer + 1, 0 = not asked yet
+};
+
 // CTAs of the decode kernels that stay resident together.
 template <typename T, int D, bool kPaged, bool kHi>
 int64_t ResidentCtas() {
-    static int resident_per_sm = 0;  // per instantiation; the same on every device of one model
-    if (resident_per_sm == 0) {
+    static PerDevice per_sm;  // per instantiation
+    const int resident_per_sm = per_sm.Get([] {
         int n = 0;
         // the query answers for the shared memory the kernel is allowed at that point
         const void* fn = reinterpret_cast<const void*>(&decode_partial_kernel<T, D, kPaged, kHi>);
@@ -723,11 +745,11 @@ int64_t ResidentCtas() {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_partial_kernel<T, D, kPaged, kHi>, kThreads,
                                                           DecodeGeom<D>::kSmemBytes) != cudaSuccess || n < 1) {
             cudaGetLastError();
-            n = 1;
+            return -1;
         }
-        resident_per_sm = n;
-    }
-    return static_cast<int64_t>(SmCount()) * resident_per_sm;
+        return n;
+    });
+    return static_cast<int64_t>(SmCount()) * std::max(1, resident_per_sm);
 }
 // Steps of the longest sequence the call may hold, as far as the host knows.
 template <bool kPaged>
@@ -739,18 +761,17 @@ int64_t MostSteps(const ScaDecodeFwdParams& p) {
 // Clusters of `cluster` CTAs of decode_cluster_kernel that run at the same time (0 when the device cannot say).
 template <typename T, int D, bool kPaged, bool kHi>
 int64_t ResidentClusters(int cluster) {
-    static int resident[kMaxCluster + 1] = {};  // per instantiation; the same on every device of one model
-    if (resident[cluster] == 0) {
+    static PerDevice resident[kMaxCluster + 1];  // per instantiation
+    return std::max(0, resident[cluster].Get([cluster] {
         cudaLaunchAttribute attr{};
         cudaLaunchConfig_t cfg = ClusterConfig(static_cast<unsigned>(cluster), cluster, DecodeGeom<D>::kSmemBytes, nullptr, &attr);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, decode_cluster_kernel<T, D, kPaged, kHi>, &cfg) != cudaSuccess) {
             cudaGetLastError();
-            n = 0;
+            return -1;
         }
-        resident[cluster] = n > 0 ? n : -1;
-    }
-    return resident[cluster] > 0 ? resident[cluster] : 0;
+        return n;
+    }));
 }
 
 // Whether the one-launch kernel is the faster one for `units` (sequence, kv head, head chunk) columns of `steps` steps
