@@ -77,21 +77,20 @@ def _empty(shape, dtype, device, stream=None) -> torch.Tensor:
         return torch.empty(shape, dtype=dtype, device=device)
 
 
-def _is_capturing(stream) -> bool:
-    if stream is None:
-        return torch.cuda.is_current_stream_capturing()
-    with _on(stream):
-        return torch.cuda.is_current_stream_capturing()
-
-
-def acquire_scratch_fp32(elements: int, device: torch.device, kind: int = 1, *, stream=None) -> torch.Tensor:
+def acquire_scratch_fp32(elements: int, device: torch.device, kind: int = 1, *, stream=None, handle: int | None = None) -> torch.Tensor:
     """Grow-only fp32 scratch of this thread per (device, kind, stream), so that calls that may overlap on the GPU never
     share it; same growth rule as the reference's pool (src/runtime/scratch_pool.cpp:38-60): 1.25 x request + 1024
-    elements. A call that is being captured gets memory of the graph's own pool: no graph points into this one."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    if _is_capturing(stream):
+    elements. A call that is being captured gets memory of the graph's own pool: no graph points into this one.
+    `handle` is the launch's stream handle where the caller has it already."""
+    if stream is None:
+        capturing = torch.cuda.is_current_stream_capturing()
+    else:
+        with _on(stream):
+            capturing = torch.cuda.is_current_stream_capturing()
+    if capturing:
         return _empty(elements, torch.float32, device, stream)
-    key = (idx, kind, _stream_ptr(stream))
+    idx = device.index
+    key = (idx if idx is not None else torch.cuda.current_device(), kind, _stream_ptr(stream) if handle is None else handle)
     pool = _scratch.pool
     cur = pool.get(key)
     if cur is None or cur.numel() < elements:
@@ -185,36 +184,36 @@ def decode_attention(q, k, v, *, scale=None, num_splits: int = 0, layout: str = 
         raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
     if hq % hkv != 0:
         raise _lib.ScaError(4, f"num_heads={hq} % num_kv_heads={hkv} != 0")
-    splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
+    device, handle = q.device, _stream_ptr(stream)
+    splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(device))
     base = b * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
-    out = _empty((b, hq, 1, d), q.dtype, q.device, stream)
+    ws = acquire_scratch_fp32(base * (2 + d), device, stream=stream, handle=handle)
+    out = _empty((b, hq, 1, d), q.dtype, device, stream)
 
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-    p.partial_m = ws.data_ptr()
-    p.partial_l = ws.data_ptr() + 4 * base
-    p.partial_o = ws.data_ptr() + 8 * base
+    scratch = ws.data_ptr()
+    p.partial_m, p.partial_l, p.partial_o = scratch, scratch + 4 * base, scratch + 8 * base
     p.batch, p.num_heads, p.num_kv_heads, p.seq_kv, p.head_dim, p.num_splits = b, hq, hkv, skv, d, splits
     p.q_stride = DecodeStrides(*_strides(layout, 1, hq, d))
     p.k_stride = DecodeStrides(*_strides(layout, skv, hkv, d))
     p.v_stride = p.k_stride
-    p.o_stride = DecodeStrides(*_strides("bhsd", 1, hq, d))
+    p.o_stride = DecodeStrides(hq * d, d, d)
     p.scale = effective_scale(scale, d)
     p.dtype = dtype_id(q.dtype)
     p.page_table = None
     p.seq_lens = seq_lens.data_ptr() if seq_lens is not None else None
-    return _launch_decode(p, num_splits, stream, out, return_stats)
+    return _launch_decode(p, num_splits, handle, out, return_stats)
 
 
-def _launch_decode(p, num_splits, stream, out, return_stats):
+def _launch_decode(p, num_splits, handle, out, return_stats):
     """An explicit split count asks for that many partials in the scratch; otherwise the size of the call decides."""
-    cluster = C.c_int32(0)
+    cluster = C.c_int32(0) if return_stats else None
     if num_splits > 0:
         launch = lib().sca_launch_decode_splitk_paged if p.page_table else lib().sca_launch_decode_splitk
-        check(launch(C.byref(p), _stream_ptr(stream)))
+        check(launch(C.byref(p), handle))
     else:
-        check(lib().sca_launch_decode_auto(C.byref(p), C.byref(cluster), _stream_ptr(stream)))
+        check(lib().sca_launch_decode_auto(C.byref(p), cluster, handle))
     if not return_stats:
         return out
     # num_splits: pieces a sequence is cut into at most; cluster: CTAs per cluster of the one-launch kernel, 0 = two kernels
@@ -246,20 +245,20 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
         raise _lib.ScaError(4, "page_table must be int32 [num_seqs, max_blocks_per_seq]")
     max_blocks = page_table.shape[1]
     upper = nblk * bs
+    device, handle = q.device, _stream_ptr(stream)
     if num_splits > 0:
         splits = min(num_splits, MAX_SPLITS)
     else:
         splits = paged_splits_for(typical_len if typical_len > 0 else min(upper, max_blocks * bs), s, hkv,
-                                  hq // hkv, sm_count(q.device), longest_len)
+                                  hq // hkv, sm_count(device), longest_len)
     base = s * hq * splits
-    ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
-    out = _empty((s, hq, 1, d), q.dtype, q.device, stream)
+    ws = acquire_scratch_fp32(base * (2 + d), device, stream=stream, handle=handle)
+    out = _empty((s, hq, 1, d), q.dtype, device, stream)
 
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr()
-    p.partial_m = ws.data_ptr()
-    p.partial_l = ws.data_ptr() + 4 * base
-    p.partial_o = ws.data_ptr() + 8 * base
+    scratch = ws.data_ptr()
+    p.partial_m, p.partial_l, p.partial_o = scratch, scratch + 4 * base, scratch + 8 * base
     p.batch, p.num_heads, p.num_kv_heads, p.seq_kv, p.head_dim, p.num_splits = s, hq, hkv, upper, d, splits
     p.q_stride = DecodeStrides(hq * d, d, d)
     p.o_stride = DecodeStrides(hq * d, d, d)
@@ -274,7 +273,7 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
     if not p.page_table:
         raise _lib.ScaError(4, "paged attention: null page table")
     p.block_size, p.max_blocks_per_seq, p.num_kv_blocks = bs, max_blocks, nblk
-    return _launch_decode(p, num_splits, stream, out, return_stats)
+    return _launch_decode(p, num_splits, handle, out, return_stats)
 
 
 def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
@@ -289,9 +288,8 @@ def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     triples = _empty((b * hq, 2 + d), torch.float32, q.device, stream)
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), None
-    p.partial_m = ws.data_ptr()
-    p.partial_l = ws.data_ptr() + 4 * base
-    p.partial_o = ws.data_ptr() + 8 * base
+    scratch = ws.data_ptr()
+    p.partial_m, p.partial_l, p.partial_o = scratch, scratch + 4 * base, scratch + 8 * base
     p.batch, p.num_heads, p.num_kv_heads, p.seq_kv, p.head_dim, p.num_splits = b, hq, hkv, skv, d, splits
     p.q_stride = DecodeStrides(*_strides("bhsd", 1, hq, d))
     p.k_stride = DecodeStrides(*_strides("bhsd", skv, hkv, d))
@@ -314,9 +312,8 @@ def decode_partials(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
     p = DecodeFwdParams()
     p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), None
-    p.partial_m = ws.data_ptr()
-    p.partial_l = ws.data_ptr() + 4 * base
-    p.partial_o = ws.data_ptr() + 8 * base
+    scratch = ws.data_ptr()
+    p.partial_m, p.partial_l, p.partial_o = scratch, scratch + 4 * base, scratch + 8 * base
     p.batch, p.num_heads, p.num_kv_heads, p.seq_kv, p.head_dim, p.num_splits = b, hq, hkv, skv, d, splits
     p.q_stride = DecodeStrides(*_strides("bhsd", 1, hq, d))
     p.k_stride = DecodeStrides(*_strides("bhsd", skv, hkv, d))

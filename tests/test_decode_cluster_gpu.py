@@ -11,14 +11,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dt,batch,hq,hkv,skv,d,cluster", [
-    (ol.DT_BF16, 1, 8, 8, 1, 128, 8),       # one key: seven CTAs of every cluster hold nothing
-    (ol.DT_F16, 1, 4, 1, 449, 64, 8),       # 8 steps for 8 CTAs, the last one with a single key
-    (ol.DT_BF16, 1, 32, 8, 1000, 128, 8),
-    (ol.DT_BF16, 6, 32, 8, 900, 128, 4),
-    (ol.DT_F16, 16, 32, 8, 500, 128, 2),
-    (ol.DT_BF16, 2, 32, 1, 700, 128, 8),    # two head chunks of 16 query heads
-    (ol.DT_F16, 1, 12, 1, 130, 96, 8),      # 12 heads: both row halves, one of them ragged
-    (ol.DT_BF16, 2, 8, 8, 300, 256, 8),     # one CTA per SM
+    (ol.DT_BF16, 1, 8, 8, 1, 128, (8,)),       # one key: seven CTAs of every cluster hold nothing
+    (ol.DT_F16, 1, 4, 1, 449, 64, (8,)),       # 8 steps for 8 CTAs, the last one with a single key
+    (ol.DT_BF16, 1, 32, 8, 1000, 128, (8,)),
+    (ol.DT_BF16, 6, 32, 8, 900, 128, (4,)),
+    (ol.DT_F16, 16, 32, 8, 500, 128, (2,)),
+    (ol.DT_BF16, 2, 32, 1, 700, 128, (8,)),    # two head chunks of 16 query heads
+    (ol.DT_F16, 1, 12, 1, 130, 96, (8,)),      # 12 heads: both row halves, one of them ragged
+    (ol.DT_BF16, 2, 8, 8, 300, 256, (4, 8)),   # one CTA per SM: 16 clusters of 8 fit or not, by the SMs per GPC
 ])
 def test_cluster_decode_matches_the_oracle(dt, batch, hq, hkv, skv, d, cluster):
     import torch
@@ -28,7 +28,7 @@ def test_cluster_decode_matches_the_oracle(dt, batch, hq, hkv, skv, d, cluster):
     vb, vd = H.uniform_inputs((batch, hkv, skv, d), 74002, dt)
     q, k, v = H.to_device(qb, dt), H.to_device(kb, dt), H.to_device(vb, dt)
     out, stats = ops.decode_attention(q, k, v, return_stats=True)
-    assert stats["cluster"] == cluster
+    assert stats["cluster"] in cluster
     H.check_close(H.to_host_f32(out), ol.attention_f64(qd, kd, vd, causal=True), dt)
     # ragged, an empty sequence among them: its rows are zero
     lens = np.array([(skv * (i + 1)) // batch for i in range(batch)], dtype=np.int32)
