@@ -780,11 +780,25 @@ int64_t ResidentClusters(int cluster) {
 // 90; B=4, S=4000 21.0 / 16.5; B=16, S=2000 29.9 / 27.5, paged with lengths from 250 to 2000 25.6 / 27.7; paged B=4, 500
 // to 4000 22.6 / 16.9, B=8 26.9 / 27.2. A step costs more the more CTAs share the memory; the schedule works on what a
 // ragged batch holds (0.55 of the bound is assumed), a cluster waits for the longest sequence.
-bool ClusterIsFaster(int64_t units, int64_t steps, int cluster, int64_t resident, bool ragged) {
+// Other head dims, from 1056 calls of D=32 to 256 (batch 1 to 32, 60 to 16000 tokens):
+//   * above 128 one CTA fills an SM and a step is up to twice the bytes, so that clusters which leave SMs idle lose to the
+//     wave: D=256, 8 kv heads, B=2, S=4000 24.2 / 20.5 (one launch / schedule), B=1, S=8000 23.1 / 21.9. Two times fitted
+//     at 192 and 256, with 0.15 us per slot for the merge and 0.7 or 0.8 of the bound for a ragged batch. Groups of more than 8
+//     heads pay for both row halves in the exchange; clusters of less than 8 do not make up for it in short streams,
+//     unless long sequences are ragged (D=256, 16 / 1 heads, B=16, S=4000 32.8 / 24.5; B=32, S=4000 34.4 / 38.5);
+//   * below 128 the memory is the limit once the stream takes 35 us, and the wave uses it better: D=64, B=32, S=8000 90 / 83.
+bool ClusterIsFaster(int64_t units, int64_t steps, int cluster, int64_t resident, bool ragged, int head_dim, bool hi, int64_t splits) {
     const double busy = static_cast<double>(units * cluster) / resident;
-    const double one_launch = 4.8 + static_cast<double>((steps + cluster - 1) / cluster) * (0.55 + 1.1 * busy);
-    const double wave = static_cast<double>(units * steps) * (ragged ? 0.55 : 1.0) / resident;
-    return one_launch < 11.5 + 1.55 * std::max(1.0, wave);
+    const double share = static_cast<double>((steps + cluster - 1) / cluster);
+    const double waves = static_cast<double>(units * steps) / resident;
+    const double stream_us = static_cast<double>(units * steps) * kSpan * head_dim * 4 / 6.5e6;
+    if (head_dim > 128) {
+        if (hi && cluster < kMaxCluster && steps > 1 && (!ragged || steps < 8) && stream_us < 12.0) return false;
+        const double one_launch = (hi ? 3.5 + 0.027 * head_dim : 5.4) + share * (0.95 + 0.3 * busy);
+        return one_launch < (hi ? 11.0 : 7.5) + 1.5 * std::max(1.0, waves * (!ragged ? 1.0 : hi ? 0.8 : 0.7)) + 0.15 * static_cast<double>(splits);
+    }
+    if (head_dim < 128 && stream_us > 35.0) return false;
+    return 4.8 + share * (0.55 + 1.1 * busy) < 11.5 + 1.55 * std::max(1.0, waves * (ragged ? 0.55 : 1.0));
 }
 
 // Launches decode_cluster_kernel if it is the kernel for this call; *taken = its CTAs per cluster, 0 if it is not.
@@ -798,7 +812,7 @@ int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     // as many CTAs per cluster as let all clusters run at the same time (B=8, S=1000: 11.6 us with 4, 16.4 with 8 in turns)
     int cluster = kMaxCluster;
     while (cluster >= 2 && units > ResidentClusters<T, D, kPaged, kHi>(cluster)) cluster /= 2;
-    if (cluster < 2 || !ClusterIsFaster(units, steps, cluster, resident, p.seq_lens != nullptr)) cluster = 0;
+    if (cluster < 2 || !ClusterIsFaster(units, steps, cluster, resident, p.seq_lens != nullptr, D, kHi, p.num_splits)) cluster = 0;
     *taken = cluster;
     if (cluster == 0) return SCA_OK;
     cudaLaunchAttribute attr{};

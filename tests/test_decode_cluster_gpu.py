@@ -64,6 +64,19 @@ def test_cluster_paged_decode_with_holes(block_size, seqs, longest):
     H.check_close(H.to_host_f32(out), expect.reshape(seqs, hq, 1, d), dt)
 
 
+@pytest.mark.parametrize("batch,hq,hkv,skv,d", [
+    (2, 8, 8, 4000, 256),    # 24.2 us on clusters of 4, 20.5 with the schedule
+    (16, 16, 1, 4000, 256),  # 32.8 / 24.5
+    (16, 8, 8, 16000, 64),   # 86.1 / 81.5
+])
+def test_calls_that_the_schedule_does_faster_stay_with_it(batch, hq, hkv, skv, d):
+    import torch
+    from scicompute_attention_b200 import ops
+    q = torch.zeros(batch, hq, 1, d, device="cuda", dtype=torch.bfloat16)
+    k = torch.zeros(batch, hkv, skv, d, device="cuda", dtype=torch.bfloat16)
+    assert ops.decode_attention(q, k, k, return_stats=True)[1]["cluster"] == 0
+
+
 @pytest.mark.parametrize("paged", [False, True])
 @pytest.mark.parametrize("batch,skv,splits", [(1, 129, 3), (3, 700, 1), (2, 64, 16)])
 def test_a_call_that_names_its_splits_leaves_its_partials(batch, skv, splits, paged):
