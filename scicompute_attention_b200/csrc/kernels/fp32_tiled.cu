@@ -14,6 +14,7 @@
 //   * rows in shared memory are padded by 16 bytes: the operand loads are free of bank conflicts;
 //   * K_j+1 is fetched (16-byte cp.async, zero-filled past the end) as soon as S_j is complete, V_j+1 after P_j V_j.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -296,28 +297,55 @@ int LaunchF32(F32Params p, int64_t bh, cudaStream_t stream) {
     return CheckLaunch("fp32_tiled_attention_kernel", stream);
 }
 
+// One CTA per SM at a time. A wave of 32-row tiles takes 0.83 of the time of a wave of 64-row tiles (93 against 112
+// us at H=8, S=1024, D=128: the shared operand loads are spread over half the products), so the flat tile pays
+// where it saves waves or where one wave holds either (H=8, S=256: 29.9 us flat, 35.1 tall).
+struct F32Tiling {
+    bool flat;
+    int64_t waves;
+};
+F32Tiling TilingFor(int64_t bh, int64_t seq_q) {
+    const int64_t sms = SmCount();
+    const int64_t tall = (bh * ((seq_q + 63) / 64) + sms - 1) / sms;
+    const int64_t flat = (bh * ((seq_q + 31) / 32) + sms - 1) / sms;
+    return flat * 5 < tall * 6 ? F32Tiling{true, flat} : F32Tiling{false, tall};
+}
+
+// Whether one warp per query row is faster: a few rows or keys under very many heads, whose tiles are mostly padding. Both
+// times in us, fitted to 490 calls (D=32 to 256; 1, 8, 32 and 512 heads in all; 1x1 to 300x300, 1x1000 and 130x1000 query
+// rows and keys; warp per row / tiled): 512 heads, D=128 1x1 18 / 34, 17x17 29 / 36, 33x33 85 / 47, 1x64 39 / 35; D=256 1x64
+// 39 / 59, 4x200 115 / 180, 33x33 89 / 71, 1x1000 1064 / 738; up to 148 tiles the tiled kernel wins at every size.
+bool WarpPerRowIsFaster(const ScaFlashFwdParams& f) {
+    const int64_t bh = f.batch * f.num_heads;
+    const F32Tiling tiling = TilingFor(bh, f.seq_q);
+    if (tiling.waves <= 1 || f.head_dim <= 32) return false;
+    const double d = static_cast<double>(f.head_dim), keys = static_cast<double>(f.seq_kv), rows = static_cast<double>(f.seq_q);
+    const double tiles = std::ceil(keys / (f.head_dim <= 128 ? 64.0 : 32.0));
+    const double tiled = static_cast<double>(tiling.waves) * (3.5 + (f.head_dim <= 128 ? 0.042 : 0.0235) * d * tiles) * (tiling.flat ? 1.0 : 1.2);
+    // a warp walks its keys one by one, more slowly where K and V do not fit into L2; many rows share the issue slots
+    const double kv_bytes = static_cast<double>(f.batch * f.num_kv_heads) * keys * d * 8.0;
+    const double chain = 6.0 + keys * (f.head_dim <= 96 ? 0.35 : 0.5) * (kv_bytes > 130e6 ? 2.1 : 1.0);
+    const double pairs = static_cast<double>(bh) * rows * (keys - (f.causal ? (rows - 1.0) / 2.0 : 0.0)) * 1e-3;
+    const double warp_per_row = std::max({chain, 18.0 + 0.07 * pairs, pairs * (f.head_dim <= 64 ? 0.13 : 0.15)});
+    return tiled > 1.05 * warp_per_row;
+}
+
 template <int D>
 int LaunchF32ForDim(const F32Params& p, int64_t bh, cudaStream_t stream) {
-    // One CTA per SM at a time. A wave of 32-row tiles takes 0.83 of the time of a wave of 64-row tiles (93 against 112
-    // us at H=8, S=1024, D=128: the shared operand loads are spread over half the products), so the flat tile pays
-    // where it saves waves or where one wave holds either (H=8, S=256: 29.9 us flat, 35.1 tall).
-    const int64_t sms = SmCount();
-    const int64_t tall = (bh * ((p.seq_q + 63) / 64) + sms - 1) / sms;
-    const int64_t flat = (bh * ((p.seq_q + 31) / 32) + sms - 1) / sms;
-    return flat * 5 < tall * 6 ? LaunchF32<D, 2>(p, bh, stream) : LaunchF32<D, 4>(p, bh, stream);
+    return TilingFor(bh, p.seq_q).flat ? LaunchF32<D, 2>(p, bh, stream) : LaunchF32<D, 4>(p, bh, stream);
 }
 
 }  // namespace
 
-// The calls the tiled kernel takes: 16-byte accesses to every row, 32-bit row indices. It is the faster one at every size
-// measured (S = 1 to 1300); unaligned rows and the 16-bit types stay with the one-warp-per-row kernel.
+// The calls the tiled kernel takes: 16-byte accesses to every row, 32-bit row indices, tiles that are not mostly padding.
+// The others and the 16-bit types stay with the one-warp-per-row kernel.
 bool Fp32TiledTakes(const ScaFlashFwdParams& f) {
     const int64_t strides[] = {f.q_sb, f.q_sh, f.q_ss, f.k_sb, f.k_sh, f.k_ss, f.v_sb, f.v_sh, f.v_ss, f.o_sb, f.o_sh, f.o_ss};
     for (const int64_t s : strides) {
         if (s % 4 != 0) return false;
     }
     return f.dtype_id == SCA_DTYPE_F32 && Aligned16(f.q) && Aligned16(f.k) && Aligned16(f.v) && Aligned16(f.out) &&
-           f.seq_q < 0x7fffff00LL && f.seq_kv < 0x7fffff00LL && f.batch * f.num_heads < 0x7fffffffLL;
+           f.seq_q < 0x7fffff00LL && f.seq_kv < 0x7fffff00LL && f.batch * f.num_heads < 0x7fffffffLL && !WarpPerRowIsFaster(f);
 }
 
 int LaunchFp32Tiled(const ScaFlashFwdParams& f, cudaStream_t stream) {

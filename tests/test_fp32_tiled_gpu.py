@@ -22,6 +22,7 @@ pytestmark = pytest.mark.gpu
     (256, 2, 1, 40, 97, True, "bhsd"),      # 32-key tiles
     (160, 2, 2, 64, 33, False, "bhsd"),
     (224, 2, 1, 17, 65, True, "bshd"),
+    (256, 256, 64, 17, 17, True, "bhsd"),   # tiles that would be mostly padding: one warp per row
 ])
 def test_tiled_fp32_matches_the_oracle(d, hq, hkv, sq, skv, causal, layout):
     from scicompute_attention_b200 import ops
