@@ -176,8 +176,9 @@ public:
 };
 
 // =================================================================================================
-// tiled: short-sequence backend of the dispatcher table (seq_kv <= 128). Same SIMT kernel; keeps the
-// reference's head_dim <= 128 contract and answers with the warp-per-row geometry it really uses.
+// tiled: short-sequence backend of the dispatcher table (seq_kv <= 128), on sca_launch_simt_forward; keeps the reference's
+// head_dim <= 128 contract. The geometry it answers with is that of the warp-per-row kernel, which takes the 16-bit types;
+// fp32 calls mostly run on larger tiles whose size the launch picks (fp32_tiled.cu).
 // =================================================================================================
 constexpr int64_t kTiledMaxHeadDim = 128;
 

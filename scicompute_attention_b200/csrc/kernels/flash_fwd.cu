@@ -51,15 +51,8 @@ using namespace sm100;
 
 constexpr int kBlockM = 128;
 
-template <typename T>
-__device__ __forceinline__ float2 Unpack2(uint32_t v);
-template <>
-__device__ __forceinline__ float2 Unpack2<__nv_bfloat16>(uint32_t v) {
+__device__ __forceinline__ float2 UnpackBf16(uint32_t v) {
     return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-}
-template <>
-__device__ __forceinline__ float2 Unpack2<__half>(uint32_t v) {
-    return __half22float2(*reinterpret_cast<const __half2*>(&v));
 }
 // bf16 inputs: the probabilities are handed to the P V product as fp16, not bf16. They lie in [0, 2^8], where fp16
 // resolves 2^-11 relative against 2^-8 - with bf16 the rounding of P alone costs about 1e-3 of relative L2 error in
@@ -159,7 +152,11 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t ring_smem = smem_base + QT * G::kQTileBytes;
     const uint32_t bar_base = ring_smem + G::kSlots * G::kKvTileBytes;
     auto bar = [&](int i) { return bar_base + 8u * i; };
-    // barrier indices
+    // Barriers. A wait names a phase by its parity, so it is sound where the role knows that the phase before is over and
+    // that the one after cannot be. For all but o_done the role waits for every phase in turn, and the next one takes an
+    // arrival that this role (or one that waits for it) makes later. o_done is waited for where O moves and at the end of
+    // an item only. The phase before it: its product went out ahead of scores the softmax has waited for since. The phase
+    // after: its product wants a P that this group has yet to write.
     constexpr int kQFull = 0;                       // [2]
     constexpr int kKvFull = 2;                      // [2 * kSlots], see RingFullBarrier
     constexpr int kKvEmpty = kKvFull + 2 * G::kSlots;   // [kSlots]
@@ -592,7 +589,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     uint32_t* word = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const float2 f = Unpack2<__nv_bfloat16>(word[e]);
+                        const float2 f = UnpackBf16(word[e]);
                         // one instruction for both lanes; values beyond the fp16 range saturate instead of becoming inf
                         asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(word[e]) : "f"(f.y), "f"(f.x));
                     }
@@ -705,7 +702,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (move) m_ref = mx;
                     }
                 }
-                // Exponentials of columns [32 * first, 32 * end): P to tensor memory, returns their sum. With kBehind the
+                // Exponentials of columns [32 * first, 32 * end): P to tensor memory, their sum onto sum[]. With kBehind the
                 // additions and conversions of a batch of 8 come behind the exponentials of the next one: a warp alone on
                 // its scheduler takes 1190 clocks for 128 exponentials that way and 1331 when it waits for each batch
                 // (1030 is the rate of the special-function unit), two warps 2070 and 2110. D=128, where the groups meet
@@ -911,7 +908,7 @@ struct VarlenWork {
     int64_t workspace_bytes;
 };
 
-// Query heads that share a tile: the largest power of two that divides the GQA group, at most kMaxPack.
+// log2 of the query heads that share a tile: the largest power of two that divides the GQA group, at most 1 << kMaxPackShift.
 constexpr int kMaxPackShift = 2;
 int PackShift(int64_t group) {
     int shift = 0;
@@ -920,7 +917,7 @@ int PackShift(int64_t group) {
 }
 
 int64_t VarlenWorkspaceBytes(int64_t num_seqs, int64_t total_q) {
-    // one int4 per sequence + one int2 per work item and packed head; an item covers at least kBlockM >> kMaxPackShift tokens
+    // one int4 per sequence + one int2 per (sequence, query block); a block covers at least kBlockM >> kMaxPackShift tokens
     return num_seqs * 16 + (total_q / (kBlockM >> kMaxPackShift) + num_seqs) * 8 + 64;
 }
 

@@ -30,7 +30,6 @@ struct F32Geom {
     static constexpr int kBM = 16 * RT;             // 4 warps x 4 row groups x RT rows
     static constexpr int kBN = D <= 128 ? 64 : 32;  // keys per tile and group
     static constexpr int kCT = kBN / 8;             // score columns per thread
-    static constexpr int kDT = D / 8;               // output columns per thread
     static constexpr int kLd = D + 4;               // padded row of Q and K
     static constexpr int kPLd = kBN + 4;            // padded row of P
     static constexpr int kQFloats = kBM * kLd;
