@@ -916,6 +916,35 @@ int PackShift(int64_t group) {
     return shift;
 }
 
+// Whether query heads should share tiles (us in a lasting load, heads alone / four to a tile, 32 / 8 heads).
+// They fill the rows that a ragged end leaves empty, and they let both tiles of a causal item need the same KV tiles: D=128,
+// S=3000 with B=1 94.5 / 92.5, B=4 350 / 342; D=64, B=8, S=1024 84 / 80; without a mask that is worth nothing. But the four
+// heads of a kv head no longer stand side by side in the work list, each of them at the same key: with many kv heads or
+// much K/V in flight that costs energy and bandwidth: D=128, B=4, S=4096 595 / 607 (no mask 1090 / 1134), B=8, S=4096 1209 /
+// 1276, B=16, S=2048 698 / 767, B=32, S=256 60 / 66.5; D=256, B=8, S=1024 without a mask 348 / 377.
+bool PackingPays(const ScaFlashFwdParams& f, int shift) {
+    const int64_t tokens = kBlockM >> shift;
+    const int64_t alone = (f.seq_q + kBlockM - 1) / kBlockM * kBlockM, packed = (f.seq_q + tokens - 1) / tokens * tokens;
+    if (alone * 100 > packed * 107) return true;  // B=8, S=700 without a mask 106 / 97
+    const int64_t pairs = f.batch * f.num_kv_heads;
+    return f.causal && pairs <= 64 && pairs * f.seq_kv * f.head_dim * 4 <= 55000000;
+}
+// The same for a packed batch, whose ends are ragged and whose entries are in the order of their weight in any case:
+// D=128, 10 sequences of 64 to 4096 594 / 580, 64 of 100 to 900 378 / 361. Long causal ones with much K/V lose: 16 of 4096
+// 2467 / 2656, 32 of 2000 1394 / 1494; not without a mask (24 of 3000 to 4000 5055 / 4989) nor at D=64 (2156 / 2108).
+bool PackingPays(const VarlenWork& vw, const ScaFlashFwdParams& f, int shift) {
+    const int64_t kv_bytes = f.seq_kv * f.num_kv_heads * f.head_dim * 4;
+    if (!f.causal || f.head_dim <= 64 || kv_bytes <= 150000000) return true;
+    const int64_t tokens = kBlockM >> shift;
+    int64_t alone = 0, packed = 0;
+    for (int64_t s = 0; s < vw.num_seqs; ++s) {
+        const int64_t rows = std::max<int64_t>(0, static_cast<int64_t>(vw.cu_q[s + 1]) - vw.cu_q[s]);
+        alone += (rows + kBlockM - 1) / kBlockM * kBlockM;
+        packed += (rows + tokens - 1) / tokens * tokens;
+    }
+    return alone * 100 > packed * 106;
+}
+
 int64_t VarlenWorkspaceBytes(int64_t num_seqs, int64_t total_q) {
     // one int4 per sequence + one int2 per (sequence, query block); a block covers at least kBlockM >> kMaxPackShift tokens
     return num_seqs * 16 + (total_q / (kBlockM >> kMaxPackShift) + num_seqs) * 8 + 64;
@@ -990,6 +1019,10 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
     // rows of a query tile: P heads x 128 / P tokens
     int pack_shift = PackShift(f.num_heads / f.num_kv_heads);
     int tiles_per_item = QT;
+    if (pack_shift > 0 && !(varlen == nullptr ? PackingPays(f, pack_shift)
+                                              : paged != nullptr || PackingPays(*varlen, f, pack_shift))) {
+        pack_shift = 0;
+    }
     if (varlen != nullptr) {
         while (pack_shift > 0 && VarlenListBytes(*varlen, (QT * kBlockM) >> pack_shift) > varlen->workspace_bytes) --pack_shift;
     }

@@ -16,6 +16,9 @@ pytestmark = pytest.mark.gpu
     (ol.DT_BF16, 1, 6, 2, 130, 257, 128, False, "bhsd"),   # a group of three: heads stay alone
     (ol.DT_F16, 1, 16, 2, 40, 100, 256, True, "bhsd"),     # eight heads in two packs of four
     (ol.DT_BF16, 1, 64, 8, 600, 600, 64, True, "bhsd"),    # more tiles than SMs: two per item
+    (ol.DT_BF16, 2, 8, 2, 257, 300, 128, False, "bhsd"),   # a row into the third tile, no mask: shared
+    (ol.DT_F16, 2, 8, 2, 384, 400, 128, False, "bshd"),    # whole tiles, no mask: every head alone
+    (ol.DT_BF16, 17, 8, 4, 256, 300, 64, True, "bhsd"),    # 68 kv heads and whole tiles: every head alone
 ])
 def test_packed_heads_match_the_oracle(dt, batch, hq, hkv, sq, skv, d, causal, layout):
     from scicompute_attention_b200 import ops
