@@ -162,10 +162,10 @@ class FlashWorkload(Workload):
         self.dtype_name, self.d, self.strong, self.B, self.S = dtype_name, head_dim, strong, batch, seq
         self.scaling = "strong" if strong else "weak"
         self.name = f"flash_prefill_causal_B{batch}_S{seq}_Hq{HQ}_Hkv{HKV}_D{head_dim}_{dtype_name}" + ("_strong" if strong else "")
-        # dram__bytes_read + dram__bytes_write of flash_fwd_sm100_kernel, ncu capture at B=1 scaled x4
-        # (profiles/flash_prefill_c2.md, _d64.md, _d256.md); the output mostly stays in L2 until after the kernel
-        captured = {128: 50.43e6 + 3.60e6, 64: 25.22e6 + 0.01e6, 256: 102.76e6 + 27.78e6}  # read + written at B=1
-        self.traffic_bytes = captured[head_dim] * batch if not strong else None
+        # dram__bytes_read + dram__bytes_write of flash_fwd_sm100_kernel, ncu capture of bf16 at B=4
+        # (profiles/flash_prefill_c2.md, _d64.md, _d256.md); part of the output stays in L2 until after the kernel
+        captured = {128: 297.0e6 + 102.3e6, 64: 101.3e6 + 33.1e6, 256: 1595.6e6 + 247.0e6}
+        self.traffic_bytes = captured[head_dim] * batch / 4 if not strong else None
 
     def setup(self, torch, device, seed, rank, world):
         from scicompute_attention_b200 import ops

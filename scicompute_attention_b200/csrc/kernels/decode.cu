@@ -18,7 +18,7 @@
 //     transposition of V is needed; XOR swizzles keep those loads bank-conflict free;
 //   * page tables are resolved once per token row by 16 lanes (one table read per row, broadcast
 //     by shuffle), never per element;
-//   * calls that do not fill the machine run in one launch: a cluster of CTAs takes each (sequence, kv head, head
+//   * calls that do not fill the machine run in one launch where the caller leaves the choice: a cluster of CTAs takes each (sequence, kv head, head
 //     chunk) and merges through distributed shared memory (decode_cluster_kernel).
 //
 // Algorithmic HBM traffic per token and kv head: 2 * D * sizeof(T) bytes (K row + V row), read once.

@@ -6,7 +6,7 @@
 // exp2, bottom-right aligned causal mask, GQA, optional log-sum-exp - on a Blackwell execution plan:
 //
 //   * one persistent CTA per SM walks a list of work items; an item is 256 query rows of one batch element and kv
-//     head - up to four query heads that share the kv head, interleaved token by token - as two 128-row tiles that
+//     head - one query head, or up to four that share the kv head, interleaved token by token - as two 128-row tiles that
 //     ping-pong, so the tensor core works on one tile while the other tile's softmax runs;
 //   * warp 0 is the TMA producer: Q tiles once, then K_j, V_j, K_j+1, ... into a ring of 128-byte
 //     swizzled shared-memory slots, each guarded by a full/empty mbarrier pair. Loads are plain
