@@ -74,7 +74,9 @@ def _empty(shape, dtype, device, stream=None) -> torch.Tensor:
     if stream is None:
         return torch.empty(shape, dtype=dtype, device=device)
     with _on(stream):
-        return torch.empty(shape, dtype=dtype, device=device)
+        t = torch.empty(shape, dtype=dtype, device=device)
+    t.record_stream(torch.cuda.current_stream(device))  # the caller goes on with the result there
+    return t
 
 
 def acquire_scratch_fp32(elements: int, device: torch.device, kind: int = 1, *, stream=None, handle: int | None = None) -> torch.Tensor:

@@ -37,6 +37,24 @@ def test_the_work_list_lives_until_the_launch_on_its_stream_has_read_it(paged):
     del held
 
 
+def test_a_result_that_the_current_stream_still_reads_is_not_reused():
+    import torch
+    from scicompute_attention_b200 import ops
+    sets = [[_rand((1, h, 500, 128), 40 + 3 * i + j) for j, h in enumerate((8, 2, 2))] for i in range(2)]
+    expect = ops.flash_attention(*sets[0], causal=True)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    out = ops.flash_attention(*sets[0], causal=True, stream=side)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda._sleep(20_000_000)  # about 10 ms
+    kept = out.clone()
+    del out  # before the copy has run
+    for _ in range(4):
+        ops.flash_attention(*sets[1], causal=True, stream=side)
+    torch.cuda.synchronize()
+    assert torch.equal(kept, expect)
+
+
 def test_decode_on_two_streams_at_once_and_in_threads():
     import threading
     import torch
