@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstddef>
+#include <memory>
+#include <mutex>
 #include <string>
 
 #include "sca_b200.h"
@@ -22,7 +24,9 @@ const IAttentionBackend* PagedBackendInstance() noexcept;
 enum class ScratchKind : int { kScoresFp32 = 0, kDecodePartials = 1, kGeneric = 2, kCount = 3 };
 struct ScratchLease {
     float* data{nullptr};
-    sci::Tensor own;  // memory of this call alone
+    sci::Tensor own;                    // memory of this call alone
+    std::shared_ptr<std::mutex> mutex;  // of the pool's buffer: threads that launch on one stream take turns
+    std::unique_lock<std::mutex> turn;
 };
 sci::Result<ScratchLease> AcquireScratchFp32(ScratchKind kind, size_t elements, sci::Device& device, void* stream);
 sci::Status ReleaseScratch();

@@ -30,6 +30,7 @@ namespace {
 struct ScratchEntry {
     sci::Tensor buffer;
     size_t elements{0};
+    std::shared_ptr<std::mutex> mutex = std::make_shared<std::mutex>();  // held by the lease, from here to the launch
 };
 std::mutex& ScratchMutex() {
     static std::mutex m;
@@ -46,8 +47,10 @@ std::map<ScratchKey, ScratchEntry>& ScratchMap() {
 size_t g_scratch_peak_bytes = 0;
 
 // The streams that used an entry may be gone, so there is nothing to order its release on: wait for the device.
+// Called with the map locked; a lease never asks for the map, so waiting for one here ends.
 void ClearScratch() {
     for (auto& item : ScratchMap()) {
+        std::lock_guard<std::mutex> no_lease(*item.second.mutex);
         if (item.second.buffer.data() != nullptr) item.second.buffer.device().synchronize();
     }
     ScratchMap().clear();
@@ -65,7 +68,6 @@ sci::Result<ScratchLease> AcquireScratchFp32(ScratchKind kind, size_t elements, 
     };
     ScratchLease lease;
     const bool capturing = sci::StreamIsCapturing(stream);
-    std::lock_guard<std::mutex> lock(ScratchMutex());
     if (capturing) {
         lease.own = allocate(elements);
         lease.data = static_cast<float*>(lease.own.data());
@@ -73,8 +75,11 @@ sci::Result<ScratchLease> AcquireScratchFp32(ScratchKind kind, size_t elements, 
         return sci::Ok(std::move(lease));
     }
     const ScratchKey key{device.id(), static_cast<int>(kind), stream};
+    std::lock_guard<std::mutex> lock(ScratchMutex());
     if (ScratchMap().size() >= kMaxScratchEntries && ScratchMap().count(key) == 0) ClearScratch();
     ScratchEntry& entry = ScratchMap()[key];
+    lease.mutex = entry.mutex;
+    lease.turn = std::unique_lock<std::mutex>(*lease.mutex);
     if (entry.buffer.data() == nullptr || entry.elements < elements) {
         const size_t grown = static_cast<size_t>(static_cast<double>(elements) * 1.25) + 1024;
         entry.buffer = allocate(grown);  // inside the call's StreamOrderedScope: the old one is released in stream order

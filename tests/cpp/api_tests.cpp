@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <memory>
 #include <numeric>
+#include <thread>
 
 #include <cuda_runtime_api.h>
 
@@ -545,6 +546,26 @@ TEST(Streams, DecodeOnTwoStreamsAtOnce) {
             ASSERT_TRUE(results[i].ok());
             EXPECT_TRUE(ReadFloats(results[i]->out) == alone[i % 2]);
         }
+    }
+    // threads that launch on the same stream
+    std::vector<std::vector<float>> from_threads[2];
+    std::vector<std::thread> threads;
+    for (int i = 0; i < 2; ++i) {
+        threads.emplace_back([&, i] {
+            for (int rep = 0; rep < 50; ++rep) {
+                sca::AttentionConfig cfg;
+                cfg.causal = true;
+                cfg.num_splits = 16;
+                cfg.stream = &streams[0];
+                const auto r = sca::decode_attention(q[i], k[i], v[i], cfg);
+                cudaStreamSynchronize(raw[0]);
+                from_threads[i].push_back(r.ok() ? ReadFloats(r->out) : std::vector<float>());
+            }
+        });
+    }
+    for (std::thread& t : threads) t.join();
+    for (int i = 0; i < 2; ++i) {
+        for (const std::vector<float>& out : from_threads[i]) EXPECT_TRUE(out == alone[i]);
     }
     for (cudaStream_t s : raw) cudaStreamDestroy(s);
 }
