@@ -15,16 +15,14 @@
 //   * warp 1 issues every tcgen05.mma from one thread: S_t = Q_t K_j^T (both operands in shared
 //     memory, K-major) into tensor memory, and O_t += P_t V_j with P_t read from tensor memory and
 //     V_j as an MN-major shared-memory operand (no transposition of V anywhere);
-//   * warps 2-5 and 6-9 are the two softmax groups, one thread per query row: they read their S row from tensor
+//   * four warps per query tile are its softmax group, one thread per query row: they read their S row from tensor
 //     memory once, exponentiate against the reference point the row already has, keep the running sum in registers
-//     and write P back over S as packed 16-bit values, handed over in two pieces so that P V starts under the last
+//     and write P to tensor memory as packed 16-bit values, handed over in two pieces so that P V starts under the last
 //     exponentials. The reference point moves (and O and the sum are rescaled) only when a row exceeds it by more
 //     than 2^8; the final division by the row sum absorbs the stale reference point exactly;
-//   * bf16: one or two more warps rewrite each V tile in shared memory as fp16 (see PvFormat);
-//   * tensor memory: S_0 | S_1 | O_0 | O_1, 128 (or D) fp32 columns each, 512 columns in total;
-//   * head dims above 128 leave room for one query tile only (O needs 256 columns). There the scores of
-//     64-key tiles are double-buffered instead: S(j+1) is computed while the softmax of tile j runs, and
-//     S(j+2) follows P(j) V_j into the buffer P(j) came from.
+//   * bf16: two to four more warps rewrite each V tile in shared memory as fp16 (see PvFormat);
+//   * tensor memory, 512 columns: at D=128 S_0 | S_1 | O_0 | O_1 take them all and P_t lies over S_t, so that the next
+//     scores follow P V. Up to D=64, and above 128 with its one query tile, P_t has columns of its own (see FlashGeom).
 //
 // Packed variable-length batches run on the same kernel: the work list then holds (sequence, query block)
 // entries and every item carries its sequence's lengths and token offsets (see sca_launch_flash_varlen).
@@ -70,22 +68,35 @@ constexpr int kTmemColumns = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain: P stays <= 2^8
 
 // DP: padded head dim (64 / 128 / 256); QT: query tiles per CTA; BN: keys per KV tile.
-// 64 and 128 run two query tiles against 128-key tiles; 256 needs 256 TMEM columns for O, so it runs one
-// query tile against 64-key tiles (S 64 + O 256 columns).
+// 64 and 128 run two query tiles; 256 needs 256 TMEM columns for O, so it runs one.
 template <int DP, int QT, int BN>
 struct FlashGeom {
     static constexpr int kKBlocks = DP / 64;               // 64-element (128-byte) column blocks per row
     static constexpr int kQBlockBytes = kBlockM * 128;      // one column block of a query tile
-    static constexpr int kKvBlockBytes = BN * 128;          // one column block of a K or V tile
     static constexpr int kQTileBytes = kKBlocks * kQBlockBytes;
-    static constexpr int kKvTileBytes = kKBlocks * kKvBlockBytes;
-    static constexpr int kSlots = (DP == 64) ? 8 : 5;  // K/V ring
+    // K/V ring. A tile of D=256 takes two slots: K in halves of its columns, V in halves of its keys, each freed when its
+    // half of the products is done.
+    static constexpr int kParts = DP == 256 ? 2 : 1;
+    static constexpr int kKBlockBytes = BN * 128;           // one column block of K in a slot
+    static constexpr int kVKeys = BN / kParts;              // keys of V in a slot
+    static constexpr int kVBlockBytes = kVKeys * 128;       // one column block of V in a slot
+    static constexpr int kSlotBytes = BN * DP * 2 / kParts;
+    static constexpr int kSlots = (DP == 64) ? 8 : 5;
     static constexpr int kBarrierBytes = 512;
-    static constexpr int kSmemBytes = 1024 + QT * kQTileBytes + kSlots * kKvTileBytes + kBarrierBytes;
-    static constexpr int kSCol = 0;                         // S_t at kSCol + t * 128
+    static constexpr int kSmemBytes = 1024 + QT * kQTileBytes + kSlots * kSlotBytes + kBarrierBytes;
+    static constexpr int kSCol = 0;                         // S_t at kSCol + t * BN
     static constexpr int kOCol = 256;                       // O_t at kOCol + t * DP
-    static_assert((DP == 64 || DP == 128) ? (QT == 2 && BN == 128) : (DP == 256 && QT == 1 && BN == 64), "geometry");
-    static_assert(kOCol + QT * DP <= kTmemColumns, "tensor memory budget");
+    // P_t has columns of its own wherever O leaves room for them: S_t(j+1) then goes out as soon as S_t(j) is in registers
+    // and is there when the softmax group comes back for it, instead of following P_t(j) V_j. At D=128 there is no room.
+    // us in a lasting load, P over S / apart: D=64 B=3 S=2900 without a mask 310 / 297, four prompts of 4096 412 / 390, 10
+    // ragged ones 415 / 371, B=1 S=800 18.5 / 16.5. D=256 went from 64-key tiles with two score buffers (where the score
+    // products run at 3/4 of their rate) to 128 keys: B=1 S=3000 168 / 149, B=2 without a mask 655 / 545. It is bound by
+    // shared memory then: 448 KB per step (Q and K for the scores, V, the loads, V rewritten) against 2048 clocks of products.
+    static constexpr bool kOwnP = DP != 128;
+    static constexpr int kPCol = !kOwnP ? kSCol : DP == 64 ? 384 : 128;  // P_t at kPCol + t * kPStride
+    static constexpr int kPStride = kOwnP ? BN / 2 : BN;
+    static_assert(BN == 128 && (DP == 256 ? QT == 1 : QT == 2), "geometry");
+    static_assert(kOCol + QT * DP <= kTmemColumns && kPCol + QT * kPStride <= kTmemColumns, "tensor memory budget");
     static_assert(kSmemBytes <= 232448, "exceeds the 227 KiB per-CTA limit");
 };
 
@@ -140,24 +151,25 @@ __device__ __forceinline__ int TilesFor(int m0, int tokens, int seq_q, int seq_k
     return static_cast<int>((limit + BN - 1) / BN);
 }
 
-// Threads of a CTA: warp 0 TMA and tensor-memory owner, 1 MMA, 2-5 softmax of tile 0, 6-9 softmax of tile 1 (where there
-// is one), and for bf16 the warps that convert V. Two of them, except for the half-size tiles of D=64 on paged K/V:
-// chunked prefill of 20 sequences, D=128: 390 us with two, 415 with one; D=64: 337 with two, 309 with one (packed
-// D=64, four prompts of 4096: 407 with two, 428 with one).
-template <typename T, int DP, bool kPaged>
+// Warps that rewrite V as fp16. At D=256 a step has twice the bytes and its slots are the scarce thing: two warps 173 us,
+// three 172, four 146 (B=1, S=3000, lasting load). One warp is too few at D=128 (four prompts of 4096: 632 against 595).
+template <typename T, int DP>
 constexpr int ConverterWarps() {
-    return !PvFormat<T>::kConvertV ? 0 : kPaged && DP == 64 ? 1 : 2;
+    return !PvFormat<T>::kConvertV ? 0 : DP == 256 ? 4 : 2;
 }
-template <typename T, int DP, int QT, bool kPaged>
+// Warps of a CTA: 0 TMA and tensor-memory owner, 1 MMA, 2 and 3 V converters (idle for fp16), then four per query tile for
+// the softmax, then what converters are left.
+constexpr int kFirstSoftmax = 4;
+template <typename T, int DP, int QT>
 constexpr int FlashThreads() {
-    return 32 * (2 + 4 * QT + ConverterWarps<T, DP, kPaged>());
+    return 32 * (kFirstSoftmax + 4 * QT + (ConverterWarps<T, DP>() > 2 ? ConverterWarps<T, DP>() - 2 : 0));
 }
 
 // kVarlen: the work list comes from the (sequence, query block) table of a packed ragged batch; otherwise it is
 // computed from the dense [B, H, S, D] geometry and every per-sequence quantity is a launch constant.
 // kPaged (only with kVarlen): K and V of a sequence are scattered over the pages of a KV pool.
 template <typename T, int DP, int QT, int BN, bool kVarlen, bool kPaged = false>
-__global__ void __launch_bounds__(FlashThreads<T, DP, QT, kPaged>(), 1)
+__global__ void __launch_bounds__(FlashThreads<T, DP, QT>(), 1)
 flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const FlashKernelParams p) {
     using G = FlashGeom<DP, QT, BN>;
@@ -167,31 +179,32 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     const uint32_t q_smem = smem_base;
     const uint32_t ring_smem = smem_base + QT * G::kQTileBytes;
-    const uint32_t bar_base = ring_smem + G::kSlots * G::kKvTileBytes;
+    const uint32_t bar_base = ring_smem + G::kSlots * G::kSlotBytes;
     auto bar = [&](int i) { return bar_base + 8u * i; };
     // Barriers. A wait names a phase by its parity, so it is sound where the role knows that the phase before is over and
     // that the one after cannot be. For all but o_done the role waits for every phase in turn, and the next one takes an
-    // arrival that this role (or one that waits for it) makes later. o_done is waited for where O moves and at the end of
-    // an item only. The phase before it: its product went out ahead of scores the softmax has waited for since. The phase
-    // after: its product wants a P that this group has yet to write.
-    constexpr int kQFull = 0;                       // [2]
-    constexpr int kKvFull = 2;                      // [2 * kSlots], see RingFullBarrier
+    // arrival that this role (or one that waits for it) makes later. Where P lies over S, o_done is waited for where O moves
+    // and at the end of an item only. The phase before it: its product went out ahead of scores the softmax has waited for
+    // since. The phase after: its product wants a P that this group has yet to write.
+    constexpr int kTiles = QT;
+    constexpr int kQFull = 0;                       // [kTiles]
+    constexpr int kKvFull = kQFull + kTiles;        // [2 * kSlots], see RingFullBarrier
     constexpr int kKvEmpty = kKvFull + 2 * G::kSlots;   // [kSlots]
-    constexpr int kSFull = kKvEmpty + G::kSlots;    // [2]
-    constexpr int kPFull = kSFull + 2;              // [2]
-    constexpr int kODone = kPFull + 2;              // [2]
-    constexpr int kQEmpty = kODone + 2;             // [2]
-    constexpr int kOFree = kQEmpty + 2;             // [2]
-    constexpr int kPLast = kOFree + 2;              // [2]
-    constexpr int kVReady = kPLast + 2;             // [kSlots] bf16: V tile rewritten as fp16 in place
-    constexpr int kNumBars = kVReady + G::kSlots;
+    constexpr int kSFull = kKvEmpty + G::kSlots;    // [kTiles]
+    constexpr int kPFull = kSFull + kTiles;         // [kTiles]
+    constexpr int kODone = kPFull + kTiles;         // [kTiles]
+    constexpr int kQEmpty = kODone + kTiles;        // [kTiles]
+    constexpr int kOFree = kQEmpty + kTiles;        // [kTiles]
+    constexpr int kPLast = kOFree + kTiles;         // [kTiles]
+    constexpr int kVReady = kPLast + kTiles;        // [kSlots] bf16: V tile rewritten as fp16 in place
+    constexpr int kSRead = kVReady + G::kSlots;     // [kTiles] kOwnP: scores in registers
+    constexpr int kNumBars = kSRead + kTiles;
     auto full_bar = [&](bool is_v, uint32_t slot) { return bar(kKvFull + RingFullBarrier(is_v, static_cast<int>(slot), G::kSlots)); };
     using PT = typename PvFormat<T>::type;
     constexpr bool kCvtInKernel = PvFormat<T>::kConvertV;
-    constexpr int kConverterThreads = 32 * ConverterWarps<T, DP, kPaged>();
-    constexpr int kFirstConverter = 2 + 4 * QT;
+    constexpr int kConverters = ConverterWarps<T, DP>();
     // P is handed over in two pieces: the first kPEarly keys let P V start while the rest is still in the softmax
-    constexpr int kPEarly = BN == 128 ? 96 : 32;
+    constexpr int kPEarly = DP == 256 ? 64 : 96;
     static_assert(!kPaged || kVarlen, "paged K/V runs on the packed work list");
     static_assert(kNumBars * 8 + 16 <= G::kBarrierBytes, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + (bar_base - smem_base) + kNumBars * 8);
@@ -202,12 +215,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     volatile uint32_t* valid_ring = reinterpret_cast<volatile uint32_t*>(tmem_slot + 2);
     static_assert(kNumBars * 8 + 8 + kValidRing * 4 <= G::kBarrierBytes, "barrier area too small");
 
-    // One query tile per CTA (head dims above 128): no second tile to ping-pong with, so the scores are double-
-    // buffered instead: S(j+1) is computed while the softmax of block j runs. The barriers s_full / p_full / o_done
-    // are then indexed by the score buffer j & 1 instead of by the query tile.
-    constexpr bool kDoubleS = (QT == 1);
+    constexpr bool kOwnP = G::kOwnP;
+    constexpr int kParts = G::kParts;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    constexpr int kEndSoftmax = kFirstSoftmax + 4 * QT;
+    const int converter = warp < kFirstSoftmax ? warp - 2 : warp >= kEndSoftmax ? warp - kEndSoftmax + 2 : -1;
 
     // ---- Packed heads: P = 1 << pack_shift query heads of one kv head share a query tile (row r = token m0 + r / P, head
     // h + r % P). They read the same K/V tiles, so the rows of a short or ragged chunk fill up with other heads instead
@@ -226,8 +239,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         int seq;                      // index of the sequence (row of the page table); 0 for dense problems
         int q_tok0, kv_tok0;          // first row of the sequence in the packed tensors (0 for dense problems)
         int seq_q, seq_kv, diagonal;  // of this item's sequence
-        int m0[2];                    // first token of each tile, relative to the sequence
-        int ntiles[2];
+        int m0[kTiles];               // first token of each tile, relative to the sequence
+        int ntiles[kTiles];
         int n_max;
     };
     auto decode_item = [&](int idx) {
@@ -258,11 +271,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             w.diagonal = p.diagonal;
         }
         w.h_kv = w.h / (p.heads / p.kv_heads);
-        w.m0[0] = mb * p.tiles_per_item * tile_tokens;
-        w.m0[1] = w.m0[0] + tile_tokens;
-        w.ntiles[0] = TilesFor<BN>(w.m0[0], tile_tokens, w.seq_q, w.seq_kv, p.causal, w.diagonal);
-        w.ntiles[1] = p.tiles_per_item > 1 ? TilesFor<BN>(w.m0[1], tile_tokens, w.seq_q, w.seq_kv, p.causal, w.diagonal) : 0;
-        w.n_max = max(w.ntiles[0], w.ntiles[1]);
+        w.n_max = 0;
+#pragma unroll
+        for (int t = 0; t < kTiles; ++t) {
+            w.m0[t] = (mb * p.tiles_per_item + t) * tile_tokens;
+            w.ntiles[t] = t < p.tiles_per_item ? TilesFor<BN>(w.m0[t], tile_tokens, w.seq_q, w.seq_kv, p.causal, w.diagonal) : 0;
+            w.n_max = max(w.n_max, w.ntiles[t]);
+        }
         return w;
     };
     const int rounds = (total_items + gridDim.x - 1) / gridDim.x;
@@ -273,7 +288,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     };
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kTiles; ++i) {
             MbarInit<1>(bar(kQFull + i));
             MbarInit<1>(bar(kQEmpty + i));
             MbarInit<1>(bar(kSFull + i));
@@ -281,11 +296,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             MbarInit<4>(bar(kPLast + i));
             MbarInit<1>(bar(kODone + i));
             MbarInit<4>(bar(kOFree + i));
+            MbarInit<4>(bar(kSRead + i));
         }
         for (int i = 0; i < 2 * G::kSlots; ++i) MbarInit<1>(bar(kKvFull + i));
         for (int i = 0; i < G::kSlots; ++i) {
             MbarInit<1>(bar(kKvEmpty + i));
-            if constexpr (kCvtInKernel) MbarInit<kConverterThreads>(bar(kVReady + i));
+            if constexpr (kCvtInKernel) MbarInit<32 * kConverters>(bar(kVReady + i));
         }
         *abort_flag = 0;
         FenceBarrierInit();
@@ -305,7 +321,9 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (warp == 0 && kPaged) {
         // ================================ TMA producer, paged K/V ===================================
         // The whole warp walks the work list: the lanes fetch the page ids of a tile together (one coalesced read
-        // of the table row), lane 0 waits for the ring slot and issues one box load per page and column block. A
+        // of the table row), lane 0 waits for the ring slot and one lane issues a box load per page and column block. The
+        // loads decide at D=256, so what can be known at compile time about them is: with run-time block counts a box took
+        // 170 clocks to issue instead of 90 (20 chunks, D=256: 1790 us, 1032 now, 1094 with 64-key tiles). A
         // page that is unmapped (entry < 0 or >= num_kv_blocks) is loaded from beyond the pool, i.e. zero-filled,
         // and its columns are masked in the softmax through valid_ring.
         if (lane == 0) {
@@ -313,11 +331,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             PrefetchTensorMap(&map_k);
             PrefetchTensorMap(&map_v);
         }
-        uint32_t q_uses[2] = {0, 0};
+        uint32_t q_uses[kTiles] = {};
         uint32_t kv_loads = 0;
         uint32_t tiles_before = 0;  // KV tiles of the items this CTA has finished
         const int pages_per_tile = BN >> p.block_shift;
         const int page_bytes = p.block_size * 128;  // one page inside one 64-element column block
+        const int pages_per_v = G::kVKeys >> p.block_shift;  // in one slot
         bool ok = true;
         for (int r = 0; r < rounds && ok; ++r) {
             const int idx = item_of_round(r);
@@ -338,17 +357,23 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             const int32_t* row = p.page_table + static_cast<int64_t>(w.seq) * p.max_blocks_per_seq;
-            for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                const RingLoad load = RingOrder(it, w.n_max, kDoubleS);
+            // page ids of a KV tile, one per lane; looked up a tile ahead, so that the ring does not wait for the table
+            auto page_ids = [&](int tile) {
+                const int logical = tile * pages_per_tile + lane;
+                const bool in = lane < pages_per_tile && logical < p.max_blocks_per_seq && (static_cast<int64_t>(logical) << p.block_shift) < w.seq_kv;
+                return in ? __ldg(row + logical) : -1;
+            };
+            int32_t ids_before = -1, ids = -1, ids_next = page_ids(0);  // of the tiles before, of and behind the last K loaded
+            for (int it = 0; it < 2 * w.n_max * kParts && ok; ++it, ++kv_loads) {
+                const RingLoad load = RingOrder(it / kParts, w.n_max, kOwnP);
                 const bool is_v = load.is_v;
                 const int tile = load.tile;
-                // page ids of this tile, one per lane
-                const int logical = tile * pages_per_tile + lane;
-                int32_t phys = -1;
-                if (lane < pages_per_tile && logical < p.max_blocks_per_seq &&
-                    (static_cast<int64_t>(logical) << p.block_shift) < w.seq_kv) {
-                    phys = __ldg(row + logical);
+                if (!is_v && it % kParts == 0) {
+                    ids_before = ids;
+                    ids = ids_next;
+                    if (tile + 1 < w.n_max) ids_next = page_ids(tile + 1);
                 }
+                const int32_t phys = is_v && kOwnP && tile + 1 < w.n_max ? ids_before : ids;
                 const bool mapped = phys >= 0 && phys < p.num_kv_blocks;
                 const uint32_t valid = __ballot_sync(0xffffffffu, mapped);
                 const uint32_t slot = kv_loads % G::kSlots;
@@ -357,22 +382,32 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     ok = MbarWait(bar(kKvEmpty + slot), phase ^ 1u, abort_flag);
                     if (ok) {
                         if (!is_v) valid_ring[(tiles_before + tile) % kValidRing] = valid;
-                        MbarExpectTx(full_bar(is_v, slot), G::kKvTileBytes);
+                        MbarExpectTx(full_bar(is_v, slot), G::kSlotBytes);
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) break;
-                const CUtensorMap* map = is_v ? &map_v : &map_k;
-                for (int pg = 0; pg < pages_per_tile; ++pg) {
-                    const int32_t id = __shfl_sync(0xffffffffu, phys, pg);
-                    // an unmapped page reads from the first row behind the pool: all zeros
-                    const int first_row = ((valid >> pg) & 1u) ? (id << p.block_shift) : (p.num_kv_blocks << p.block_shift);
-                    if (ElectOne()) {
-                        for (int kb = 0; kb < G::kKBlocks; ++kb) {
-                            TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes + pg * page_bytes, map,
-                                      full_bar(is_v, slot), kb * 64, first_row, w.h_kv, 0);
+                const int part = it % kParts;
+                // `blocks` column blocks of every page of the slot; an unmapped page reads from the first row behind the pool
+                auto load_pages = [&](const CUtensorMap* map, int first_page, int pages, int first_block, auto blocks, uint32_t block_bytes) {
+                    const uint32_t full = full_bar(is_v, slot);
+                    uint32_t dst = ring_smem + slot * G::kSlotBytes;
+                    for (int pg = 0; pg < pages; ++pg, dst += page_bytes) {
+                        const int32_t id = __shfl_sync(0xffffffffu, phys, first_page + pg);
+                        const int first_row = ((valid >> (first_page + pg)) & 1u) ? (id << p.block_shift) : (p.num_kv_blocks << p.block_shift);
+                        if (ElectOne()) {
+#pragma unroll
+                            for (int kb = 0; kb < blocks.value; ++kb) {
+                                TmaLoad4D(dst + kb * block_bytes, map, full, (first_block + kb) * 64, first_row, w.h_kv, 0);
+                            }
                         }
                     }
+                };
+                if (is_v) {
+                    load_pages(&map_v, part * pages_per_v, pages_per_v, 0, std::integral_constant<int, G::kKBlocks>{}, G::kVBlockBytes);
+                } else {
+                    load_pages(&map_k, 0, pages_per_tile, part * (G::kKBlocks / kParts), std::integral_constant<int, G::kKBlocks / kParts>{},
+                               G::kKBlockBytes);
                 }
             }
             tiles_before += static_cast<uint32_t>(w.n_max);
@@ -384,7 +419,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             PrefetchTensorMap(&map_q);
             PrefetchTensorMap(&map_k);
             PrefetchTensorMap(&map_v);
-            uint32_t q_uses[2] = {0, 0};   // how often each query buffer has been filled so far
+            uint32_t q_uses[kTiles] = {};   // how often each query buffer has been filled so far
             uint32_t kv_loads = 0;         // K/V tiles loaded so far (ring position)
             bool ok = true;
             for (int r = 0; r < rounds && ok; ++r) {
@@ -403,18 +438,25 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                     ++q_uses[t];
                 }
-                for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                    const RingLoad load = RingOrder(it, w.n_max, kDoubleS);
+                for (int it = 0; it < 2 * w.n_max * kParts && ok; ++it, ++kv_loads) {
+                    const RingLoad load = RingOrder(it / kParts, w.n_max, kOwnP);
                     const uint32_t slot = kv_loads % G::kSlots;
                     const uint32_t phase = (kv_loads / G::kSlots) & 1u;
                     ok = MbarWait(bar(kKvEmpty + slot), phase ^ 1u, abort_flag);
                     if (!ok) break;
                     const uint32_t full = full_bar(load.is_v, slot);
-                    MbarExpectTx(full, G::kKvTileBytes);
-                    const CUtensorMap* map = load.is_v ? &map_v : &map_k;
-                    for (int kb = 0; kb < G::kKBlocks; ++kb) {
-                        TmaLoad4D(ring_smem + slot * G::kKvTileBytes + kb * G::kKvBlockBytes, map, full, kb * 64,
-                                  w.kv_tok0 + load.tile * BN, w.h_kv, w.b);
+                    MbarExpectTx(full, G::kSlotBytes);
+                    const int part = it % kParts;
+                    const uint32_t dst = ring_smem + slot * G::kSlotBytes;
+                    if (load.is_v) {
+                        for (int kb = 0; kb < G::kKBlocks; ++kb) {
+                            TmaLoad4D(dst + kb * G::kVBlockBytes, &map_v, full, kb * 64, w.kv_tok0 + load.tile * BN + part * G::kVKeys, w.h_kv, w.b);
+                        }
+                    } else {
+                        for (int kb = 0; kb < G::kKBlocks / kParts; ++kb) {
+                            TmaLoad4D(dst + kb * G::kKBlockBytes, &map_k, full, (part * (G::kKBlocks / kParts) + kb) * 64,
+                                      w.kv_tok0 + load.tile * BN, w.h_kv, w.b);
+                        }
                     }
                 }
             }
@@ -431,44 +473,42 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // Descriptors are built once and advanced by compile-time constants, so that issuing one
             // tcgen05.mma costs a handful of instructions (this thread alone has to keep the tensor pipe fed).
             const uint64_t kmajor_hi = MakeSmemDesc(0, 16, 1024);                 // K-major operands (Q and K)
-            const uint64_t vmajor_hi = MakeSmemDesc(0, G::kKvBlockBytes, 1024);   // MN-major operand (V)
-            const uint64_t q_desc[2] = {kmajor_hi | (q_smem >> 4), kmajor_hi | ((q_smem + G::kQTileBytes) >> 4)};
-            const uint32_t s_tmem[2] = {tmem_base + G::kSCol, tmem_base + G::kSCol + 128};
-            uint32_t s_tmem_db = tmem_base + G::kSCol;  // current score buffer when the scores are double-buffered
-            const uint32_t o_tmem[2] = {tmem_base + G::kOCol, tmem_base + G::kOCol + DP};
-            auto issue_s = [&](int t, uint32_t slot) {
-                const uint64_t a0 = q_desc[t];
-                const uint64_t b0 = kmajor_hi | ((ring_smem + slot * G::kKvTileBytes) >> 4);
+            const uint64_t vmajor_hi = MakeSmemDesc(0, G::kVBlockBytes, 1024);    // MN-major operand (V)
+            auto q_desc = [&](int t) { return kmajor_hi | ((q_smem + t * G::kQTileBytes) >> 4); };
+            auto s_tmem = [&](int t) { return tmem_base + G::kSCol + t * BN; };
+            auto p_tmem = [&](int t) { return tmem_base + G::kPCol + t * G::kPStride; };
+            auto o_tmem = [&](int t) { return tmem_base + G::kOCol + t * DP; };
+            // the columns of S that the K of this slot contributes to: all of Q K^T, or one half of its products
+            auto issue_s = [&](int t, uint32_t slot, int part) {
+                const uint64_t a0 = q_desc(t) + ((part * (G::kKBlocks / kParts) * G::kQBlockBytes) >> 4);
+                const uint64_t b0 = kmajor_hi | ((ring_smem + slot * G::kSlotBytes) >> 4);
 #pragma unroll
-                for (int ks = 0; ks < DP / 16; ++ks) {
+                for (int ks = 0; ks < DP / kParts / 16; ++ks) {
                     constexpr int kStep = 32 >> 4;  // 16 elements = 32 bytes inside a 128-byte swizzle row
                     const uint32_t qa = ((ks >> 2) * G::kQBlockBytes >> 4) + (ks & 3) * kStep;
-                    const uint32_t kb = ((ks >> 2) * G::kKvBlockBytes >> 4) + (ks & 3) * kStep;
-                    const uint32_t d = kDoubleS ? s_tmem_db : s_tmem[t];
-                    if (ks == 0) MmaSS<false>(d, a0 + qa, b0 + kb, idesc_s);
-                    else MmaSS<true>(d, a0 + qa, b0 + kb, idesc_s);
+                    const uint32_t kb = ((ks >> 2) * G::kKBlockBytes >> 4) + (ks & 3) * kStep;
+                    if (ks == 0 && part == 0) MmaSS<false>(s_tmem(t), a0 + qa, b0 + kb, idesc_s);
+                    else MmaSS<true>(s_tmem(t), a0 + qa, b0 + kb, idesc_s);
                 }
             };
-            // waits for the second piece of P (barriers `sync`, parity `parity`) half-way
-            auto issue_pv = [&](int t, uint32_t slot, bool first, int sync, uint32_t parity) {
-                const uint64_t b0 = vmajor_hi | ((ring_smem + slot * G::kKvTileBytes) >> 4);
-                const uint32_t a = kDoubleS ? s_tmem_db : s_tmem[t];
+            // P V over the keys of V in this slot; waits for the second piece of P (parity `parity`) where it begins
+            auto issue_pv = [&](int t, uint32_t slot, int part, bool first, uint32_t parity) {
+                const uint64_t b0 = vmajor_hi | ((ring_smem + slot * G::kSlotBytes) >> 4);
 #pragma unroll
-                for (int ks = 0; ks < kPEarly / 16; ++ks) {
+                for (int i = 0; i < G::kVKeys / 16; ++i) {
                     // 16 keys further: 8 packed P columns in tensor memory, 16 rows (2048 bytes) of V
-                    if (ks == 0) MmaTSFlag(o_tmem[t], a, b0, idesc_o, first ? 0u : 1u);
-                    else MmaTS<true>(o_tmem[t], a + ks * 8, b0 + ks * (2048 >> 4), idesc_o);
-                }
-                if (!MbarWait(bar(kPLast + sync), parity, abort_flag)) return false;
-                TcFenceAfter();
-#pragma unroll
-                for (int ks = kPEarly / 16; ks < BN / 16; ++ks) {
-                    MmaTS<true>(o_tmem[t], a + ks * 8, b0 + ks * (2048 >> 4), idesc_o);
+                    const int ks = part * (G::kVKeys / 16) + i;
+                    if (ks == kPEarly / 16) {
+                        if (!MbarWait(bar(kPLast + t), parity, abort_flag)) return false;
+                        TcFenceAfter();
+                    }
+                    if (ks == 0) MmaTSFlag(o_tmem(t), p_tmem(t), b0, idesc_o, first ? 0u : 1u);
+                    else MmaTS<true>(o_tmem(t), p_tmem(t) + ks * 8, b0 + i * (2048 >> 4), idesc_o);
                 }
                 return true;
             };
-            uint32_t q_uses[2] = {0, 0};    // items finished per query buffer
-            uint32_t steps[2] = {0, 0};     // KV tiles processed per query tile (phase of s_full / p_full / o_done)
+            uint32_t q_uses[kTiles] = {};    // items finished per query buffer
+            uint32_t steps[kTiles] = {};     // KV tiles processed per query tile (phase of s_full / p_full / o_done)
             uint32_t kv_base = 0;           // ring position of this item's K_0
             RingPhases k_phases, v_phases;  // of the K barriers and of v_ready (no converter: the V barriers)
             bool ok = true;
@@ -476,13 +516,28 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             auto v_ready = [&](uint32_t slot) {
                 return MbarWait(kCvtInKernel ? bar(kVReady + slot) : full_bar(true, slot), v_phases.Take(slot), abort_flag);
             };
-            if constexpr (kDoubleS) {
-                // single query tile, two score buffers: S(0), S(1), then P(j) V_j followed by S(j+2) into the buffer
-                // P(j) came from (same in-order stream, so the overwrite happens after the read)
-                uint32_t buf_uses[2] = {0, 0};  // P tiles consumed per score buffer (phase of p_full)
-                auto next_slot = [&](uint32_t* slot, bool is_v) {
-                    *slot = kv_base++ % G::kSlots;
-                    return is_v ? v_ready(*slot) : k_landed(*slot);
+            if constexpr (kOwnP) {
+                // S_t(j+1) goes out as soon as S_t(j) is in registers, P_t(j) V_j when P_t(j) has been written
+                uint32_t scores[kTiles] = {};  // score tiles issued per query tile (phase of s_read)
+                auto next_slots = [&](uint32_t (&slots)[kParts]) {
+                    for (int part = 0; part < kParts; ++part) slots[part] = kv_base++ % G::kSlots;
+                };
+                // K and V are waited for with the first query tile, also where it has no use for them, and freed with the last
+                auto score_step = [&](int t, const uint32_t (&k)[kParts], bool active, bool wait_k, bool last) {
+                    if (active && scores[t] > 0 && !MbarWait(bar(kSRead + t), (scores[t] - 1) & 1u, abort_flag)) return false;
+#pragma unroll
+                    for (int part = 0; part < kParts; ++part) {
+                        if (wait_k && !k_landed(k[part])) return false;
+                        TcFenceAfter();
+                        if (active) issue_s(t, k[part], part);
+                        if (t == QT - 1) MmaCommit(bar(kKvEmpty + k[part]));
+                    }
+                    if (active) {
+                        MmaCommit(bar(kSFull + t));
+                        if (last) MmaCommit(bar(kQEmpty + t));
+                        ++scores[t];
+                    }
+                    return true;
                 };
                 for (int r = 0; r < rounds && ok; ++r) {
                     const int idx = item_of_round(r);
@@ -490,45 +545,49 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     const Item w = decode_item(idx);
                     const int n = w.n_max;
                     if (n == 0) continue;
-                    ok = MbarWait(bar(kQFull), q_uses[0] & 1u, abort_flag);
-                    uint32_t slot = 0;
-                    for (int i = 0; i < 2 && i < n && ok; ++i) {
-                        ok = next_slot(&slot, false);
+                    uint32_t k[kParts], v[kParts];
+                    next_slots(k);
+#pragma unroll
+                    for (int t = 0; t < QT; ++t) {
                         if (!ok) break;
-                        TcFenceAfter();
-                        s_tmem_db = tmem_base + G::kSCol + i * 64;
-                        issue_s(0, slot);
-                        MmaCommit(bar(kSFull + i));
-                        if (i == n - 1) MmaCommit(bar(kQEmpty));
-                        MmaCommit(bar(kKvEmpty + slot));
+                        if (w.ntiles[t] > 0) ok = MbarWait(bar(kQFull + t), q_uses[t] & 1u, abort_flag);
+                        ok = ok && score_step(t, k, w.ntiles[t] > 0, t == 0, w.ntiles[t] == 1);
                     }
                     for (int j = 0; j < n && ok; ++j) {
-                        const uint32_t buf = j & 1;
-                        const uint32_t p_parity = buf_uses[buf]++ & 1u;
-                        ok = MbarWait(bar(kPFull + buf), p_parity, abort_flag);
-                        if (ok && j == 0 && q_uses[0] > 0) ok = MbarWait(bar(kOFree), (q_uses[0] - 1) & 1u, abort_flag);
-                        if (ok) ok = next_slot(&slot, true);  // V_j
-                        if (!ok) break;
-                        TcFenceAfter();
-                        s_tmem_db = tmem_base + G::kSCol + buf * 64;
-                        ok = issue_pv(0, slot, j == 0, buf, p_parity);
-                        if (!ok) break;
-                        MmaCommit(bar(kODone + buf));
-                        MmaCommit(bar(kKvEmpty + slot));
-                        if (j + 2 < n) {
-                            ok = next_slot(&slot, false);  // K_j+2
+                        if (j + 1 < n) next_slots(k);
+                        next_slots(v);
+#pragma unroll
+                        for (int t = 0; t < QT; ++t) {
                             if (!ok) break;
-                            TcFenceAfter();
-                            issue_s(0, slot);
-                            MmaCommit(bar(kSFull + buf));
-                            if (j + 2 == n - 1) MmaCommit(bar(kQEmpty));
-                            MmaCommit(bar(kKvEmpty + slot));
+                            if (j + 1 < n) ok = score_step(t, k, j + 1 < w.ntiles[t], t == 0, j + 2 == w.ntiles[t]);
+                            const bool active = j < w.ntiles[t];
+                            if (ok && active) ok = MbarWait(bar(kPFull + t), steps[t] & 1u, abort_flag);
+                            // the first P V of an item overwrites O: the previous item's O must have been read out
+                            if (ok && active && j == 0 && q_uses[t] > 0) ok = MbarWait(bar(kOFree + t), (q_uses[t] - 1) & 1u, abort_flag);
+                            if (!ok) break;
+#pragma unroll
+                            for (int part = 0; part < kParts; ++part) {
+                                if (t == 0) ok = v_ready(v[part]);
+                                if (!ok) break;
+                                TcFenceAfter();
+                                if (active) ok = issue_pv(t, v[part], part, j == 0, steps[t] & 1u);
+                                if (!ok) break;
+                                if (t == QT - 1) MmaCommit(bar(kKvEmpty + v[part]));
+                            }
+                            if (ok && active) {
+                                MmaCommit(bar(kODone + t));
+                                ++steps[t];
+                            }
                         }
                     }
-                    ++q_uses[0];
+#pragma unroll
+                    for (int t = 0; t < QT; ++t) {
+                        if (w.ntiles[t] > 0) ++q_uses[t];
+                    }
                 }
             }
-            for (int r = 0; r < rounds && ok && !kDoubleS; ++r) {
+            // P over S: P_t(j) V_j, then S_t(j+1), tile by tile
+            for (int r = 0; r < rounds && ok && !kOwnP; ++r) {
                 const int idx = item_of_round(r);
                 if (idx < 0) continue;
                 const Item w = decode_item(idx);
@@ -542,7 +601,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         TcFenceAfter();
                         for (int t = 0; t < QT; ++t) {
                             if (w.ntiles[t] == 0) continue;
-                            issue_s(t, slot_of(0));
+                            issue_s(t, slot_of(0), 0);
                             MmaCommit(bar(kSFull + t));
                             if (w.ntiles[t] == 1) MmaCommit(bar(kQEmpty + t));  // last read of this query tile
                         }
@@ -562,12 +621,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         if (ok && j == 0 && q_uses[t] > 0) ok = MbarWait(bar(kOFree + t), (q_uses[t] - 1) & 1u, abort_flag);
                         if (!ok) break;
                         TcFenceAfter();
-                        ok = issue_pv(t, slot_of(it_v), j == 0, t, steps[t] & 1u);
+                        ok = issue_pv(t, slot_of(it_v), 0, j == 0, steps[t] & 1u);
                         if (!ok) break;
                         MmaCommit(bar(kODone + t));
                         ++steps[t];
                         if (j + 1 < w.ntiles[t]) {
-                            issue_s(t, slot_of(it_k));
+                            issue_s(t, slot_of(it_k), 0);
                             MmaCommit(bar(kSFull + t));
                             if (j + 2 == w.ntiles[t]) MmaCommit(bar(kQEmpty + t));
                         }
@@ -583,7 +642,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             failed = !ok;
         }
-    } else if (kCvtInKernel && warp >= kFirstConverter) {
+    } else if (converter >= 0 && converter < kConverters) {
         // ================================ V converter (bf16) ========================================
         // Walks the ring in the producer's order; every V tile is rewritten in place from bf16 to fp16 once its
         // bytes have landed, then handed to the MMA thread through v_ready. K tiles are not touched.
@@ -594,14 +653,14 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const int idx = item_of_round(r);
             if (idx < 0) continue;
             const Item w = decode_item(idx);
-            for (int it = 0; it < 2 * w.n_max && ok; ++it, ++kv_loads) {
-                if (!RingOrder(it, w.n_max, kDoubleS).is_v) continue;
+            for (int it = 0; it < 2 * w.n_max * kParts && ok; ++it, ++kv_loads) {
+                if (!RingOrder(it / kParts, w.n_max, kOwnP).is_v) continue;
                 const uint32_t slot = kv_loads % G::kSlots;
                 ok = __all_sync(0xffffffffu, MbarWait(full_bar(true, slot), v_phases.Take(slot), abort_flag));
                 if (!ok) break;
-                uint4* tile = reinterpret_cast<uint4*>(smem + (ring_smem - smem_base) + slot * G::kKvTileBytes);
+                uint4* tile = reinterpret_cast<uint4*>(smem + (ring_smem - smem_base) + slot * G::kSlotBytes);
 #pragma unroll 8
-                for (int c = threadIdx.x - 32 * kFirstConverter; c < G::kKvTileBytes / 16; c += kConverterThreads) {
+                for (int c = converter * 32 + lane; c < G::kSlotBytes / 16; c += 32 * kConverters) {
                     uint4 x = tile[c];
                     uint32_t* word = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
@@ -617,53 +676,46 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
         }
         failed = !ok;
-    } else {
+    } else if (warp >= kFirstSoftmax && warp < kEndSoftmax) {
         // ================================ softmax groups ============================================
-        const int t = (warp - 2) >> 2;
+        const int t = (warp - kFirstSoftmax) >> 2;
         const int quad = warp & 3;
         const int row_in_tile = quad * 32 + lane;
         const uint32_t lane_bits = static_cast<uint32_t>(quad * 32) << 16;
-        const uint32_t s_addr0 = tmem_base + lane_bits + G::kSCol + t * 128;
+        const uint32_t s_addr = tmem_base + lane_bits + G::kSCol + t * BN;
+        const uint32_t p_addr = tmem_base + lane_bits + G::kPCol + t * G::kPStride;
         const uint32_t o_addr = tmem_base + lane_bits + G::kOCol + t * DP;
         uint32_t steps = 0;  // KV tiles this group has processed (phase of s_full / p_full / o_done)
-        uint32_t buf_steps0 = 0, buf_steps1 = 0;  // double-buffered scores: tiles taken from each buffer
         uint32_t tiles_before = 0;  // paged K/V: KV tiles of the items this CTA has finished (index into valid_ring)
         const uint32_t all_pages = kPaged ? ((BN >> p.block_shift) >= 32 ? 0xffffffffu : (1u << (BN >> p.block_shift)) - 1u) : 0u;
         bool ok = true;
 
-        for (int r = 0; r < rounds && ok && t < QT; ++r) {
+        for (int r = 0; r < rounds && ok; ++r) {
             const int idx = item_of_round(r);
             if (idx < 0) continue;
             const Item w = decode_item(idx);
-            const int n_t = w.ntiles[t];
+            int n_t = 0, m_t = 0;
+#pragma unroll
+            for (int i = 0; i < kTiles; ++i) {
+                if (i == t) n_t = w.ntiles[i], m_t = w.m0[i];
+            }
             const uint32_t tiles_base = tiles_before;
             tiles_before += static_cast<uint32_t>(w.n_max);
             if (n_t == 0) continue;
-            const int row = w.m0[t] + (row_in_tile >> p.pack_shift);                 // token of the sequence
+            const int row = m_t + (row_in_tile >> p.pack_shift);                 // token of the sequence
             const int head = w.h + (row_in_tile & ((1 << p.pack_shift) - 1));
             float m_ref = -CUDART_INF_F;  // reference point of the exponentials (log2 domain)
             float l_sum = 0.0f;
 
             for (int j = 0; j < n_t; ++j, ++steps) {
-                // which score buffer / barrier set this step uses, and the phases to wait for
-                const uint32_t buf = kDoubleS ? (j & 1) : 0;
-                const uint32_t s_addr = s_addr0 + buf * 64;
-                const int sync = kDoubleS ? static_cast<int>(buf) : t;          // index into s_full / p_full
-                const uint32_t s_phase = kDoubleS ? ((buf ? buf_steps1 : buf_steps0) & 1u) : (steps & 1u);
-                // the product P(j-1) V_j-1 that must be complete before O may be rescaled
-                const int prev_sync = kDoubleS ? static_cast<int>(buf ^ 1) : t;
-                const uint32_t prev_phase = kDoubleS ? (((buf ? buf_steps0 : buf_steps1) - 1) & 1u) : ((steps - 1) & 1u);
-                if (kDoubleS) {
-                    if (buf) ++buf_steps1; else ++buf_steps0;
-                }
-                ok = __all_sync(0xffffffffu, MbarWait(bar(kSFull + sync), s_phase, abort_flag));
+                ok = __all_sync(0xffffffffu, MbarWait(bar(kSFull + t), steps & 1u, abort_flag));
                 if (!ok) break;
                 TcFenceAfter();
                 // The row goes to registers whole. The exponentials use the reference point the row already has; the
                 // row's maximum is only checked against it. If it exceeds the reference by more than the threshold
                 // (always in the first step of an item), the reference moves and O and the row sum are rescaled.
-                // P (16-bit pairs) lands on the first BN / 2 columns of S_t, which has been read by then; its first
-                // kPEarly keys are handed over early, so that P V starts under the last exponentials.
+                // P (16-bit pairs) goes to columns of its own or to the first BN / 2 columns of S_t, which has been read by
+                // then; its first kPEarly keys are handed over early, so that P V starts under the last exponentials.
                 const int col0 = j * BN;
                 const int kv_limit = w.seq_kv - col0;                                   // columns >= kv_limit do not exist
                 const int causal_limit = p.causal ? (row + w.diagonal - col0 + 1) : BN;  // columns >= limit are masked
@@ -675,6 +727,19 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
                 for (int c = 0; c < BN / 32; ++c) TmemLd32(s_addr + c * 32, sc[c]);
                 TmemWaitLd();
+                if constexpr (kOwnP) {
+                    TcFenceBefore();
+                    __syncwarp();
+                    if (lane == 0) MbarArrive(bar(kSRead + t));
+                }
+                bool pv_done = j == 0;  // P(j-1) V_j-1: O and the columns of P may be written
+                auto wait_pv = [&] {
+                    if (!pv_done) {
+                        ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + t), (steps - 1) & 1u, abort_flag));
+                        TcFenceAfter();
+                        pv_done = true;
+                    }
+                };
                 if (ragged) {
 #pragma unroll
                     for (int c = 0; c < BN / 32; ++c) {
@@ -702,9 +767,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (__any_sync(0xffffffffu, move)) {
                         const float alpha = move ? Exp2(m_ref - mx) : 1.0f;  // m_ref = -inf -> 0
                         if (j > 0) {
-                            ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + prev_sync), prev_phase, abort_flag));
+                            wait_pv();
                             if (!ok) break;
-                            TcFenceAfter();
 #pragma unroll 1
                             for (int cblk = 0; cblk < DP / 16; ++cblk) {
                                 uint32_t r[16];
@@ -725,7 +789,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 // (1030 is the rate of the special-function unit), two warps 2070 and 2110. D=128, where the groups meet
                 // the products half of the time, gains 2 % (528 against 535 us at B=4, S=4096); D=64, where they mostly
                 // run side by side, loses 10 % (359 against 322 us at B=3, S=2900).
-                constexpr bool kBehind = DP == 128;
+                constexpr bool kBehind = DP != 64;
                 const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
                 float2 sum[4];
 #pragma unroll
@@ -754,7 +818,10 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                                 pk[(d % 4) * 4 + e] = Pack2<PT>(x[d & 1][e].x, x[d & 1][e].y);
                             }
                         }
-                        if (b - kLag >= 4 * first && (b - kLag) % 4 == 3) TmemSt16(s_addr + (b - kLag) / 4 * 16, pk);
+                        if (b - kLag >= 4 * first && (b - kLag) % 4 == 3) {
+                            if (kOwnP && b - kLag == 3) wait_pv();
+                            TmemSt16(p_addr + (b - kLag) / 4 * 16, pk);
+                        }
                     }
                 };
                 auto hand_over = [&](uint32_t barrier) {
@@ -764,25 +831,23 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (lane == 0) MbarArrive(barrier);
                 };
                 exponentials(0, kPEarly / 32);
-                hand_over(bar(kPFull + sync));
-                if (kBehind) {  // eight registers less across the second piece
+                if (!ok) break;
+                hand_over(bar(kPFull + t));
+                if (kBehind && kPEarly < BN) {  // eight registers less across the second piece
                     fold_sum();
 #pragma unroll
                     for (int e = 0; e < 4; ++e) sum[e] = make_float2(0.0f, 0.0f);
                 }
-                exponentials(kPEarly / 32, BN / 32);
-                hand_over(bar(kPLast + sync));
+                if constexpr (kPEarly < BN) {
+                    exponentials(kPEarly / 32, BN / 32);
+                    hand_over(bar(kPLast + t));
+                }
                 fold_sum();
             }
             if (!ok) break;
 
             // ---- epilogue: O / l -> global, optional LSE; O is handed back as soon as it is in registers ----
-            if (kDoubleS) {
-                const uint32_t last = (n_t - 1) & 1;
-                ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + last), ((last ? buf_steps1 : buf_steps0) - 1) & 1u, abort_flag));
-            } else {
-                ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + t), (steps - 1) & 1u, abort_flag));
-            }
+            ok = __all_sync(0xffffffffu, MbarWait(bar(kODone + t), (steps - 1) & 1u, abort_flag));
             if (!ok) break;
             TcFenceAfter();
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
@@ -799,13 +864,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
                 if (row < w.seq_q) {
 #pragma unroll
-                    for (int piece = 0; piece < 2; ++piece) {
+                    for (int half = 0; half < 2; ++half) {
                         uint32_t pk[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            pk[i] = Pack2<T>(__uint_as_float(r[piece * 16 + 2 * i]) * inv, __uint_as_float(r[piece * 16 + 2 * i + 1]) * inv);
+                            pk[i] = Pack2<T>(__uint_as_float(r[half * 16 + 2 * i]) * inv, __uint_as_float(r[half * 16 + 2 * i + 1]) * inv);
                         }
-                        const int d0 = cblk * 32 + piece * 16;
+                        const int d0 = cblk * 32 + half * 16;
                         if (d0 < p.head_dim) StoreRow16(o_row + d0, pk, p.wide_stores);
                     }
                 }
@@ -1064,7 +1129,7 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         if (PvFormat<T>::kConvertV && (!Aligned16(f.v) || f.v_sb % 8 != 0 || f.v_sh % 8 != 0 || f.v_ss % 8 != 0)) {
             return Fail(SCA_INVALID_ARGUMENT, "flash attention: v must be 16-byte aligned with strides that are multiples of 8 elements");
         }
-        if (int rc = MakeMap(&map_v, f.v, f.dtype_id, f.head_dim, f.seq_kv, f.num_kv_heads, f.batch, f.v_ss, f.v_sh, f.v_sb, BN, "v")) return rc;
+        if (int rc = MakeMap(&map_v, f.v, f.dtype_id, f.head_dim, f.seq_kv, f.num_kv_heads, f.batch, f.v_ss, f.v_sh, f.v_sb, G::kVKeys, "v")) return rc;
     }
 
     FlashKernelParams p{};
@@ -1097,7 +1162,7 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         return Fail(SCA_INVALID_ARGUMENT, "flash attention: grid of " + std::to_string(ctas) + " blocks is out of range");
     }
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ctas, SmCount()));  // one persistent CTA per SM
-    const unsigned threads = paged != nullptr ? FlashThreads<T, DP, QT, true>() : FlashThreads<T, DP, QT, false>();
+    constexpr unsigned threads = FlashThreads<T, DP, QT>();
     if (paged != nullptr) {
         p.page_table = paged->page_table;
         p.max_blocks_per_seq = static_cast<int>(paged->max_blocks_per_seq);
@@ -1166,7 +1231,7 @@ int LaunchFlashTyped(const ScaFlashFwdParams& f, cudaStream_t stream, const Varl
         case 128: return LaunchFlash<T, 128, 2, 128>(f, stream, varlen, paged);
         case 160:
         case 192:
-        case 256: return LaunchFlash<T, 256, 1, 64>(f, stream, varlen, paged);
+        case 256: return LaunchFlash<T, 256, 1, 128>(f, stream, varlen, paged);
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT, "flash attention: head_dim=" + std::to_string(f.head_dim) + " is not instantiated");
