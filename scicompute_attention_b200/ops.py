@@ -5,6 +5,9 @@ taking torch CUDA tensors only as device memory + stream providers.
 Argument meaning follows the reference's public API (include/scicompute_attention/*.hpp):
 q is [B, H_q, S_q, D] (layout "bhsd") or [B, S_q, H_q, D] ("bshd"); k/v likewise with H_kv;
 outputs are always freshly allocated contiguous BHSD tensors, allocated on `stream` where one is given.
+
+A call in its plain form (tensors, the current stream) goes through one C function of _native (csrc/torch/native_ops.cpp),
+which answers None where it does not take the call; the code here is the general form, and the one that raises the errors.
 """
 from __future__ import annotations
 
@@ -24,6 +27,23 @@ MAX_SPLITS = 64          # upper bound of the automatic split count on B200
 
 _DTYPE_IDS = {torch.float32: DTYPE_F32, torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16}
 MAX_SCRATCH_BUFFERS = 32  # scratch buffers a thread keeps
+
+
+_native_module = None
+
+
+def _native():
+    """The native form of the operators. There is no fallback: on a GPU it has to have been built."""
+    global _native_module
+    if _native_module is None:
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError("scicompute_attention_b200/_native.so is missing or does not fit this torch: build it with "
+                               "`python -m scicompute_attention_b200.build`") from e
+        module.init(_scratch, acquire_scratch_fp32)
+        _native_module = module
+    return _native_module
 
 
 class _Scratch(threading.local):
@@ -177,6 +197,10 @@ def _default_scale(head_dim: int) -> float:
 def decode_attention(q, k, v, *, scale=None, num_splits: int = 0, layout: str = "bhsd",
                      seq_lens=None, stream=None, return_stats: bool = False):
     """Split-K decode over a contiguous KV cache; S_q must be 1 (sca::decode_attention)."""
+    if stream is None and num_splits <= 0 and not return_stats and q.is_cuda:
+        out = _native().decode(q, k, v, scale, layout, seq_lens)
+        if out is not None:
+            return out
     _require_cuda(q, k, v)
     b, hq, sq, d = _dims(q, layout)
     bk, hkv, skv, dk = _dims(k, layout)
@@ -234,6 +258,10 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
     `typical_len` / `longest_len` are optional host-side hints (the mean and the maximum sequence length, which a
     cache object tracks anyway) used only to size the partial scratch: enough slots for an even schedule. seq_order
     is accepted for compatibility and ignored: the kernel balances the work itself."""
+    if stream is None and num_splits <= 0 and not return_stats and seq_order is None and q.is_cuda:
+        out = _native().paged(q, k_pool, v_pool, page_table, seq_lens, block_size, scale, typical_len, longest_len)
+        if out is not None:
+            return out
     _require_cuda(q, k_pool, v_pool, page_table, seq_lens)
     if q.dim() != 4:
         raise _lib.ScaError(4, f"paged_attention expects q=[num_seqs, H_q, seq_q, D]; got ndims={q.dim()}")
@@ -383,6 +411,10 @@ def flash_status(device=None) -> int:
 def flash_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layout="bhsd", stream=None,
                     out=None, lse=None):
     """tcgen05 flash prefill (sca::flash_attention); fp16 / bf16 only."""
+    if stream is None and out is None and q.is_cuda:
+        res = _native().flash(q, k, v, causal, scale, return_lse, layout, False)
+        if res is not None:
+            return res
     _require_cuda(q, k, v)
     if q.dtype == torch.float32:
         raise _lib.ScaError(4, "flash backend computes in fp16/bf16; dtype=float32 is served by the naive "
@@ -397,6 +429,10 @@ def flash_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layo
 def flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_kv, *, causal=False, scale=None, stream=None):
     """Packed variable-length prefill in one launch. q [T_q, H_q, D], k / v [T_kv, H_kv, D] on the device;
     cu_seqlens_* are HOST int32 offsets (num_seqs + 1 entries, as in the reference API). Returns [T_q, H_q, D]."""
+    if stream is None and q.is_cuda:
+        out = _native().varlen(q, k, v, cu_seqlens_q, cu_seqlens_kv, causal, scale)
+        if out is not None:
+            return out
     import numpy as np
     _require_cuda(q, k, v)
     if q.dim() != 3 or k.dim() != 3 or tuple(k.shape) != tuple(v.shape) or not (q.is_contiguous() and k.is_contiguous() and v.is_contiguous()):
@@ -428,6 +464,10 @@ def flash_attention_paged(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_
     sequence), pools [num_blocks, block_size, H_kv, D], page_table int32 [num_seqs, max_blocks_per_seq] on the device,
     cu_seqlens_q (num_seqs + 1) and seq_lens_kv (num_seqs: tokens of each sequence in the cache, the new ones
     included) on the HOST. Returns [T_q, H_q, D]."""
+    if stream is None and q.is_cuda:
+        out = _native().chunk(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_kv, causal, scale)
+        if out is not None:
+            return out
     import numpy as np
     _require_cuda(q, k_pool, v_pool, page_table)
     if q.dim() != 3 or k_pool.dim() != 4 or tuple(k_pool.shape) != tuple(v_pool.shape) or not (
@@ -462,6 +502,10 @@ def flash_attention_paged(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_
 
 def simt_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layout="bhsd", stream=None):
     """Functional SIMT attention behind the naive / tiled backends (any compute dtype)."""
+    if stream is None and q.is_cuda:
+        res = _native().flash(q, k, v, causal, scale, return_lse, layout, True)
+        if res is not None:
+            return res
     _require_cuda(q, k, v)
     out, lse = _alloc_out(q, layout, return_lse, stream)
     p = _fwd_params(q, k, v, out, lse, causal, scale, layout)
@@ -492,6 +536,8 @@ def _kv_shape(pool: torch.Tensor) -> KvCacheShape:
 
 def kv_append(layer_k, layer_v, k_new, v_new, slot_mapping, *, stream=None) -> None:
     """k_new/v_new [num_tokens, H_kv, D]; slot_mapping int32 [num_tokens] on the device."""
+    if stream is None and layer_k.is_cuda and _native().append(layer_k, layer_v, k_new, v_new, slot_mapping):
+        return
     _require_cuda(layer_k, layer_v, k_new, v_new, slot_mapping)
     shape = _kv_shape(layer_k)
     check(lib().sca_launch_kv_append(layer_k.data_ptr(), layer_v.data_ptr(), k_new.data_ptr(),
@@ -501,6 +547,8 @@ def kv_append(layer_k, layer_v, k_new, v_new, slot_mapping, *, stream=None) -> N
 
 def kv_append_batched(layer_k, layer_v, k_new, v_new, page_table, seq_lens, *, stream=None) -> None:
     """One new token per sequence; the slot comes from the page table at position seq_lens[s] - 1."""
+    if stream is None and layer_k.is_cuda and _native().append_batched(layer_k, layer_v, k_new, v_new, page_table, seq_lens):
+        return
     _require_cuda(layer_k, layer_v, k_new, v_new, page_table, seq_lens)
     shape = _kv_shape(layer_k)
     check(lib().sca_launch_kv_append_batched(layer_k.data_ptr(), layer_v.data_ptr(), k_new.data_ptr(),
@@ -510,6 +558,8 @@ def kv_append_batched(layer_k, layer_v, k_new, v_new, page_table, seq_lens, *, s
 
 
 def kv_reset(layer_k, layer_v, block_ids, *, stream=None) -> None:
+    if stream is None and layer_k.is_cuda and _native().reset(layer_k, layer_v, block_ids):
+        return
     _require_cuda(layer_k, layer_v, block_ids)
     shape = _kv_shape(layer_k)
     check(lib().sca_launch_kv_reset_block(layer_k.data_ptr(), layer_v.data_ptr(), block_ids.data_ptr(),
@@ -518,6 +568,10 @@ def kv_reset(layer_k, layer_v, block_ids, *, stream=None) -> None:
 
 
 def kv_gather(layer, block_ids, *, stream=None) -> torch.Tensor:
+    if stream is None and layer.is_cuda:
+        out = _native().gather(layer, block_ids)
+        if out is not None:
+            return out
     _require_cuda(layer, block_ids)
     shape = _kv_shape(layer)
     out = _empty((block_ids.numel(),) + tuple(layer.shape[1:]), layer.dtype, layer.device, stream)
