@@ -6,12 +6,13 @@
 // whole row per thread in a byte loop (append). Here every thread moves 16 bytes, consecutive
 // threads touch consecutive 16-byte chunks of the same row (fully coalesced 128-byte lines), and K
 // and V are handled in the same pass. Addressing follows src/kv_cache/kv_cache_layout.cuh:32-38.
-// Rows whose byte length or base addresses are not 16-byte multiples fall back to a byte loop so
+// Rows whose byte length or base addresses are not 16-byte multiples fall back to single bytes so
 // the result is bit-exact for any geometry.
 //
 // Algorithmic traffic: append = 2 * tokens * kv_heads * D * elem bytes read + the same written;
 // reset = 2 * blocks * block_bytes written; gather = blocks * block_bytes read + written.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -20,24 +21,43 @@ namespace {
 
 constexpr int kKvThreads = 256;
 
-template <typename V>
+// A list of rows of `width` pieces of type V, cut into runs of kPieces * kKvThreads consecutive pieces, one run per CTA at a
+// time. A thread takes kPieces of a run, kKvThreads apart, and has all of their loads in flight before its first store. I is
+// 32 bits wide where the pieces can be counted in it: a 64-bit division per piece costs more than moving 16 bytes. Bound by
+// HBM: 668 MB (50 thousand tokens appended, 3000 blocks of 32 KB copied out, 1000 cleared, four launches) 126.4 us with one
+// piece and 64-bit counters, 115.4 now (5.8 TB/s); pieces of 32 bytes two at a time 115.2, four at a time 117.7.
+constexpr int kPieces = 4;
+
+template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
 kv_append_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __restrict__ k_new,
                  const V* __restrict__ v_new, const int32_t* __restrict__ slots,
-                 const int64_t num_tokens, const ScaKvCacheShape shape, const int64_t token_vecs) {
+                 const I total, const ScaKvCacheShape shape, const I token_vecs) {
     // token_vecs = kv_heads * D * elem_bytes / sizeof(V): one token's K (or V) payload is contiguous
     // both in the source [token][head][D] and in the pool [slot][head][D].
-    const int64_t total = num_tokens * token_vecs;
-    for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-         idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t token = idx / token_vecs;
-        const int64_t within = idx % token_vecs;
-        const int32_t slot = __ldg(slots + token);
-        if (slot < 0) continue;                                  // "do not store" sentinel
-        if (slot / shape.block_size >= shape.num_blocks) continue;  // never write out of range
-        const int64_t dst = static_cast<int64_t>(slot) * token_vecs + within;
-        layer_k[dst] = k_new[idx];
-        layer_v[dst] = v_new[idx];
+    constexpr int N = kPieces;
+    const int64_t pool_tokens = shape.num_blocks * shape.block_size;
+    for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
+        V k[N], v[N];
+        int64_t dst[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const I idx = run + i * kKvThreads + threadIdx.x;
+            dst[i] = -1;
+            if (idx >= total) continue;
+            const int32_t slot = __ldg(slots + idx / token_vecs);
+            if (slot < 0) continue;                    // "do not store" sentinel
+            if (slot >= pool_tokens) continue;         // never write out of range
+            dst[i] = static_cast<int64_t>(slot) * token_vecs + idx % token_vecs;
+            k[i] = k_new[idx];
+            v[i] = v_new[idx];
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (dst[i] < 0) continue;
+            layer_k[dst[i]] = k[i];
+            layer_v[dst[i]] = v[i];
+        }
     }
 }
 
@@ -68,36 +88,47 @@ kv_append_batched_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const
     }
 }
 
-template <typename V>
+template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
 kv_reset_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const int32_t* __restrict__ ids,
-                const int64_t count, const int64_t num_blocks, const int64_t block_vecs) {
-    const int64_t total = count * block_vecs;
+                const I total, const int64_t num_blocks, const I block_vecs) {
+    constexpr int N = kPieces;
     V zero;
     memset(&zero, 0, sizeof(V));
-    for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-         idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t phys = __ldg(ids + idx / block_vecs);
-        if (phys < 0 || phys >= num_blocks) continue;
-        const int64_t dst = static_cast<int64_t>(phys) * block_vecs + idx % block_vecs;
-        layer_k[dst] = zero;
-        layer_v[dst] = zero;
+    for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const I idx = run + i * kKvThreads + threadIdx.x;
+            if (idx >= total) continue;
+            const int32_t phys = __ldg(ids + idx / block_vecs);
+            if (phys < 0 || phys >= num_blocks) continue;
+            const int64_t dst = static_cast<int64_t>(phys) * block_vecs + idx % block_vecs;
+            layer_k[dst] = zero;
+            layer_v[dst] = zero;
+        }
     }
 }
 
-template <typename V>
+template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
-kv_gather_kernel(const V* __restrict__ layer, const int32_t* __restrict__ ids, const int64_t count,
-                 V* __restrict__ out, const int64_t num_blocks, const int64_t block_vecs) {
-    const int64_t total = count * block_vecs;
-    V zero;
-    memset(&zero, 0, sizeof(V));
-    for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-         idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t phys = __ldg(ids + idx / block_vecs);
-        out[idx] = (phys < 0 || phys >= num_blocks)
-                       ? zero
-                       : layer[static_cast<int64_t>(phys) * block_vecs + idx % block_vecs];
+kv_gather_kernel(const V* __restrict__ layer, const int32_t* __restrict__ ids, const I total,
+                 V* __restrict__ out, const int64_t num_blocks, const I block_vecs) {
+    constexpr int N = kPieces;
+    for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
+        V v[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const I idx = run + i * kKvThreads + threadIdx.x;
+            if (idx >= total) continue;
+            const int32_t phys = __ldg(ids + idx / block_vecs);
+            if (phys < 0 || phys >= num_blocks) memset(&v[i], 0, sizeof(V));
+            else v[i] = layer[static_cast<int64_t>(phys) * block_vecs + idx % block_vecs];
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const I idx = run + i * kKvThreads + threadIdx.x;
+            if (idx < total) out[idx] = v[i];
+        }
     }
 }
 
@@ -107,6 +138,19 @@ unsigned GridFor(int64_t items) {
     const int64_t want = (items + kKvThreads - 1) / kKvThreads;
     const int64_t cap = static_cast<int64_t>(SmCount()) * 32;
     return static_cast<unsigned>(std::max<int64_t>(1, std::min(want, cap)));
+}
+
+// Calls f(piece, total, width) with a null pointer to the piece type and counters of the index type the call allows: `rows`
+// rows of `row_bytes` bytes; `aligned`: all pointers lie on 16-byte boundaries. What a run may step past `total` fits too.
+template <typename F>
+void ForPieces(int64_t rows, int64_t row_bytes, bool aligned, const F& f) {
+    auto counted = [&](auto* piece) {
+        const int64_t width = row_bytes / static_cast<int64_t>(sizeof(*piece)), total = rows * width;
+        if (total < (1ll << 31)) f(piece, static_cast<uint32_t>(total), static_cast<uint32_t>(width));
+        else f(piece, total, width);
+    };
+    if (row_bytes % 16 == 0 && aligned) counted(static_cast<uint4*>(nullptr));
+    else counted(static_cast<unsigned char*>(nullptr));
 }
 
 int CheckShape(const ScaKvCacheShape* shape, int64_t elem_bytes, const char* what) {
@@ -184,19 +228,13 @@ extern "C" int sca_launch_kv_append(void* layer_k, void* layer_v, const void* k_
     if (int rc = CheckShape(shape, elem_bytes, "kv append")) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t token_bytes = shape->num_kv_heads * shape->head_dim * elem_bytes;
-    const bool vec = token_bytes % 16 == 0 && Aligned16(layer_k) && Aligned16(layer_v) &&
-                     Aligned16(k_new) && Aligned16(v_new);
-    if (vec) {
-        const int64_t tv = token_bytes / 16;
-        kv_append_kernel<uint4><<<GridFor(num_tokens * tv), kKvThreads, 0, s>>>(
-            static_cast<uint4*>(layer_k), static_cast<uint4*>(layer_v), static_cast<const uint4*>(k_new),
-            static_cast<const uint4*>(v_new), slot_mapping, num_tokens, *shape, tv);
-    } else {
-        kv_append_kernel<unsigned char><<<GridFor(num_tokens * token_bytes), kKvThreads, 0, s>>>(
-            static_cast<unsigned char*>(layer_k), static_cast<unsigned char*>(layer_v),
-            static_cast<const unsigned char*>(k_new), static_cast<const unsigned char*>(v_new),
-            slot_mapping, num_tokens, *shape, token_bytes);
-    }
+    const bool aligned = Aligned16(layer_k) && Aligned16(layer_v) && Aligned16(k_new) && Aligned16(v_new);
+    ForPieces(num_tokens, token_bytes, aligned, [&](auto* piece, auto total, auto width) {
+        using V = std::remove_pointer_t<decltype(piece)>;
+        kv_append_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+            static_cast<V*>(layer_k), static_cast<V*>(layer_v), static_cast<const V*>(k_new), static_cast<const V*>(v_new), slot_mapping,
+            total, *shape, width);
+    });
     return CheckLaunch("kv_append_kernel", s);
 }
 
@@ -246,16 +284,11 @@ extern "C" int sca_launch_kv_reset_block(void* layer_k, void* layer_v, const int
     if (int rc = ids.Stage(block_ids, num_blocks, s, "kv reset: staging host block ids")) return rc;
     block_ids = ids.get();
     const int64_t block_bytes = shape->block_size * shape->num_kv_heads * shape->head_dim * elem_bytes;
-    if (block_bytes % 16 == 0 && Aligned16(layer_k) && Aligned16(layer_v)) {
-        const int64_t bv = block_bytes / 16;
-        kv_reset_kernel<uint4><<<GridFor(num_blocks * bv), kKvThreads, 0, s>>>(
-            static_cast<uint4*>(layer_k), static_cast<uint4*>(layer_v), block_ids, num_blocks,
-            shape->num_blocks, bv);
-    } else {
-        kv_reset_kernel<unsigned char><<<GridFor(num_blocks * block_bytes), kKvThreads, 0, s>>>(
-            static_cast<unsigned char*>(layer_k), static_cast<unsigned char*>(layer_v), block_ids,
-            num_blocks, shape->num_blocks, block_bytes);
-    }
+    ForPieces(num_blocks, block_bytes, Aligned16(layer_k) && Aligned16(layer_v), [&](auto* piece, auto total, auto width) {
+        using V = std::remove_pointer_t<decltype(piece)>;
+        kv_reset_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+            static_cast<V*>(layer_k), static_cast<V*>(layer_v), block_ids, total, shape->num_blocks, width);
+    });
     return CheckLaunch("kv_reset_kernel", s);
 }
 
@@ -273,15 +306,10 @@ extern "C" int sca_launch_kv_gather(const void* layer, const int32_t* block_ids,
     if (int rc = ids.Stage(block_ids, num_blocks, s, "kv gather: staging host block ids")) return rc;
     block_ids = ids.get();
     const int64_t block_bytes = shape->block_size * shape->num_kv_heads * shape->head_dim * elem_bytes;
-    if (block_bytes % 16 == 0 && Aligned16(layer) && Aligned16(out)) {
-        const int64_t bv = block_bytes / 16;
-        kv_gather_kernel<uint4><<<GridFor(num_blocks * bv), kKvThreads, 0, s>>>(
-            static_cast<const uint4*>(layer), block_ids, num_blocks, static_cast<uint4*>(out),
-            shape->num_blocks, bv);
-    } else {
-        kv_gather_kernel<unsigned char><<<GridFor(num_blocks * block_bytes), kKvThreads, 0, s>>>(
-            static_cast<const unsigned char*>(layer), block_ids, num_blocks,
-            static_cast<unsigned char*>(out), shape->num_blocks, block_bytes);
-    }
+    ForPieces(num_blocks, block_bytes, Aligned16(layer) && Aligned16(out), [&](auto* piece, auto total, auto width) {
+        using V = std::remove_pointer_t<decltype(piece)>;
+        kv_gather_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+            static_cast<const V*>(layer), block_ids, total, static_cast<V*>(out), shape->num_blocks, width);
+    });
     return CheckLaunch("kv_gather_kernel", s);
 }
