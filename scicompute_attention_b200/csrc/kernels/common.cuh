@@ -30,11 +30,44 @@ int EnsureDynamicSmem(const void* kernel, size_t bytes, const char* kernel_name)
 // Cached SM count of the current device.
 int SmCount();
 
+// Launches `kernel` as a programmatic dependent of the kernel ahead of it on the stream (cluster > 1: on clusters of that many
+// CTAs): its CTAs may be set up while that one still runs. So the kernel calls one of the two functions below ahead of its first
+// access to global memory, reads and writes alike, in every CTA - its end then says that all kernels before it have ended.
+// Back to back on one stream, without / with: decode of one sequence 8.2 / 5.8 us a call, append + paged decode of 6 sequences
+// 14.3 / 10.3, a prompt of 203 tokens 10.3 / 8.1, KV append + two gathers + reset 115.7 / 109.
+template <typename... Params, typename... Args>
+void LaunchDependent(void (*kernel)(Params...), int64_t grid, int block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+    cudaLaunchAttribute attrs[2]{};
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attrs;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // CheckLaunch reports a failure
+}
+
 inline bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- device helpers -----------------------------------------------------------------------------
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
+
+// Kernels launched by LaunchDependent: waits until the kernel ahead on the stream has ended and its writes are visible (at
+// once where there is none).
+__device__ __forceinline__ void WaitForPredecessor() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// The same, and lets the next kernel on the stream be set up from here on.
+__device__ __forceinline__ void BeginAfterPredecessor() {
+    WaitForPredecessor();
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -432,6 +432,7 @@ decode_partial_kernel(const ScaDecodeFwdParams p, const int head_chunks) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int64_t s_part[kWarps][2];
     __shared__ int64_t s_found[2];
+    WaitForPredecessor();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int columns = static_cast<int>(p.num_kv_heads) * head_chunks;
@@ -585,6 +586,7 @@ template <typename T, int D, bool kPaged, bool kHi>
 __global__ void __launch_bounds__(kThreads)
 decode_cluster_kernel(const ScaDecodeFwdParams p, const int head_chunks, const int cluster) {
     extern __shared__ __align__(128) unsigned char smem[];
+    BeginAfterPredecessor();
     const int columns = static_cast<int>(p.num_kv_heads) * head_chunks;
     const int rank = static_cast<int>(ClusterRank());
     const int unit = static_cast<int>(blockIdx.x) / cluster;
@@ -815,9 +817,8 @@ int LaunchCluster(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     if (cluster < 2 || !ClusterIsFaster(units, steps, cluster, resident, p.seq_lens != nullptr, D, kHi, p.num_splits)) cluster = 0;
     *taken = cluster;
     if (cluster == 0) return SCA_OK;
-    cudaLaunchAttribute attr{};
-    const cudaLaunchConfig_t cfg = ClusterConfig(static_cast<unsigned>(units * cluster), cluster, DecodeGeom<D>::kSmemBytes, stream, &attr);
-    cudaLaunchKernelEx(&cfg, decode_cluster_kernel<T, D, kPaged, kHi>, p, head_chunks, cluster);
+    LaunchDependent(decode_cluster_kernel<T, D, kPaged, kHi>, units * cluster, kThreads, DecodeGeom<D>::kSmemBytes, stream, cluster, p,
+                    head_chunks, cluster);
     return CheckLaunch("decode_cluster_kernel", stream);
 }
 
@@ -838,8 +839,7 @@ int LaunchPartial(const ScaDecodeFwdParams& p, int head_chunks, cudaStream_t str
     } else {
         blocks = resident;  // more columns than resident CTAs: every CTA walks several columns
     }
-    decode_partial_kernel<T, D, kPaged, kHi>
-        <<<static_cast<unsigned>(blocks), kThreads, G::kSmemBytes, stream>>>(p, head_chunks);
+    LaunchDependent(decode_partial_kernel<T, D, kPaged, kHi>, blocks, kThreads, G::kSmemBytes, stream, 1, p, head_chunks);
     return CheckLaunch("decode_partial_kernel", stream);
 }
 

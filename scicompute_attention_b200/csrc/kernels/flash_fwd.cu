@@ -315,6 +315,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmem_base = *tmem_slot;
+    BeginAfterPredecessor();
 
     bool failed = false;
 
@@ -1172,15 +1173,15 @@ int LaunchFlash(const ScaFlashFwdParams& f, cudaStream_t stream, const VarlenWor
         while ((1 << p.block_shift) < p.block_size) ++p.block_shift;
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, true, true>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, true, true><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        LaunchDependent(flash_fwd_sm100_kernel<T, DP, QT, BN, true, true>, grid, threads, G::kSmemBytes, stream, 1, map_q, map_k, map_v, p);
     } else if (varlen != nullptr) {
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, true>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, true><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        LaunchDependent(flash_fwd_sm100_kernel<T, DP, QT, BN, true>, grid, threads, G::kSmemBytes, stream, 1, map_q, map_k, map_v, p);
     } else {
         const void* fn = reinterpret_cast<const void*>(&flash_fwd_sm100_kernel<T, DP, QT, BN, false>);
         if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "flash_fwd_sm100_kernel")) return rc;
-        flash_fwd_sm100_kernel<T, DP, QT, BN, false><<<grid, threads, G::kSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        LaunchDependent(flash_fwd_sm100_kernel<T, DP, QT, BN, false>, grid, threads, G::kSmemBytes, stream, 1, map_q, map_k, map_v, p);
     }
     if (int rc = CheckLaunch("flash_fwd_sm100_kernel", stream)) return rc;
     // With SCI_ATTENTION_DEBUG_SYNC=1 CheckLaunch has waited for the kernel: a wait that ran out is known now.

@@ -96,6 +96,7 @@ template <int D, int RT>
 __global__ void __launch_bounds__(kF32Threads, 1) fp32_tiled_attention_kernel(const F32Params p) {
     using G = F32Geom<D, RT>;
     extern __shared__ __align__(128) float f32_smem[];
+    BeginAfterPredecessor();
     const int lane = threadIdx.x & 31;
     const int group = threadIdx.x / kGroupThreads;
     const int tid = threadIdx.x % kGroupThreads;
@@ -292,7 +293,7 @@ int LaunchF32(F32Params p, int64_t bh, cudaStream_t stream) {
     }
     const void* fn = reinterpret_cast<const void*>(&fp32_tiled_attention_kernel<D, RT>);
     if (int rc = EnsureDynamicSmem(fn, G::kSmemBytes, "fp32_tiled_attention_kernel")) return rc;
-    fp32_tiled_attention_kernel<D, RT><<<static_cast<unsigned>(grid), kF32Threads, G::kSmemBytes, stream>>>(p);
+    LaunchDependent(fp32_tiled_attention_kernel<D, RT>, grid, kF32Threads, G::kSmemBytes, stream, 1, p);
     return CheckLaunch("fp32_tiled_attention_kernel", stream);
 }
 

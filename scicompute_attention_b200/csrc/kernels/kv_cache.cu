@@ -35,6 +35,7 @@ kv_append_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __re
                  const I total, const ScaKvCacheShape shape, const I token_vecs) {
     // token_vecs = kv_heads * D * elem_bytes / sizeof(V): one token's K (or V) payload is contiguous
     // both in the source [token][head][D] and in the pool [slot][head][D].
+    BeginAfterPredecessor();
     constexpr int N = kPieces;
     const int64_t pool_tokens = shape.num_blocks * shape.block_size;
     for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
@@ -70,6 +71,7 @@ kv_append_batched_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const
                          const int32_t* __restrict__ seq_lens, const int64_t num_seqs,
                          const int64_t max_blocks_per_seq, const ScaKvCacheShape shape,
                          const int64_t token_vecs) {
+    BeginAfterPredecessor();
     const int64_t total = num_seqs * token_vecs;
     for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
          idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -92,6 +94,7 @@ template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
 kv_reset_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const int32_t* __restrict__ ids,
                 const I total, const int64_t num_blocks, const I block_vecs) {
+    BeginAfterPredecessor();
     constexpr int N = kPieces;
     V zero;
     memset(&zero, 0, sizeof(V));
@@ -113,6 +116,7 @@ template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
 kv_gather_kernel(const V* __restrict__ layer, const int32_t* __restrict__ ids, const I total,
                  V* __restrict__ out, const int64_t num_blocks, const I block_vecs) {
+    BeginAfterPredecessor();
     constexpr int N = kPieces;
     for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
         V v[N];
@@ -231,7 +235,7 @@ extern "C" int sca_launch_kv_append(void* layer_k, void* layer_v, const void* k_
     const bool aligned = Aligned16(layer_k) && Aligned16(layer_v) && Aligned16(k_new) && Aligned16(v_new);
     ForPieces(num_tokens, token_bytes, aligned, [&](auto* piece, auto total, auto width) {
         using V = std::remove_pointer_t<decltype(piece)>;
-        kv_append_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+        LaunchDependent(kv_append_kernel<V, decltype(total)>, GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s, 1,
             static_cast<V*>(layer_k), static_cast<V*>(layer_v), static_cast<const V*>(k_new), static_cast<const V*>(v_new), slot_mapping,
             total, *shape, width);
     });
@@ -258,11 +262,11 @@ extern "C" int sca_launch_kv_append_batched(void* layer_k, void* layer_v, const 
                      Aligned16(k_new) && Aligned16(v_new);
     if (vec) {
         const int64_t tv = token_bytes / 16;
-        kv_append_batched_kernel<uint4><<<GridFor(num_seqs * tv), kKvThreads, 0, s>>>(
+        LaunchDependent(kv_append_batched_kernel<uint4>, GridFor(num_seqs * tv), kKvThreads, 0, s, 1,
             static_cast<uint4*>(layer_k), static_cast<uint4*>(layer_v), static_cast<const uint4*>(k_new),
             static_cast<const uint4*>(v_new), page_table, seq_lens, num_seqs, max_blocks_per_seq, *shape, tv);
     } else {
-        kv_append_batched_kernel<unsigned char><<<GridFor(num_seqs * token_bytes), kKvThreads, 0, s>>>(
+        LaunchDependent(kv_append_batched_kernel<unsigned char>, GridFor(num_seqs * token_bytes), kKvThreads, 0, s, 1,
             static_cast<unsigned char*>(layer_k), static_cast<unsigned char*>(layer_v),
             static_cast<const unsigned char*>(k_new), static_cast<const unsigned char*>(v_new), page_table,
             seq_lens, num_seqs, max_blocks_per_seq, *shape, token_bytes);
@@ -286,7 +290,7 @@ extern "C" int sca_launch_kv_reset_block(void* layer_k, void* layer_v, const int
     const int64_t block_bytes = shape->block_size * shape->num_kv_heads * shape->head_dim * elem_bytes;
     ForPieces(num_blocks, block_bytes, Aligned16(layer_k) && Aligned16(layer_v), [&](auto* piece, auto total, auto width) {
         using V = std::remove_pointer_t<decltype(piece)>;
-        kv_reset_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+        LaunchDependent(kv_reset_kernel<V, decltype(total)>, GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s, 1,
             static_cast<V*>(layer_k), static_cast<V*>(layer_v), block_ids, total, shape->num_blocks, width);
     });
     return CheckLaunch("kv_reset_kernel", s);
@@ -308,7 +312,7 @@ extern "C" int sca_launch_kv_gather(const void* layer, const int32_t* block_ids,
     const int64_t block_bytes = shape->block_size * shape->num_kv_heads * shape->head_dim * elem_bytes;
     ForPieces(num_blocks, block_bytes, Aligned16(layer) && Aligned16(out), [&](auto* piece, auto total, auto width) {
         using V = std::remove_pointer_t<decltype(piece)>;
-        kv_gather_kernel<V><<<GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s>>>(
+        LaunchDependent(kv_gather_kernel<V, decltype(total)>, GridFor((total + kPieces - 1) / kPieces), kKvThreads, 0, s, 1,
             static_cast<const V*>(layer), block_ids, total, static_cast<V*>(out), shape->num_blocks, width);
     });
     return CheckLaunch("kv_gather_kernel", s);

@@ -39,6 +39,7 @@ constexpr int kMaxPerLane = 8;  // head_dim <= 256
 
 template <typename T>
 __global__ void __launch_bounds__(128) simt_attention_kernel(const SimtParams p) {
+    BeginAfterPredecessor();
     const int lane = threadIdx.x & 31;
     const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t total = p.batch * p.heads * p.seq_q * p.splits;
@@ -135,9 +136,9 @@ int LaunchSimt(const SimtParams& p, int dtype, cudaStream_t stream) {
     }
     const unsigned grid = static_cast<unsigned>(blocks);
     switch (dtype) {
-        case SCA_DTYPE_F32: simt_attention_kernel<float><<<grid, 128, 0, stream>>>(p); break;
-        case SCA_DTYPE_F16: simt_attention_kernel<__half><<<grid, 128, 0, stream>>>(p); break;
-        case SCA_DTYPE_BF16: simt_attention_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>(p); break;
+        case SCA_DTYPE_F32: LaunchDependent(simt_attention_kernel<float>, grid, 128, 0, stream, 1, p); break;
+        case SCA_DTYPE_F16: LaunchDependent(simt_attention_kernel<__half>, grid, 128, 0, stream, 1, p); break;
+        case SCA_DTYPE_BF16: LaunchDependent(simt_attention_kernel<__nv_bfloat16>, grid, 128, 0, stream, 1, p); break;
         default: return Fail(SCA_INVALID_ARGUMENT, "simt attention: unsupported dtype id " + std::to_string(dtype));
     }
     return CheckLaunch("simt_attention_kernel", stream);
