@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 
@@ -54,6 +55,27 @@ void LaunchDependent(void (*kernel)(Params...), int64_t grid, int block, size_t 
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // CheckLaunch reports a failure
 }
 
+// The answer of an occupancy query, kept per device. `ask` returns a negative number when the device cannot say; that is
+// not kept. Threads that ask at the same time store the same number.
+class PerDevice {
+public:
+    template <typename Ask>
+    int Get(Ask ask) {
+        int device = 0;
+        const bool kept = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < kMaxDevices;
+        if (kept) {
+            if (const int n = answers_[device].load(std::memory_order_relaxed); n != 0) return n - 1;
+        }
+        const int n = ask();
+        if (kept && n >= 0) answers_[device].store(n + 1, std::memory_order_relaxed);
+        return n;
+    }
+
+private:
+    static constexpr int kMaxDevices = 64;
+    std::atomic<int> answers_[kMaxDevices] = {};  // answer + 1, 0 = not asked yet
+};
+
 inline bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- device helpers -----------------------------------------------------------------------------
@@ -67,6 +89,37 @@ __device__ __forceinline__ void WaitForPredecessor() { asm volatile("griddepcont
 __device__ __forceinline__ void BeginAfterPredecessor() {
     WaitForPredecessor();
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t ClusterRank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void ClusterBarrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// A float in the shared memory of CTA `rank` of this cluster, at this CTA's address `addr`.
+__device__ __forceinline__ float LoadFromRank(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 LoadFromRank2(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float2 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 LoadFromRank4(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
 }
 
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {

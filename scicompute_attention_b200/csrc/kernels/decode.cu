@@ -562,23 +562,6 @@ decode_partial_kernel(const ScaDecodeFwdParams p, const int head_chunks) {
     }
 }
 
-__device__ __forceinline__ uint32_t ClusterRank() {
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void ClusterBarrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// A float in the shared memory of CTA `rank` of this cluster, at this CTA's address `addr`.
-__device__ __forceinline__ float LoadFromRank(uint32_t addr, uint32_t rank) {
-    uint32_t remote;
-    float v;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-    return v;
-}
-
 // Decode of a problem that does not fill the machine, in one launch: the CTAs of a cluster split one (sequence, kv head,
 // head chunk) and merge their partials through distributed shared memory. Bound by latency - a step or two of K/V per
 // CTA, then the exchange - so what counts is that there is no second kernel and no trip through memory in between.
@@ -713,27 +696,6 @@ cudaLaunchConfig_t ClusterConfig(unsigned grid, int cluster, int smem_bytes, cud
     cfg.numAttrs = 1;
     return cfg;
 }
-
-// The answer of an occupancy query, kept per device. `ask` returns a negative number when the device cannot say; that is
-// not kept. Threads that ask at the same time store the same number.
-class PerDevice {
-public:
-    template <typename Ask>
-    int Get(Ask ask) {
-        int device = 0;
-        const bool kept = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < kMaxDevices;
-        if (kept) {
-            if (const int n = answers_[device].load(std::memory_order_relaxed); n != 0) return n - 1;
-        }
-        const int n = ask();
-        if (kept && n >= 0) answers_[device].store(n + 1, std::memory_order_relaxed);
-        return n;
-    }
-
-private:
-    static constexpr int kMaxDevices = 64;
-    std::atomic<int> answers_[kMaxDevices] = {};  // answer + 1, 0 = not asked yet
-};
 
 // CTAs of the decode kernels that stay resident together.
 template <typename T, int D, bool kPaged, bool kHi>
