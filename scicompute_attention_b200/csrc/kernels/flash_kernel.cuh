@@ -372,23 +372,31 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             const int32_t* row = p.page_table + static_cast<int64_t>(w.seq) * p.max_blocks_per_seq;
-            // page ids of a KV tile, one per lane; looked up a tile ahead, so that the ring does not wait for the table
+            // Page ids of a KV tile, one per lane; looked up a tile ahead, so that the ring does not wait for the table. At D=128 a
+            // look-up per load is short against the step, and what looking ahead adds to the loop costs more than it saves (20
+            // chunks against 512 to 6000 keys, lasting load, ahead / per load: D=128 429 / 400 us, D=64 299 / 324, D=256 1032 / 1125).
+            constexpr bool kLookAhead = kOwnP;
             auto page_ids = [&](int tile) {
                 const int logical = ((kSplit ? w.first_tile : 0) + tile) * pages_per_tile + lane;
                 const bool in = lane < pages_per_tile && logical < p.max_blocks_per_seq && (static_cast<int64_t>(logical) << p.block_shift) < w.seq_kv;
                 return in ? __ldg(row + logical) : -1;
             };
-            int32_t ids_before = -1, ids = -1, ids_next = page_ids(0);  // of the tiles before, of and behind the last K loaded
+            int32_t ids_before = -1, ids = -1, ids_next = kLookAhead ? page_ids(0) : -1;  // of the tiles before, of and behind the last K loaded
             for (int it = 0; it < 2 * w.n_max * kParts && ok; ++it, ++kv_loads) {
                 const RingLoad load = RingOrder(it / kParts, w.n_max, kOwnP);
                 const bool is_v = load.is_v;
                 const int tile = load.tile;
-                if (!is_v && it % kParts == 0) {
-                    ids_before = ids;
-                    ids = ids_next;
-                    if (tile + 1 < w.n_max) ids_next = page_ids(tile + 1);
+                int32_t phys;
+                if constexpr (kLookAhead) {
+                    if (!is_v && it % kParts == 0) {
+                        ids_before = ids;
+                        ids = ids_next;
+                        if (tile + 1 < w.n_max) ids_next = page_ids(tile + 1);
+                    }
+                    phys = is_v && tile + 1 < w.n_max ? ids_before : ids;
+                } else {
+                    phys = page_ids(tile);
                 }
-                const int32_t phys = is_v && kOwnP && tile + 1 < w.n_max ? ids_before : ids;
                 const bool mapped = phys >= 0 && phys < p.num_kv_blocks;
                 const uint32_t valid = __ballot_sync(0xffffffffu, mapped);
                 const uint32_t slot = kv_loads % G::kSlots;
@@ -766,11 +774,18 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 if (ragged) {
 #pragma unroll
                     for (int c = 0; c < BN / 32; ++c) {
+                        // bit i: column 32 * c + i is visible
+                        const int seen = limit - 32 * c;
+                        uint32_t visible = seen >= 32 ? 0xffffffffu : seen <= 0 ? 0u : (1u << seen) - 1u;
+                        if (kPaged && holes) {
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) {  // a page has 8 keys at least
+                                if (!((pages >> ((32 * c + 8 * g) >> p.block_shift)) & 1u)) visible &= ~(0xffu << (8 * g));
+                            }
+                        }
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const int col = c * 32 + i;
-                            const bool gone = kPaged && holes && !((pages >> (col >> p.block_shift)) & 1u);
-                            if (col >= limit || gone) sc[c][i] = 0xff800000u;  // -inf
+                            if (!(visible & (1u << i))) sc[c][i] = 0xff800000u;  // -inf
                         }
                     }
                 }
