@@ -34,6 +34,9 @@ int SmCount();
 // Launches `kernel` as a programmatic dependent of the kernel ahead of it on the stream (cluster > 1: on clusters of that many
 // CTAs): its CTAs may be set up while that one still runs. So the kernel calls one of the two functions below ahead of its first
 // access to global memory, reads and writes alike, in every CTA - its end then says that all kernels before it have ended.
+// It also reads global memory with ordinary loads only: the kernel ahead may write while this one is already there, and the
+// loads of __ldg and of const __restrict__ pointers are for memory that nobody writes while the kernel lives; neither the
+// wait nor its memory clobber holds such a load back.
 // Back to back on one stream, without / with: decode of one sequence 8.2 / 5.8 us a call, append + paged decode of 6 sequences
 // 14.3 / 10.3, a prompt of 203 tokens 10.3 / 8.1, KV append + two gathers + reset 115.7 / 109.
 template <typename... Params, typename... Args>

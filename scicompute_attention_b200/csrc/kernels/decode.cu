@@ -75,7 +75,7 @@ constexpr int kSpan = kWarps * kTile;
 // kSpan-token steps it takes. An empty sequence still counts one (empty) step so that somebody writes its partial.
 template <bool kPaged>
 __device__ __forceinline__ int64_t SeqLen(const ScaDecodeFwdParams& p, int64_t b) {
-    int64_t len = p.seq_lens != nullptr ? static_cast<int64_t>(__ldg(p.seq_lens + b)) : p.seq_kv;
+    int64_t len = p.seq_lens != nullptr ? static_cast<int64_t>(p.seq_lens[b]) : p.seq_kv;
     if (len < 0) len = 0;
     const int64_t cap = kPaged ? p.max_blocks_per_seq * p.block_size : p.seq_kv;
     return len < cap ? len : cap;
@@ -149,7 +149,7 @@ __device__ __forceinline__ void DecodeSegment(const ScaDecodeFwdParams& p, unsig
     int offset = 0, offset_step = 0, block_size = 1;
     int32_t phys_next = -1;
     auto fetch_entry = [&](int64_t jt) {
-        phys_next = (lane < kTile && jt < j_end && page < p.max_blocks_per_seq) ? __ldg(table_row + page) : -1;
+        phys_next = (lane < kTile && jt < j_end && page < p.max_blocks_per_seq) ? table_row[page] : -1;
     };
     if (kPaged) {
         block_size = static_cast<int>(p.block_size);
@@ -625,7 +625,7 @@ struct MergeSource {
 template <typename T, bool kTriples>
 __global__ void __launch_bounds__(256)
 decode_merge_kernel(const MergeSource src, const int64_t rows, const int parts, const int head_dim,
-                    void* __restrict__ out, const int64_t heads, const int64_t o_sb, const int64_t o_sh) {
+                    void* out, const int64_t heads, const int64_t o_sb, const int64_t o_sh) {
     // launched with programmatic stream serialisation: the grid may start before the kernel that produces the parts
     // has finished; this returns once that kernel is complete and its writes are visible (a no-op otherwise)
     asm volatile("griddepcontrol.wait;\n" ::: "memory");

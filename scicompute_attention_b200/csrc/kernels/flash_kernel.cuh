@@ -251,8 +251,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         Item w;
         int mb;
         if constexpr (kVarlen) {
-            const int2 entry = __ldg(p.entries + idx / packed_heads);
-            const int4 seq = __ldg(p.seqs + entry.x);
+            const int2 entry = p.entries[idx / packed_heads];
+            const int4 seq = p.seqs[entry.x];
             mb = entry.y;
             w.seq = entry.x;
             w.b = 0;
@@ -379,7 +379,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             auto page_ids = [&](int tile) {
                 const int logical = ((kSplit ? w.first_tile : 0) + tile) * pages_per_tile + lane;
                 const bool in = lane < pages_per_tile && logical < p.max_blocks_per_seq && (static_cast<int64_t>(logical) << p.block_shift) < w.seq_kv;
-                return in ? __ldg(row + logical) : -1;
+                return in ? row[logical] : -1;
             };
             int32_t ids_before = -1, ids = -1, ids_next = kLookAhead ? page_ids(0) : -1;  // of the tiles before, of and behind the last K loaded
             for (int it = 0; it < 2 * w.n_max * kParts && ok; ++it, ++kv_loads) {

@@ -30,9 +30,8 @@ constexpr int kPieces = 4;
 
 template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
-kv_append_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __restrict__ k_new,
-                 const V* __restrict__ v_new, const int32_t* __restrict__ slots,
-                 const I total, const ScaKvCacheShape shape, const I token_vecs) {
+kv_append_kernel(V* layer_k, V* layer_v, const V* k_new, const V* v_new, const int32_t* slots, const I total,
+                 const ScaKvCacheShape shape, const I token_vecs) {
     // token_vecs = kv_heads * D * elem_bytes / sizeof(V): one token's K (or V) payload is contiguous
     // both in the source [token][head][D] and in the pool [slot][head][D].
     BeginAfterPredecessor();
@@ -46,7 +45,7 @@ kv_append_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __re
             const I idx = run + i * kKvThreads + threadIdx.x;
             dst[i] = -1;
             if (idx >= total) continue;
-            const int32_t slot = __ldg(slots + idx / token_vecs);
+            const int32_t slot = slots[idx / token_vecs];
             if (slot < 0) continue;                    // "do not store" sentinel
             if (slot >= pool_tokens) continue;         // never write out of range
             dst[i] = static_cast<int64_t>(slot) * token_vecs + idx % token_vecs;
@@ -66,10 +65,8 @@ kv_append_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __re
 // sequence at position seq_lens[s] - 1.
 template <typename V>
 __global__ void __launch_bounds__(kKvThreads)
-kv_append_batched_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const V* __restrict__ k_new,
-                         const V* __restrict__ v_new, const int32_t* __restrict__ page_table,
-                         const int32_t* __restrict__ seq_lens, const int64_t num_seqs,
-                         const int64_t max_blocks_per_seq, const ScaKvCacheShape shape,
+kv_append_batched_kernel(V* layer_k, V* layer_v, const V* k_new, const V* v_new, const int32_t* page_table, const int32_t* seq_lens,
+                         const int64_t num_seqs, const int64_t max_blocks_per_seq, const ScaKvCacheShape shape,
                          const int64_t token_vecs) {
     BeginAfterPredecessor();
     const int64_t total = num_seqs * token_vecs;
@@ -77,45 +74,50 @@ kv_append_batched_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const
          idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t seq = idx / token_vecs;
         const int64_t within = idx % token_vecs;
-        const int64_t pos = static_cast<int64_t>(__ldg(seq_lens + seq)) - 1;
+        const V k = k_new[idx], v = v_new[idx];  // on their way while the length and the table entry are looked up
+        const int64_t pos = static_cast<int64_t>(seq_lens[seq]) - 1;
         if (pos < 0) continue;
         const int64_t logical = pos / shape.block_size;
         if (logical >= max_blocks_per_seq) continue;
-        const int32_t phys = __ldg(page_table + seq * max_blocks_per_seq + logical);
+        const int32_t phys = page_table[seq * max_blocks_per_seq + logical];
         if (phys < 0 || phys >= shape.num_blocks) continue;
         const int64_t slot = static_cast<int64_t>(phys) * shape.block_size + pos % shape.block_size;
         const int64_t dst = slot * token_vecs + within;
-        layer_k[dst] = k_new[idx];
-        layer_v[dst] = v_new[idx];
+        layer_k[dst] = k;
+        layer_v[dst] = v;
     }
 }
 
 template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
-kv_reset_kernel(V* __restrict__ layer_k, V* __restrict__ layer_v, const int32_t* __restrict__ ids,
-                const I total, const int64_t num_blocks, const I block_vecs) {
+kv_reset_kernel(V* layer_k, V* layer_v, const int32_t* ids, const I total, const int64_t num_blocks, const I block_vecs) {
     BeginAfterPredecessor();
     constexpr int N = kPieces;
     V zero;
     memset(&zero, 0, sizeof(V));
     for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
+        int64_t dst[N];  // all of a run's ids are read ahead of its first store
 #pragma unroll
         for (int i = 0; i < N; ++i) {
             const I idx = run + i * kKvThreads + threadIdx.x;
+            dst[i] = -1;
             if (idx >= total) continue;
-            const int32_t phys = __ldg(ids + idx / block_vecs);
+            const int32_t phys = ids[idx / block_vecs];
             if (phys < 0 || phys >= num_blocks) continue;
-            const int64_t dst = static_cast<int64_t>(phys) * block_vecs + idx % block_vecs;
-            layer_k[dst] = zero;
-            layer_v[dst] = zero;
+            dst[i] = static_cast<int64_t>(phys) * block_vecs + idx % block_vecs;
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (dst[i] < 0) continue;
+            layer_k[dst[i]] = zero;
+            layer_v[dst[i]] = zero;
         }
     }
 }
 
 template <typename V, typename I>
 __global__ void __launch_bounds__(kKvThreads)
-kv_gather_kernel(const V* __restrict__ layer, const int32_t* __restrict__ ids, const I total,
-                 V* __restrict__ out, const int64_t num_blocks, const I block_vecs) {
+kv_gather_kernel(const V* layer, const int32_t* ids, const I total, V* out, const int64_t num_blocks, const I block_vecs) {
     BeginAfterPredecessor();
     constexpr int N = kPieces;
     for (I run = static_cast<I>(blockIdx.x) * (N * kKvThreads); run < total; run += static_cast<I>(gridDim.x) * (N * kKvThreads)) {
@@ -124,7 +126,7 @@ kv_gather_kernel(const V* __restrict__ layer, const int32_t* __restrict__ ids, c
         for (int i = 0; i < N; ++i) {
             const I idx = run + i * kKvThreads + threadIdx.x;
             if (idx >= total) continue;
-            const int32_t phys = __ldg(ids + idx / block_vecs);
+            const int32_t phys = ids[idx / block_vecs];
             if (phys < 0 || phys >= num_blocks) memset(&v[i], 0, sizeof(V));
             else v[i] = layer[static_cast<int64_t>(phys) * block_vecs + idx % block_vecs];
         }

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(128) simt_attention_kernel(const SimtParams p)
         if (paged) {
             const int64_t logical = j / p.block_size;
             if (logical >= p.max_blocks_per_seq) continue;
-            const int32_t phys = __ldg(p.page_table + b * p.max_blocks_per_seq + logical);
+            const int32_t phys = p.page_table[b * p.max_blocks_per_seq + logical];
             if (phys < 0 || phys >= p.num_kv_blocks) continue;
             row = static_cast<int64_t>(phys) * p.block_size + j % p.block_size;
         }
