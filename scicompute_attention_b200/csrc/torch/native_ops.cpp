@@ -69,6 +69,13 @@ bool Int(PyObject* obj, int64_t* value) {
     *value = PyLong_AsLongLongAndOverflow(obj, &overflow);
     return overflow == 0;
 }
+// A device list of at least `count` int32 entries.
+bool Ints(const at::Tensor& t, int64_t count) { return t.scalar_type() == at::kInt && t.is_contiguous() && t.numel() >= count; }
+// A page table of at least `rows` rows.
+bool Table(const at::Tensor& t, int64_t rows) { return t.scalar_type() == at::kInt && t.dim() == 2 && t.size(0) >= rows && t.is_contiguous(); }
+bool SameType(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v) {
+    return q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type();
+}
 // An int32 array on the host (numpy), one-dimensional and contiguous.
 class HostInts {
 public:
@@ -153,8 +160,8 @@ PyObject* Flash(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (!q || !k || !v || !Flag(a[3], &causal) || !Flag(a[5], &want_lse) || !Flag(a[7], &simt) || !PyUnicode_Check(a[6])) return NotTaken();
         bshd = PyUnicode_CompareWithASCIIString(a[6], "bshd") == 0;
         if (!bshd && PyUnicode_CompareWithASCIIString(a[6], "bhsd") != 0) return NotTaken();
-        if (q->dim() != 4 || k->dim() != 4 || !q->is_contiguous() || !k->is_contiguous() || k->sizes() != v->sizes() ||
-            q->scalar_type() != k->scalar_type() || q->scalar_type() != v->scalar_type() || !DtypeId(*q, &p.dtype_id) ||
+        if (q->dim() != 4 || k->dim() != 4 || !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() ||
+            k->sizes() != v->sizes() || !SameType(*q, *k, *v) || !DtypeId(*q, &p.dtype_id) ||
             (!simt && p.dtype_id == SCA_DTYPE_F32)) {
             return NotTaken();
         }
@@ -220,15 +227,15 @@ PyObject* Decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const bool bshd = PyUnicode_CompareWithASCIIString(a[4], "bshd") == 0;
         if (!bshd && PyUnicode_CompareWithASCIIString(a[4], "bhsd") != 0) return NotTaken();
         ScaDecodeFwdParams p{};
-        if (q->dim() != 4 || k->dim() != 4 || !q->is_contiguous() || !k->is_contiguous() || k->sizes() != v->sizes() ||
-            q->scalar_type() != k->scalar_type() || q->scalar_type() != v->scalar_type() || !DtypeId(*q, &p.dtype)) {
+        if (q->dim() != 4 || k->dim() != 4 || !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() ||
+            k->sizes() != v->sizes() || !SameType(*q, *k, *v) || !DtypeId(*q, &p.dtype)) {
             return NotTaken();
         }
         const int head = bshd ? 2 : 1, seq = bshd ? 1 : 2;
         p.batch = q->size(0), p.num_heads = q->size(head), p.head_dim = q->size(3), p.num_kv_heads = k->size(head), p.seq_kv = k->size(seq);
         const int64_t d = p.head_dim;
         if (q->size(seq) != 1 || k->size(0) != p.batch || k->size(3) != d || p.num_kv_heads < 1 || p.num_heads % p.num_kv_heads != 0 ||
-            !Scale(a[3], d, &p.scale)) {
+            (lens != nullptr && !Ints(*lens, p.batch)) || !Scale(a[3], d, &p.scale)) {
             return NotTaken();
         }
         const int64_t group = p.num_heads / p.num_kv_heads, steps = Steps(p.seq_kv);
@@ -255,7 +262,8 @@ PyObject* Paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (!q || !k || !v || !table || !Int(a[5], &block_size) || !Int(a[7], &typical) || !Int(a[8], &longest)) return NotTaken();
         if (a[4] != Py_None && (lens = Plain(a[4])) == nullptr) return NotTaken();
         if (q->dim() != 4 || q->size(2) != 1 || k->dim() != 4 || k->size(1) != block_size || k->size(3) != q->size(3) || k->sizes() != v->sizes() ||
-            table->scalar_type() != at::kInt || table->dim() != 2 || table->size(0) < q->size(0) || !DtypeId(*q, &p.dtype)) {
+            !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() || !SameType(*q, *k, *v) || !Table(*table, q->size(0)) ||
+            (lens != nullptr && !Ints(*lens, q->size(0))) || !DtypeId(*q, &p.dtype)) {
             return NotTaken();
         }
         p.batch = q->size(0), p.num_heads = q->size(1), p.head_dim = q->size(3), p.num_kv_heads = k->size(2);
@@ -293,7 +301,7 @@ PyObject* Varlen(PyObject*, PyObject* const* a, Py_ssize_t n) {
         bool causal;
         ScaFlashVarlenParams p{};
         if (!q || !k || !v || !cu_q.Take(a[3]) || !cu_kv.Take(a[4]) || !Flag(a[5], &causal) || !DtypeId(*q, &p.dtype_id)) return NotTaken();
-        if (q->dim() != 3 || k->dim() != 3 || k->sizes() != v->sizes() || !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() ||
+        if (q->dim() != 3 || k->dim() != 3 || k->size(2) != q->size(2) || k->sizes() != v->sizes() || !SameType(*q, *k, *v) || !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() ||
             cu_q.size() != cu_kv.size() || cu_q.size() < 2 || !Scale(a[6], q->size(2), &p.scale)) {
             return NotTaken();
         }
@@ -318,9 +326,8 @@ PyObject* Chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
         bool causal;
         ScaFlashPagedParams p{};
         if (!q || !k || !v || !table || !cu_q.Take(a[4]) || !lens.Take(a[5]) || !Flag(a[6], &causal) || !DtypeId(*q, &p.dtype_id)) return NotTaken();
-        if (q->dim() != 3 || k->dim() != 4 || k->sizes() != v->sizes() || !q->is_contiguous() || !k->is_contiguous() || !v->is_contiguous() ||
-            !table->is_contiguous() || table->scalar_type() != at::kInt || table->dim() != 2 || cu_q.size() != lens.size() + 1 ||
-            table->size(0) < lens.size() || k->size(3) != q->size(2) || !Scale(a[7], q->size(2), &p.scale)) {
+        if (q->dim() != 3 || k->dim() != 4 || k->sizes() != v->sizes() || !SameType(*q, *k, *v) || !q->is_contiguous() || !k->is_contiguous() ||
+            !v->is_contiguous() || !Table(*table, lens.size()) || cu_q.size() != lens.size() + 1 || k->size(3) != q->size(2) || !Scale(a[7], q->size(2), &p.scale)) {
             return NotTaken();
         }
         p.total_q = q->size(0), p.num_heads = q->size(1), p.head_dim = q->size(2), p.num_seqs = lens.size();
@@ -338,9 +345,23 @@ PyObject* Chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ---- KV cache ------------------------------------------------------------------------------------------------------------
 bool PoolShape(const at::Tensor& pool, ScaKvCacheShape* s) {
-    if (pool.dim() != 4) return false;
+    if (pool.dim() != 4 || !pool.is_contiguous()) return false;
     *s = ScaKvCacheShape{pool.size(0), pool.size(1), pool.size(2), pool.size(3)};
     return true;
+}
+// As _same_kind, _require_pools and _require_rows in ops.py.
+bool SameKind(const at::Tensor& a, const at::Tensor& b) {
+    return a.scalar_type() == b.scalar_type() || (a.element_size() == b.element_size() && !(a.is_floating_point() && b.is_floating_point()));
+}
+bool Pools(const at::Tensor& k, const at::Tensor& v, ScaKvCacheShape* s) {
+    return PoolShape(k, s) && v.dim() == 4 && v.is_contiguous() && v.sizes().slice(1) == k.sizes().slice(1) && v.size(0) >= k.size(0) && SameKind(v, k);
+}
+bool Rows(const at::Tensor& t, int64_t rows, const at::Tensor& pool) {
+    return t.is_contiguous() && t.size(0) >= rows && t.numel() == t.size(0) * pool.size(2) * pool.size(3) && SameKind(t, pool);
+}
+// New K / V of `kn`'s rows for the pools.
+bool NewRows(const at::Tensor& k, const at::Tensor& v, const at::Tensor& kn, const at::Tensor& vn, ScaKvCacheShape* s) {
+    return Pools(k, v, s) && kn.dim() >= 1 && vn.dim() >= 1 && Rows(kn, kn.size(0), k) && Rows(vn, kn.size(0), k);
 }
 
 // append(k_pool, v_pool, k_new, v_new, slots)
@@ -349,7 +370,7 @@ PyObject* Append(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (n != 5) return NotTaken();
         const at::Tensor *k = Plain(a[0]), *v = Plain(a[1]), *kn = Plain(a[2]), *vn = Plain(a[3]), *slots = Plain(a[4]);
         ScaKvCacheShape shape;
-        if (!k || !v || !kn || !vn || !slots || !PoolShape(*k, &shape) || kn->dim() < 1) return NotTaken();
+        if (!k || !v || !kn || !vn || !slots || !NewRows(*k, *v, *kn, *vn, &shape) || !Ints(*slots, kn->size(0))) return NotTaken();
         void* stream = CurrentStream();
         const int rc = Launch([&] {
             return sca_launch_kv_append(k->data_ptr(), v->data_ptr(), kn->data_ptr(), vn->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
@@ -365,7 +386,10 @@ PyObject* AppendBatched(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (n != 6) return NotTaken();
         const at::Tensor *k = Plain(a[0]), *v = Plain(a[1]), *kn = Plain(a[2]), *vn = Plain(a[3]), *table = Plain(a[4]), *lens = Plain(a[5]);
         ScaKvCacheShape shape;
-        if (!k || !v || !kn || !vn || !table || !lens || !PoolShape(*k, &shape) || kn->dim() < 1 || table->dim() < 2) return NotTaken();
+        if (!k || !v || !kn || !vn || !table || !lens || !NewRows(*k, *v, *kn, *vn, &shape) || !Table(*table, kn->size(0)) ||
+            !Ints(*lens, kn->size(0))) {
+            return NotTaken();
+        }
         void* stream = CurrentStream();
         const int rc = Launch([&] {
             return sca_launch_kv_append_batched(k->data_ptr(), v->data_ptr(), kn->data_ptr(), vn->data_ptr(), static_cast<const int32_t*>(table->data_ptr()),
@@ -382,7 +406,7 @@ PyObject* Reset(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (n != 3) return NotTaken();
         const at::Tensor *k = Plain(a[0]), *v = Plain(a[1]), *ids = Plain(a[2]);
         ScaKvCacheShape shape;
-        if (!k || !v || !ids || !PoolShape(*k, &shape)) return NotTaken();
+        if (!k || !v || !ids || !Pools(*k, *v, &shape) || !Ints(*ids, 0)) return NotTaken();
         void* stream = CurrentStream();
         const int rc = Launch([&] {
             return sca_launch_kv_reset_block(k->data_ptr(), v->data_ptr(), static_cast<const int32_t*>(ids->data_ptr()), ids->numel(), &shape,
@@ -398,7 +422,7 @@ PyObject* Gather(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (n != 2) return NotTaken();
         const at::Tensor *pool = Plain(a[0]), *ids = Plain(a[1]);
         ScaKvCacheShape shape;
-        if (!pool || !ids || !PoolShape(*pool, &shape)) return NotTaken();
+        if (!pool || !ids || !PoolShape(*pool, &shape) || !Ints(*ids, 0)) return NotTaken();
         at::Tensor out = Empty({ids->numel(), pool->size(1), pool->size(2), pool->size(3)}, *pool, pool->scalar_type());
         void* stream = CurrentStream();
         const int rc = Launch([&] {

@@ -77,6 +77,50 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise _lib.ScaError(5, "device=cpu (attention kernels run on CUDA devices only; there is no CPU path)")
 
 
+def _require_packed(what: str, *tensors: torch.Tensor) -> None:
+    """The kernels address rows through the strides of a contiguous tensor."""
+    for t in tensors:
+        if not t.is_contiguous():
+            raise _lib.ScaError(4, f"non-contiguous {what} rejected; pass a contiguous tensor")
+
+
+def _require_ints(what: str, t: torch.Tensor, count: int) -> None:
+    """A device list of at least `count` int32 entries."""
+    _require_cuda(t)
+    if t.dtype != torch.int32 or not t.is_contiguous() or t.numel() < count:
+        raise _lib.ScaError(4, f"{what} must be a contiguous int32 tensor of at least {count} entries; got {t.dtype}{list(t.shape)}")
+
+
+def _require_table(page_table: torch.Tensor, rows: int) -> None:
+    if page_table.dtype != torch.int32 or page_table.dim() != 2 or page_table.shape[0] < rows or not page_table.is_contiguous():
+        raise _lib.ScaError(4, "page_table must be int32 [num_seqs, max_blocks_per_seq], contiguous")
+
+
+def _require_like(q, k, v) -> None:
+    if q.dtype != k.dtype or q.dtype != v.dtype:
+        raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
+
+
+def _same_kind(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """Whether rows of `a` may be stored as rows of `b`: the same type, or raw integers of its width on one side."""
+    return a.dtype == b.dtype or (a.element_size() == b.element_size() and not (a.is_floating_point() and b.is_floating_point()))
+
+
+def _require_pools(layer_k, layer_v) -> None:
+    _require_packed("pool", layer_k, layer_v)
+    if tuple(layer_k.shape[1:]) != tuple(layer_v.shape[1:]) or layer_v.shape[0] < layer_k.shape[0] or not _same_kind(layer_v, layer_k):
+        raise _lib.ScaError(4, "pool geometry mismatch")
+
+
+def _require_rows(pool, rows: int, *tensors: torch.Tensor) -> None:
+    """New K / V rows: at least `rows` of them, each [H_kv, D] of the pool in any shape, of the pool's type."""
+    width = pool.shape[2] * pool.shape[3]
+    for t in tensors:
+        if not t.is_contiguous() or t.dim() < 1 or t.shape[0] < rows or t.numel() != t.shape[0] * width or not _same_kind(t, pool):
+            raise _lib.ScaError(4, f"new K / V must be contiguous [{rows}, {pool.shape[2]}, {pool.shape[3]}] of the pool's type {pool.dtype}; "
+                                   f"got {t.dtype}{list(t.shape)}")
+
+
 def sm_count(device: torch.device) -> int:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _sm_count:
@@ -208,8 +252,11 @@ def decode_attention(q, k, v, *, scale=None, num_splits: int = 0, layout: str = 
         raise _lib.ScaError(5, f"decode backend requires seq_q=1; seq_q={sq} belongs to the flash backend")
     if (bk, dk) != (b, d) or tuple(v.shape) != tuple(k.shape) or q.dtype != k.dtype or q.dtype != v.dtype:
         raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
+    _require_packed("v", v)
     if hq % hkv != 0:
         raise _lib.ScaError(4, f"num_heads={hq} % num_kv_heads={hkv} != 0")
+    if seq_lens is not None:
+        _require_ints("seq_lens", seq_lens, b)
     device, handle = q.device, _stream_ptr(stream)
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(device))
     base = b * hq * splits
@@ -271,8 +318,11 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
     nblk, bs, hkv, dk = k_pool.shape
     if bs != block_size or dk != d or tuple(v_pool.shape) != tuple(k_pool.shape):
         raise _lib.ScaError(4, "pool geometry mismatch")
-    if page_table.dtype != torch.int32 or page_table.dim() != 2 or page_table.shape[0] < s:
-        raise _lib.ScaError(4, "page_table must be int32 [num_seqs, max_blocks_per_seq]")
+    _require_like(q, k_pool, v_pool)
+    _require_packed("q or pool", q, k_pool, v_pool)
+    _require_table(page_table, s)
+    if seq_lens is not None:
+        _require_ints("seq_lens", seq_lens, s)
     max_blocks = page_table.shape[1]
     upper = nblk * bs
     device, handle = q.device, _stream_ptr(stream)
@@ -306,12 +356,21 @@ def paged_attention(q, k_pool, v_pool, page_table, seq_lens, *, block_size: int,
     return _launch_decode(p, num_splits, handle, out, return_stats)
 
 
+def _shard_dims(q, k, v):
+    b, hq, sq, d = _dims(q, "bhsd")
+    bk, hkv, skv, dk = _dims(k, "bhsd")
+    if sq != 1 or (bk, dk) != (b, d) or tuple(v.shape) != tuple(k.shape):
+        raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
+    _require_like(q, k, v)
+    _require_packed("v", v)
+    return b, hq, hkv, skv, d
+
+
 def decode_triples(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     """This rank's share of a sequence-split decode: merged but unnormalised {m, l, O[D]} per
     (batch, head), fp32 [B*H_q, 2 + D]."""
     _require_cuda(q, k, v)
-    b, hq, sq, d = _dims(q, "bhsd")
-    _, hkv, skv, _ = _dims(k, "bhsd")
+    b, hq, hkv, skv, d = _shard_dims(q, k, v)
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
     base = b * hq * splits
     ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
@@ -335,8 +394,7 @@ def decode_partials(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
     """The split-K partial kernel alone. Returns (m [rows, splits], l [rows, splits], O [rows, splits, D],
     splits) as fp32 views of the scratch pool (valid until this thread's next decode call on the stream)."""
     _require_cuda(q, k, v)
-    b, hq, sq, d = _dims(q, "bhsd")
-    _, hkv, skv, _ = _dims(k, "bhsd")
+    b, hq, hkv, skv, d = _shard_dims(q, k, v)
     splits = min(num_splits, MAX_SPLITS) if num_splits > 0 else splits_for(skv, b, hkv, hq // hkv, sm_count(q.device))
     base = b * hq * splits
     ws = acquire_scratch_fp32(base * (2 + d), q.device, stream=stream)
@@ -358,6 +416,9 @@ def decode_partials(q, k, v, *, scale=None, num_splits: int = 0, stream=None):
 def merge_triples(gathered, out_dtype, *, stream=None):
     """gathered fp32 [ranks, rows, 2 + D] -> normalised output [rows, D] of `out_dtype`."""
     _require_cuda(gathered)
+    _require_packed("triples", gathered)
+    if gathered.dtype != torch.float32:
+        raise _lib.ScaError(4, f"triples must be float32; got {gathered.dtype}")
     ranks, rows, width = gathered.shape
     d = width - 2
     out = _empty((rows, d), out_dtype, gathered.device, stream)
@@ -374,6 +435,10 @@ def _fwd_params(q, k, v, out, lse, causal, scale, layout):
     bk, hkv, skv, dk = _dims(k, layout)
     if (bk, dk) != (b, d) or tuple(v.shape) != tuple(k.shape) or q.dtype != k.dtype or q.dtype != v.dtype:
         raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
+    _require_packed("v", v)
+    if not out.is_contiguous() or out.dtype != q.dtype or out.numel() < q.numel() or (
+            lse is not None and (not lse.is_contiguous() or lse.dtype != torch.float32 or lse.numel() < b * hq * sq)):
+        raise _lib.ScaError(4, "out must be a contiguous tensor of q's type and size, lse of float32 and one entry per row")
     if causal and skv < sq:
         raise _lib.ScaError(4, f"causal=true but seq_kv({skv}) < seq_q({sq})")
     p = FlashFwdParams()
@@ -421,6 +486,8 @@ def flash_attention(q, k, v, *, causal=False, scale=None, return_lse=False, layo
                                "(reference) or tiled backend")
     if out is None:
         out, lse = _alloc_out(q, layout, return_lse, stream)
+    else:
+        _require_cuda(out, lse)
     p = _fwd_params(q, k, v, out, lse, causal, scale, layout)
     check(lib().sca_launch_flash_fwd(C.byref(p), _stream_ptr(stream)))
     return (out, lse) if return_lse else out
@@ -437,6 +504,9 @@ def flash_attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_kv, *, causal=False
     _require_cuda(q, k, v)
     if q.dim() != 3 or k.dim() != 3 or tuple(k.shape) != tuple(v.shape) or not (q.is_contiguous() and k.is_contiguous() and v.is_contiguous()):
         raise _lib.ScaError(4, "varlen expects contiguous packed [T, H, D] tensors")
+    _require_like(q, k, v)
+    if k.shape[2] != q.shape[2]:
+        raise _lib.ScaError(4, "q/k/v shape or dtype mismatch")
     cu_q = np.ascontiguousarray(cu_seqlens_q, dtype=np.int32)
     cu_kv = np.ascontiguousarray(cu_seqlens_kv, dtype=np.int32)
     if cu_q.ndim != 1 or cu_q.shape != cu_kv.shape or cu_q.shape[0] < 2:
@@ -473,6 +543,7 @@ def flash_attention_paged(q, k_pool, v_pool, page_table, cu_seqlens_q, seq_lens_
     if q.dim() != 3 or k_pool.dim() != 4 or tuple(k_pool.shape) != tuple(v_pool.shape) or not (
             q.is_contiguous() and k_pool.is_contiguous() and v_pool.is_contiguous() and page_table.is_contiguous()):
         raise _lib.ScaError(4, "paged prefill expects packed q [T, H, D] and contiguous pools [blocks, block_size, H_kv, D]")
+    _require_like(q, k_pool, v_pool)
     if page_table.dtype != torch.int32 or page_table.dim() != 2:
         raise _lib.ScaError(4, "page_table must be int32 [num_seqs, max_blocks_per_seq]")
     cu_q = np.ascontiguousarray(cu_seqlens_q, dtype=np.int32)
@@ -540,6 +611,9 @@ def kv_append(layer_k, layer_v, k_new, v_new, slot_mapping, *, stream=None) -> N
         return
     _require_cuda(layer_k, layer_v, k_new, v_new, slot_mapping)
     shape = _kv_shape(layer_k)
+    _require_pools(layer_k, layer_v)
+    _require_rows(layer_k, k_new.shape[0], k_new, v_new)
+    _require_ints("slot_mapping", slot_mapping, k_new.shape[0])
     check(lib().sca_launch_kv_append(layer_k.data_ptr(), layer_v.data_ptr(), k_new.data_ptr(),
                                      v_new.data_ptr(), slot_mapping.data_ptr(), k_new.shape[0],
                                      C.byref(shape), layer_k.element_size(), _stream_ptr(stream)))
@@ -551,6 +625,10 @@ def kv_append_batched(layer_k, layer_v, k_new, v_new, page_table, seq_lens, *, s
         return
     _require_cuda(layer_k, layer_v, k_new, v_new, page_table, seq_lens)
     shape = _kv_shape(layer_k)
+    _require_pools(layer_k, layer_v)
+    _require_rows(layer_k, k_new.shape[0], k_new, v_new)
+    _require_table(page_table, k_new.shape[0])
+    _require_ints("seq_lens", seq_lens, k_new.shape[0])
     check(lib().sca_launch_kv_append_batched(layer_k.data_ptr(), layer_v.data_ptr(), k_new.data_ptr(),
                                              v_new.data_ptr(), page_table.data_ptr(), seq_lens.data_ptr(),
                                              k_new.shape[0], page_table.shape[1], C.byref(shape),
@@ -562,6 +640,8 @@ def kv_reset(layer_k, layer_v, block_ids, *, stream=None) -> None:
         return
     _require_cuda(layer_k, layer_v, block_ids)
     shape = _kv_shape(layer_k)
+    _require_pools(layer_k, layer_v)
+    _require_ints("block_ids", block_ids, 0)
     check(lib().sca_launch_kv_reset_block(layer_k.data_ptr(), layer_v.data_ptr(), block_ids.data_ptr(),
                                           block_ids.numel(), C.byref(shape), layer_k.element_size(),
                                           _stream_ptr(stream)))
@@ -574,6 +654,8 @@ def kv_gather(layer, block_ids, *, stream=None) -> torch.Tensor:
             return out
     _require_cuda(layer, block_ids)
     shape = _kv_shape(layer)
+    _require_packed("pool", layer)
+    _require_ints("block_ids", block_ids, 0)
     out = _empty((block_ids.numel(),) + tuple(layer.shape[1:]), layer.dtype, layer.device, stream)
     check(lib().sca_launch_kv_gather(layer.data_ptr(), block_ids.data_ptr(), block_ids.numel(),
                                      out.data_ptr(), C.byref(shape), layer.element_size(),
