@@ -154,6 +154,20 @@ int64_t VarlenListBytes(const VarlenWork& vw, int64_t tokens) {
     return vw.num_seqs * static_cast<int64_t>(sizeof(int4)) + VarlenEntries(vw, tokens) * static_cast<int64_t>(sizeof(int2));
 }
 
+// Every sequence has tokens on both sides. Nothing may be sized by the offsets before this holds: offsets that go up and down
+// between the right ends describe any number of entries.
+int CheckSequences(const VarlenWork& vw, bool causal) {
+    for (int64_t s = 0; s < vw.num_seqs; ++s) {
+        const int64_t sq = static_cast<int64_t>(vw.cu_q[s + 1]) - vw.cu_q[s];
+        const int64_t skv = static_cast<int64_t>(vw.cu_kv[s + 1]) - vw.cu_kv[s];
+        if (sq <= 0 || skv <= 0 || (causal && skv < sq)) {
+            return Fail(SCA_INVALID_ARGUMENT, "flash varlen: sequence " + std::to_string(s) + " has S_q=" + std::to_string(sq) +
+                                                  ", S_kv=" + std::to_string(skv) + (causal ? " (causal needs 0 < S_q <= S_kv)" : " (both must be > 0)"));
+        }
+    }
+    return SCA_OK;
+}
+
 // Builds {first q token, first kv token, S_q, S_kv} per sequence and the (sequence, query block) list, heaviest
 // block first, and copies both into the workspace (stream-ordered; the host vector may die on return).
 int UploadVarlenWork(const VarlenWork& vw, int tokens_per_entry, int block_n, bool causal, cudaStream_t stream,
@@ -169,10 +183,6 @@ int UploadVarlenWork(const VarlenWork& vw, int tokens_per_entry, int block_n, bo
     for (int64_t s = 0; s < vw.num_seqs; ++s) {
         const int64_t sq = static_cast<int64_t>(vw.cu_q[s + 1]) - vw.cu_q[s];
         const int64_t skv = static_cast<int64_t>(vw.cu_kv[s + 1]) - vw.cu_kv[s];
-        if (sq <= 0 || skv <= 0 || (causal && skv < sq)) {
-            return Fail(SCA_INVALID_ARGUMENT, "flash varlen: sequence " + std::to_string(s) + " has S_q=" + std::to_string(sq) +
-                                                  ", S_kv=" + std::to_string(skv) + (causal ? " (causal needs 0 < S_q <= S_kv)" : " (both must be > 0)"));
-        }
         image[static_cast<size_t>(s)] = make_int4(vw.cu_q[s], vw.cu_kv[s], static_cast<int>(sq), static_cast<int>(skv));
         for (int64_t mb = 0; mb * tokens_per_entry < sq; ++mb) {
             int64_t limit = skv;
@@ -432,7 +442,7 @@ extern "C" long long sca_flash_varlen_workspace_bytes(int64_t num_seqs, int64_t 
 
 // Packed variable-length prefill in ONE launch (the reference loops over the sequences on the host,
 // src/backends/flash/flash_backend.cpp:312-363): the persistent kernel's work list simply spans all sequences.
-extern "C" int sca_launch_flash_varlen(const ScaFlashVarlenParams* params, void* stream) {
+extern "C" int sca_launch_flash_varlen(const ScaFlashVarlenParams* params, void* stream) try {
     ClearError();
     if (params == nullptr || params->cu_seqlens_q == nullptr || params->cu_seqlens_kv == nullptr) {
         return Fail(SCA_INVALID_ARGUMENT, "flash varlen: null parameter block or host offsets");
@@ -471,12 +481,15 @@ extern "C" int sca_launch_flash_varlen(const ScaFlashVarlenParams* params, void*
     f.dtype_id = x.dtype_id;
     if (int rc = ValidateFlash(&f)) return rc;
     VarlenWork vw{x.cu_seqlens_q, x.cu_seqlens_kv, x.num_seqs, x.workspace, x.workspace_bytes};
+    if (int rc = CheckSequences(vw, f.causal != 0)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return f.dtype_id == SCA_DTYPE_F16 ? LaunchFlashTyped<__half>(f, s, &vw)
                                        : LaunchFlashTyped<__nv_bfloat16>(f, s, &vw);
+} catch (const std::exception& e) {  // host memory for the work list
+    return Fail(SCA_CUDA_ERROR, std::string("flash varlen: on the host: ") + e.what());
 }
 
-extern "C" int sca_launch_flash_paged(const ScaFlashPagedParams* params, void* stream) {
+extern "C" int sca_launch_flash_paged(const ScaFlashPagedParams* params, void* stream) try {
     ClearError();
     if (params == nullptr || params->cu_seqlens_q == nullptr || params->seq_lens_kv == nullptr) {
         return Fail(SCA_INVALID_ARGUMENT, "flash paged: null parameter block or host lengths");
@@ -531,6 +544,7 @@ extern "C" int sca_launch_flash_paged(const ScaFlashPagedParams* params, void* s
     f.dtype_id = x.dtype_id;
     if (int rc = ValidateFlash(&f)) return rc;
     VarlenWork vw{x.cu_seqlens_q, cu_kv.data(), x.num_seqs, x.workspace, x.workspace_bytes};
+    if (int rc = CheckSequences(vw, f.causal != 0)) return rc;
     PagedWork pw{x.page_table, x.num_blocks, x.block_size, x.max_blocks_per_seq};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     switch (f.dtype_id) {
@@ -539,4 +553,6 @@ extern "C" int sca_launch_flash_paged(const ScaFlashPagedParams* params, void* s
         default: break;
     }
     return Fail(SCA_INVALID_ARGUMENT, "flash paged: unsupported dtype id");
+} catch (const std::exception& e) {  // host memory for the work list
+    return Fail(SCA_CUDA_ERROR, std::string("flash paged: on the host: ") + e.what());
 }

@@ -107,13 +107,20 @@ at::Tensor Empty(at::IntArrayRef shape, const at::Tensor& like, at::ScalarType t
     return at::empty(shape, at::TensorOptions().dtype(type).device(like.device()));
 }
 // Other threads run while a launch waits for room in the stream's queue.
+class OtherThreadsRun {
+public:
+    OtherThreadsRun() : state_(PyEval_SaveThread()) {}
+    ~OtherThreadsRun() { PyEval_RestoreThread(state_); }  // also when the launch throws
+    OtherThreadsRun(const OtherThreadsRun&) = delete;
+    OtherThreadsRun& operator=(const OtherThreadsRun&) = delete;
+
+private:
+    PyThreadState* state_;
+};
 template <typename F>
 int Launch(const F& f) {
-    int rc = 0;
-    Py_BEGIN_ALLOW_THREADS
-    rc = f();
-    Py_END_ALLOW_THREADS
-    return rc;
+    OtherThreadsRun here;
+    return f();
 }
 // Nothing that goes wrong here is an error of its own: the general path meets it again and says what it is.
 template <typename F>
