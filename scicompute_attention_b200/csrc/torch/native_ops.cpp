@@ -2,7 +2,8 @@
 //
 // Each function looks at its arguments, allocates the outputs, fills the parameter block of the C ABI and launches. It returns
 // what the operator returns (True where that is None), or None for "not taken": arguments in any other form than the plain
-// one, anything ops.py would refuse, a launch that reported an error. ops.py then goes its own way, which raises the errors.
+// one, anything ops.py would refuse. ops.py then goes its own way, which raises the errors. A launch that failed is not tried
+// again: its error is raised here.
 // No state is kept here: scratch comes from the calling thread's pool in ops.py.
 //
 // Why: decode_attention at B=1 took 14.6 us a call on the host (ctypes fields one by one, shape tuples, dictionary look-ups)
@@ -27,6 +28,7 @@ constexpr int64_t kDecodeStepTokens = 64;
 
 PyObject* g_scratch = nullptr;          // ops._scratch: threading.local with the dict `pool`
 PyObject* g_acquire_scratch = nullptr;  // ops.acquire_scratch_fp32
+PyObject* g_check = nullptr;            // _lib.check: raises the error of a status code
 
 // ---- arguments ---------------------------------------------------------------------------------------------------------
 // A plain CUDA tensor with memory of its own kind; null for anything else (subclasses, transforms' wrappers, sparse, ...).
@@ -122,7 +124,19 @@ int Launch(const F& f) {
     OtherThreadsRun here;
     return f();
 }
-// Nothing that goes wrong here is an error of its own: the general path meets it again and says what it is.
+// What a launch that did not return SCA_OK comes to. A refusal leaves nothing behind, so the general path may meet it again and
+// say what it is. Anything else has been told once: the last error and the word of a prefill that gave up have been read, and
+// a second launch that succeeds would hide them.
+PyObject* NotLaunched(int rc) {
+    if (rc == SCA_INVALID_ARGUMENT || rc == SCA_NOT_IMPLEMENTED) return NotTaken();
+    PyObject* none = PyObject_CallFunction(g_check, "i", rc);
+    if (none != nullptr) {
+        Py_DECREF(none);
+        PyErr_Format(PyExc_RuntimeError, "a launch failed with status %d", rc);
+    }
+    return nullptr;
+}
+// Nothing else that goes wrong here is an error of its own: the general path meets it again.
 template <typename F>
 PyObject* Guarded(const F& f) {
     try {
@@ -187,7 +201,7 @@ PyObject* Flash(PyObject*, PyObject* const* a, Py_ssize_t n) {
         p.q = q->data_ptr(), p.k = k->data_ptr(), p.v = v->data_ptr(), p.out = out.data_ptr();
         p.lse = want_lse ? static_cast<float*>(lse.data_ptr()) : nullptr;
         void* stream = CurrentStream();
-        if (Launch([&] { return simt ? sca_launch_simt_forward(&p, stream) : sca_launch_flash_fwd(&p, stream); }) != SCA_OK) return NotTaken();
+        if (const int rc = Launch([&] { return simt ? sca_launch_simt_forward(&p, stream) : sca_launch_flash_fwd(&p, stream); })) return NotLaunched(rc);
         if (!want_lse) return THPVariable_Wrap(std::move(out));
         return Py_BuildValue("(NN)", THPVariable_Wrap(std::move(out)), THPVariable_Wrap(std::move(lse)));
     });
@@ -220,7 +234,7 @@ PyObject* FinishDecode(ScaDecodeFwdParams& p, const at::Tensor& q, PyObject* q_o
     at::Tensor out = Empty({p.batch, p.num_heads, 1, d}, q, q.scalar_type());
     p.out = out.data_ptr();
     p.partial_m = scratch, p.partial_l = scratch + base, p.partial_o = scratch + 2 * base;
-    if (Launch([&] { return sca_launch_decode_auto(&p, nullptr, stream); }) != SCA_OK) return NotTaken();
+    if (const int rc = Launch([&] { return sca_launch_decode_auto(&p, nullptr, stream); })) return NotLaunched(rc);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -319,7 +333,7 @@ PyObject* Varlen(PyObject*, PyObject* const* a, Py_ssize_t n) {
         p.cu_seqlens_q = cu_q.data(), p.cu_seqlens_kv = cu_kv.data(), p.causal = causal;
         p.workspace = ws.data_ptr(), p.workspace_bytes = ws.numel();
         void* stream = CurrentStream();
-        if (Launch([&] { return sca_launch_flash_varlen(&p, stream); }) != SCA_OK) return NotTaken();
+        if (const int rc = Launch([&] { return sca_launch_flash_varlen(&p, stream); })) return NotLaunched(rc);
         return THPVariable_Wrap(std::move(out));
     });
 }
@@ -345,7 +359,7 @@ PyObject* Chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
         p.cu_seqlens_q = cu_q.data(), p.seq_lens_kv = lens.data(), p.causal = causal;
         p.workspace = ws.data_ptr(), p.workspace_bytes = ws.numel();
         void* stream = CurrentStream();
-        if (Launch([&] { return sca_launch_flash_paged(&p, stream); }) != SCA_OK) return NotTaken();
+        if (const int rc = Launch([&] { return sca_launch_flash_paged(&p, stream); })) return NotLaunched(rc);
         return THPVariable_Wrap(std::move(out));
     });
 }
@@ -383,7 +397,7 @@ PyObject* Append(PyObject*, PyObject* const* a, Py_ssize_t n) {
             return sca_launch_kv_append(k->data_ptr(), v->data_ptr(), kn->data_ptr(), vn->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
                                         kn->size(0), &shape, k->element_size(), stream);
         });
-        return rc == SCA_OK ? Done() : NotTaken();
+        return rc == SCA_OK ? Done() : NotLaunched(rc);
     });
 }
 
@@ -403,7 +417,7 @@ PyObject* AppendBatched(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                                 static_cast<const int32_t*>(lens->data_ptr()), kn->size(0), table->size(1), &shape,
                                                 k->element_size(), stream);
         });
-        return rc == SCA_OK ? Done() : NotTaken();
+        return rc == SCA_OK ? Done() : NotLaunched(rc);
     });
 }
 
@@ -419,7 +433,7 @@ PyObject* Reset(PyObject*, PyObject* const* a, Py_ssize_t n) {
             return sca_launch_kv_reset_block(k->data_ptr(), v->data_ptr(), static_cast<const int32_t*>(ids->data_ptr()), ids->numel(), &shape,
                                              k->element_size(), stream);
         });
-        return rc == SCA_OK ? Done() : NotTaken();
+        return rc == SCA_OK ? Done() : NotLaunched(rc);
     });
 }
 
@@ -436,18 +450,19 @@ PyObject* Gather(PyObject*, PyObject* const* a, Py_ssize_t n) {
             return sca_launch_kv_gather(pool->data_ptr(), static_cast<const int32_t*>(ids->data_ptr()), ids->numel(), out.data_ptr(), &shape,
                                         pool->element_size(), stream);
         });
-        return rc == SCA_OK ? THPVariable_Wrap(std::move(out)) : NotTaken();
+        return rc == SCA_OK ? THPVariable_Wrap(std::move(out)) : NotLaunched(rc);
     });
 }
 
-// init(scratch_local, acquire_scratch)
+// init(scratch_local, acquire_scratch, check)
 PyObject* Init(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 2) {
-        PyErr_SetString(PyExc_TypeError, "init(scratch_local, acquire_scratch)");
+    if (n != 3) {
+        PyErr_SetString(PyExc_TypeError, "init(scratch_local, acquire_scratch, check)");
         return nullptr;
     }
     Py_XSETREF(g_scratch, Py_NewRef(a[0]));
     Py_XSETREF(g_acquire_scratch, Py_NewRef(a[1]));
+    Py_XSETREF(g_check, Py_NewRef(a[2]));
     Py_RETURN_NONE;
 }
 

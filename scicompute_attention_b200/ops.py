@@ -41,7 +41,7 @@ def _native():
         except ImportError as e:
             raise RuntimeError("scicompute_attention_b200/_native.so is missing or does not fit this torch: build it with "
                                "`python -m scicompute_attention_b200.build`") from e
-        module.init(_scratch, acquire_scratch_fp32)
+        module.init(_scratch, acquire_scratch_fp32, check)
         _native_module = module
     return _native_module
 
