@@ -3,7 +3,7 @@ so that they travel with the source tree).
 
   libsca_b200.so      hand-written sm_100a CUDA behind the C ABI of include/sca_b200.h
   libsci_attention.so C++ host layer (public sca:: API, dispatcher, KV cache) on top of it
-  _native.so          the operators of ops.py for torch tensors, without the Python in between
+  _native.<abi>.so    the operators of ops.py for torch tensors, without the Python in between
 
 `python -m scicompute_attention_b200.build` builds them all; `--force` rebuilds everything.
 """
@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -23,7 +24,7 @@ OBJ = os.path.join(ROOT, "build", "obj")
 INCLUDE = os.path.join(ROOT, "include")
 KERNEL_LIB = os.path.join(PKG, "libsca_b200.so")
 HOST_LIB = os.path.join(PKG, "libsci_attention.so")
-NATIVE_OPS = os.path.join(PKG, "_native.so")
+NATIVE_OPS = os.path.join(PKG, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))  # another Python does not import it
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -112,22 +113,25 @@ def build_host(force: bool = False, verbose: bool = False) -> str | None:
 
 
 def build_native_ops(force: bool = False, verbose: bool = False) -> str:
-    """csrc/torch/native_ops.cpp -> _native.so, a CPython module against the installed torch."""
-    import sysconfig
-
+    """csrc/torch/native_ops.cpp -> _native.<abi>.so, a CPython module against the installed torch."""
     import torch
+
+    from .ops import torch_build
     src = os.path.join(CSRC, "torch", "native_ops.cpp")
     # a module that was built against another torch or Python is built again
     stamp = os.path.join(OBJ, "native_ops.built_with")
-    built_with = f"{torch.__version__} {sys.version}"
+    built_with = f"{torch_build()} {sys.version}"
     same = os.path.exists(stamp) and open(stamp).read() == built_with
     if force or not same or not _newer(NATIVE_OPS, [src, os.path.join(INCLUDE, "sca_b200.h")]):
         os.makedirs(OBJ, exist_ok=True)
+        plain = os.path.join(PKG, "_native.so")  # the module's name once, which any Python would import
+        if os.path.exists(plain):
+            os.remove(plain)
         torch_dir = os.path.dirname(torch.__file__)
         torch_lib = os.path.join(torch_dir, "lib")
         cuda = os.path.dirname(os.path.dirname(_nvcc()))
         _run([shutil.which("g++") or "g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
-              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", INCLUDE,
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DSCA_BUILT_WITH="{torch_build()}"', "-I", INCLUDE,
               "-isystem", os.path.join(torch_dir, "include"), "-isystem", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
               "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"), src, "-o", NATIVE_OPS,
               "-L", PKG, "-l:libsca_b200.so", "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",

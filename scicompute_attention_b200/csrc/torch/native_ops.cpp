@@ -487,4 +487,8 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Plain operator calls 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__native() {
+    PyObject* module = PyModule_Create(&g_module);
+    if (module != nullptr && PyModule_AddStringConstant(module, "built_with", SCA_BUILT_WITH) != 0) Py_CLEAR(module);
+    return module;
+}

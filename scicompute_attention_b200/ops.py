@@ -16,6 +16,7 @@ import functools
 import math
 import struct
 import threading
+import warnings
 
 import torch
 
@@ -32,16 +33,32 @@ MAX_SCRATCH_BUFFERS = 32  # scratch buffers a thread keeps
 _native_module = None
 
 
+def torch_build() -> str:
+    """The torch a native module fits: it reads tensors through this build's headers."""
+    return f"{torch.__version__} {torch.version.git_version}"
+
+
+class _GeneralFormOnly:
+    def __getattr__(self, name):
+        return lambda *args: None  # takes no call
+
+
 def _native():
-    """The native form of the operators. There is no fallback: on a GPU it has to have been built."""
+    """The native form of the operators. Where it has not been built, or for another torch, the general form serves every call
+    (the kernels are the same ones) and a warning says so once."""
     global _native_module
     if _native_module is None:
         try:
             from . import _native as module
+            why = None if module.built_with == torch_build() else f"was built for torch {module.built_with}, this is {torch_build()}"
         except ImportError as e:
-            raise RuntimeError("scicompute_attention_b200/_native.so is missing or does not fit this torch: build it with "
-                               "`python -m scicompute_attention_b200.build`") from e
-        module.init(_scratch, acquire_scratch_fp32, check)
+            why = f"does not load ({e})"
+        if why is None:
+            module.init(_scratch, acquire_scratch_fp32, check)
+        else:
+            warnings.warn(f"scicompute_attention_b200._native {why}: calls take 5 to 10 us longer on the host. Build it with "
+                          "`python -m scicompute_attention_b200.build`", RuntimeWarning, stacklevel=3)
+            module = _GeneralFormOnly()
         _native_module = module
     return _native_module
 
