@@ -76,12 +76,12 @@ struct FlashGeom {
     static constexpr int kQTileBytes = kKBlocks * kQBlockBytes;
     // K/V ring. A tile of D=256 takes two slots: K in halves of its columns, V in halves of its keys, each freed when its
     // half of the products is done.
-    static constexpr int kParts = DP == 256 ? 2 : 1;
+    static constexpr int kParts = RingOf(DP).parts;
     static constexpr int kKBlockBytes = BN * 128;           // one column block of K in a slot
     static constexpr int kVKeys = BN / kParts;              // keys of V in a slot
     static constexpr int kVBlockBytes = kVKeys * 128;       // one column block of V in a slot
     static constexpr int kSlotBytes = BN * DP * 2 / kParts;
-    static constexpr int kSlots = (DP == 64) ? 8 : 5;
+    static constexpr int kSlots = RingOf(DP).slots;
     static constexpr int kBarrierBytes = 512;
     static constexpr int kSmemBytes = 1024 + QT * kQTileBytes + kSlots * kSlotBytes + kBarrierBytes;
     static constexpr int kSCol = 0;                         // S_t at kSCol + t * BN
@@ -92,7 +92,7 @@ struct FlashGeom {
     // ragged ones 415 / 371, B=1 S=800 18.5 / 16.5. D=256 went from 64-key tiles with two score buffers (where the score
     // products run at 3/4 of their rate) to 128 keys: B=1 S=3000 168 / 149, B=2 without a mask 655 / 545. It is bound by
     // shared memory then: 448 KB per step (Q and K for the scores, V, the loads, V rewritten) against 2048 clocks of products.
-    static constexpr bool kOwnP = DP != 128;
+    static constexpr bool kOwnP = RingOf(DP).scores_ahead;
     static constexpr int kPCol = !kOwnP ? kSCol : DP == 64 ? 384 : 128;  // P_t at kPCol + t * kPStride
     static constexpr int kPStride = kOwnP ? BN / 2 : BN;
     static_assert(BN == 128 && (DP == 256 ? QT == 1 : QT == 2), "geometry");
@@ -156,7 +156,7 @@ __device__ __forceinline__ int TilesFor(int m0, int tokens, int seq_q, int seq_k
 // three 172, four 146 (B=1, S=3000, lasting load). One warp is too few at D=128 (four prompts of 4096: 632 against 595).
 template <typename T, int DP>
 constexpr int ConverterWarps() {
-    return !PvFormat<T>::kConvertV ? 0 : DP == 256 ? 4 : 2;
+    return PvFormat<T>::kConvertV ? RingOf(DP).converters : 0;
 }
 // Warps of a CTA: 0 TMA and tensor-memory owner, 1 MMA, 2 and 3 V converters (idle for fp16), then four per query tile for
 // the softmax, then what converters are left.

@@ -12,14 +12,26 @@
 
 namespace sca_b200 {
 
+// The ring of a padded head dim: how many slots it has, whether the scores of a tile go out ahead of the products of the one
+// before (see kOwnP in flash_kernel.cuh), how many slots a K or V tile takes, and how many warps rewrite V (bf16; none for fp16).
+struct RingShape {
+    int slots;
+    bool scores_ahead;
+    int parts;
+    int converters;
+};
+constexpr RingShape RingOf(int padded_dim) {
+    return padded_dim == 64 ? RingShape{8, true, 1, 2} : padded_dim == 128 ? RingShape{5, false, 1, 2} : RingShape{5, true, 2, 4};
+}
+
 struct RingLoad {
     bool is_v;
     int tile;
 };
 // The it-th of the 2 * n loads of an item of n KV tiles, in the order in which the products consume them:
-// K_0 V_0 K_1 V_1 ..., or with double-buffered scores K_0 K_1 V_0 K_2 V_1 K_3 ... (S(j+2) follows P(j) V_j).
-SCA_RING_FN RingLoad RingOrder(int it, int n, bool double_scores) {
-    if (!double_scores) return {(it & 1) != 0, it >> 1};
+// K_0 V_0 K_1 V_1 ..., or with the scores ahead K_0 K_1 V_0 K_2 V_1 K_3 ... (S(j+1) does not wait for P(j) V_j).
+SCA_RING_FN RingLoad RingOrder(int it, int n, bool scores_ahead) {
+    if (!scores_ahead) return {(it & 1) != 0, it >> 1};
     const int lead = n > 1 ? 2 : 1;
     if (it < lead) return {false, it};
     const int f = it - lead, rest = n - lead;  // `rest` K tiles still to come, one after each V
