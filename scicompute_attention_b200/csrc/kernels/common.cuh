@@ -30,6 +30,8 @@ bool DebugSyncEnabled();
 int EnsureDynamicSmem(const void* kernel, size_t bytes, const char* kernel_name);
 // Cached SM count of the current device.
 int SmCount();
+// Sends `bytes` of host memory that may go away on return to the device, in the order of the stream.
+int SendToDevice(void* device, const void* host, size_t bytes, cudaStream_t stream, const char* what);
 
 // Launches `kernel` as a programmatic dependent of the kernel ahead of it on the stream (cluster > 1: on clusters of that many
 // CTAs): its CTAs may be set up while that one still runs. So the kernel calls one of the two functions below ahead of its first

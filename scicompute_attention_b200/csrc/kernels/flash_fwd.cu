@@ -200,9 +200,7 @@ int UploadVarlenWork(const VarlenWork& vw, int tokens_per_entry, int block_n, bo
     int2* entries = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(image.data()) + seq_bytes);
     for (size_t i = 0; i < list.size(); ++i) entries[i] = list[i].entry;
     unsigned char* base = static_cast<unsigned char*>(vw.workspace);
-    if (cudaError_t e = cudaMemcpyAsync(base, image.data(), bytes, cudaMemcpyHostToDevice, stream); e != cudaSuccess) {
-        return FailCuda(e, "cudaMemcpyAsync(varlen work list)");
-    }
+    if (int rc = SendToDevice(base, image.data(), bytes, stream, "cudaMemcpyAsync(varlen work list)")) return rc;
     *seqs_out = reinterpret_cast<const int4*>(base);
     *entries_out = reinterpret_cast<const int2*>(base + seq_bytes);
     *num_entries_out = static_cast<int>(list.size());

@@ -195,17 +195,12 @@ public:
         }
         const size_t bytes = static_cast<size_t>(count) * sizeof(int32_t);
         stream_ = stream;
-        cudaError_t err = cudaMallocAsync(reinterpret_cast<void**>(&staged_), bytes, stream);
-        if (err != cudaSuccess) {
+        if (cudaError_t err = cudaMallocAsync(reinterpret_cast<void**>(&staged_), bytes, stream); err != cudaSuccess) {
             staged_ = nullptr;
             cudaGetLastError();
             return FailCuda(err, what);
         }
-        err = cudaMemcpyAsync(staged_, ids, bytes, cudaMemcpyHostToDevice, stream);
-        if (err != cudaSuccess) {
-            cudaGetLastError();
-            return FailCuda(err, what);
-        }
+        if (int rc = SendToDevice(staged_, ids, bytes, stream, what)) return rc;
         ids_ = staged_;
         return SCA_OK;
     }

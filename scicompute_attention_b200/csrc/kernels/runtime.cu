@@ -77,6 +77,35 @@ int EnsureDynamicSmem(const void* kernel, size_t bytes, const char* kernel_name)
     return SCA_OK;
 }
 
+int SendToDevice(void* device, const void* host, size_t bytes, cudaStream_t stream, const char* what) {
+    auto send = [&] {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        cudaGraph_t graph = nullptr;
+        if (cudaError_t err = cudaStreamGetCaptureInfo_v3(stream, &status, nullptr, &graph); err != cudaSuccess) return err;
+        if (status == cudaStreamCaptureStatusActive) {
+            // Every replay reads the host side again, so the graph gets a copy that lives as long as it does.
+            void* kept = std::malloc(bytes);
+            if (kept == nullptr) return cudaErrorMemoryAllocation;
+            std::memcpy(kept, host, bytes);
+            cudaUserObject_t owner = nullptr;
+            if (cudaError_t err = cudaUserObjectCreate(&owner, kept, std::free, 1, cudaUserObjectNoDestructorSync); err != cudaSuccess) {
+                std::free(kept);
+                return err;
+            }
+            if (cudaError_t err = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove); err != cudaSuccess) {
+                cudaUserObjectRelease(owner, 1);
+                return err;
+            }
+            host = kept;
+        }
+        return cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, stream);
+    };
+    const cudaError_t err = send();
+    if (err == cudaSuccess) return SCA_OK;
+    cudaGetLastError();
+    return FailCuda(err, what);
+}
+
 int SmCount() {
     static thread_local int cached_device = -1;
     static thread_local int cached = 0;
