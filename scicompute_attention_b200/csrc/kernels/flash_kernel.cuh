@@ -90,8 +90,9 @@ struct FlashGeom {
     // and is there when the softmax group comes back for it, instead of following P_t(j) V_j. At D=128 there is no room.
     // us in a lasting load, P over S / apart: D=64 B=3 S=2900 without a mask 310 / 297, four prompts of 4096 412 / 390, 10
     // ragged ones 415 / 371, B=1 S=800 18.5 / 16.5. D=256 went from 64-key tiles with two score buffers (where the score
-    // products run at 3/4 of their rate) to 128 keys: B=1 S=3000 168 / 149, B=2 without a mask 655 / 545. It is bound by
-    // shared memory then: 448 KB per step (Q and K for the scores, V, the loads, V rewritten) against 2048 clocks of products.
+    // products run at 3/4 of their rate) to 128 keys: B=1 S=3000 168 / 149, B=2 without a mask 655 / 545. A step takes 2960
+    // clocks then, 2420 for fp16, 2048 of them products; 448 KB go through shared memory (Q and K for the scores, V, the loads,
+    // V rewritten), 320 KB where V is not rewritten.
     static constexpr bool kOwnP = RingOf(DP).scores_ahead;
     static constexpr int kPCol = !kOwnP ? kSCol : DP == 64 ? 384 : 128;  // P_t at kPCol + t * kPStride
     static constexpr int kPStride = kOwnP ? BN / 2 : BN;
