@@ -7,7 +7,8 @@ q is [B, H_q, S_q, D] (layout "bhsd") or [B, S_q, H_q, D] ("bshd"); k/v likewise
 outputs are always freshly allocated contiguous BHSD tensors, allocated on `stream` where one is given.
 
 A call in its plain form (tensors, the current stream) goes through one C function of _native (csrc/torch/native_ops.cpp),
-which answers None where it does not take the call; the code here is the general form, and the one that raises the errors.
+which answers None where it does not take the call; the code here is the general form, and the one that refuses. A launch that
+failed raises its error on either way.
 """
 from __future__ import annotations
 
